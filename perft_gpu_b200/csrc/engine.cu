@@ -84,6 +84,7 @@ constexpr int TILE_CAP = 1 << TILE_CAP_LOG2;
 constexpr int TILE_MIN_LOG2 = 10;  // small levels use tiles down to 1024 items to fill every SM
 constexpr u64 MAX_TILES_PER_NODE_DIV = 1ull << TILE_MIN_LOG2;
 constexpr int TILE_MAXP = TILE_NT;
+constexpr int WEIGHT_BITS = 19;
 constexpr int TILE_MINB = PG_TILE_MINB;          // resident CTAs per SM the register budget targets
 constexpr int MAX_LEGAL_MOVES = 218;
 
@@ -102,6 +103,17 @@ enum { MODE_EXPAND = 0, MODE_LEAF = 1 };
 // share of the tile index (4 B per TILE_CAP items, up to 218 items a node)
 // and of the scan's block sums, rounded up.
 constexpr u64 NODE_BYTES = 6 * 8 + 4 + 4 + 8 + 1;  // (tile index sized for the smallest tile: < 1 B/node)
+// With merged transpositions a node also has a path weight, and the level's
+// set takes MERGE_SLOTS 8-byte slots per node until the scan (whose entries
+// and tile index reuse that memory).
+constexpr u64 MERGE_SLOTS = 2;
+constexpr u64 NODE_BYTES_MERGE = 6 * 8 + 4 + 4 + 8 + 8 * MERGE_SLOTS + 1;
+// Plies from the root at which merging starts: two plies reach almost no
+// position twice, the third brings the first a-x-b = b-x-a pairs.
+constexpr int MERGE_MIN_PLIES = 3;
+// Share of a merged level's nodes predicted to stay (measured: 0.54-0.68 in
+// 8-30-ply playouts); predictions only choose the path and the grids.
+constexpr double MERGE_KEPT = 0.7;
 
 // ------------------------------------------------------- level node boards
 // A level's boards in HBM are a structure of arrays of plane pairs: pair j of
@@ -243,7 +255,7 @@ __global__ void __launch_bounds__(SCAN_NT) k_scan_apply(const u32 *__restrict__ 
 // ----------------------------------------------------------------- roots
 __global__ void k_init_roots(const u64 *__restrict__ pos48, const u32 *__restrict__ ids, u32 n,
                              u64 *__restrict__ planes, u64 stride, u32 *__restrict__ cnt,
-                             u32 *__restrict__ root, int depth,
+                             u32 *__restrict__ root, unsigned long long *__restrict__ weight, int depth,
                              unsigned long long *__restrict__ rootCounts, u32 *err)
 {
     const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -262,6 +274,7 @@ __global__ void k_init_roots(const u64 *__restrict__ pos48, const u32 *__restric
     level_put(planes, stride, i, b);
     cnt[i] = c;
     root[i] = id;
+    if (weight) weight[i] = 1ull;
     if (depth == 0) rootCounts[id] = 1ull;
     if (depth == 1) rootCounts[id] = c;
 }
@@ -280,6 +293,8 @@ struct LevelDesc {
     u64 stride;
     u32 *cnt;
     u32 *root;
+    unsigned long long *weight;  // merged runs: paths that reach the node
+    unsigned long long *set;     // merged levels: the set's slots (transient), null when they do not fit
     u64 n;        // nodes: the previous ply's children, then the roots joining here
     u64 nChild;   // children written by the previous ply's tile kernel
     u64 *pscan;
@@ -294,6 +309,7 @@ struct TileParams {
     u64 pstride;
     const u64 *pscan; // nParents + 1 item offsets
     const u32 *proot;  // root id of each parent; null: sums go to the parent's own slot
+    const unsigned long long *pweight;  // paths that reach each parent; null: one each
     u64 nParents;
     const u32 *tileFirst;  // indexed by absolute tile number
     u64 itemBase;     // first item of this launch (multiple of the tile size)
@@ -305,6 +321,7 @@ struct TileParams {
     u64 cstride;
     u32 *ccnt;
     u32 *croot;
+    unsigned long long *cweight;  // null: not kept
     // last ply output
     unsigned long long *rootCounts;
     u32 *err;
@@ -314,6 +331,11 @@ struct TileParams {
     const struct TileParams *planEntry;
 };
 
+
+// The nodes of one root in a level (they are contiguous).
+struct MergeSeg {
+    u32 begin, end;
+};
 
 constexpr int DD_MAX_LEVELS = 24;
 // Largest predicted tree (bytes of materialised plies) run as a graph, on top
@@ -333,6 +355,10 @@ struct DevPlan {
     u32 joinN[DD_MAX_LEVELS];
     const u32 *joinIds[DD_MAX_LEVELS];
     int capMax[DD_MAX_LEVELS];  // largest tile (log2 items) for the items of level k
+    int weighted;                  // levels carry path weights (some level is merged)
+    int mergeLv[DD_MAX_LEVELS];    // level k's transpositions are merged
+    MergeSeg *segs;                // per root: its nodes in the level being merged
+    const uint8_t *rootDepth;
     // the tile launch of level k's items, completed on the device by the scan
     // (level pointers and sizes) and copied into c_ddTile before that launch
     TileParams tp[DD_MAX_LEVELS];
@@ -453,6 +479,7 @@ __device__ void dd_plan_level(DevPlan *plan, int lv, int last, u64 total)
     T.pstride = L.stride;
     T.pscan = L.pscan;
     T.proot = L.root;
+    T.pweight = L.weight;
     T.nParents = L.n;
     T.tileFirst = L.tileFirst;
     T.itemBase = 0;
@@ -468,6 +495,7 @@ __device__ void dd_plan_level(DevPlan *plan, int lv, int last, u64 total)
     C.planes = (u64 *)dd_take(plan, 48 * C.stride);
     C.cnt = (u32 *)dd_take(plan, 4 * C.stride);
     C.root = (u32 *)dd_take(plan, 4 * C.stride);
+    C.weight = plan->weighted ? (unsigned long long *)dd_take(plan, 8 * C.stride) : nullptr;
     C.pscan = (u64 *)dd_take(plan, 8 * (m + 1));
     C.tileFirst = (u32 *)dd_take(plan, 4 * ((m * MAX_LEGAL_MOVES) / MAX_TILES_PER_NODE_DIV + 2));
     C.bsum = (u64 *)dd_take(plan, 8 * ((m + SCAN_CHUNK - 1) / SCAN_CHUNK + 1));
@@ -475,11 +503,19 @@ __device__ void dd_plan_level(DevPlan *plan, int lv, int last, u64 total)
         C.n = 0;
         L.total = 0;  // nothing is expanded into a level that does not exist
     }
+    // The merge set lies above the bump mark: it is done with before the next
+    // level's buffers are placed there.  A set that does not fit leaves the
+    // level unmerged.
+    const u64 setAt = (plan->bump + 255) & ~255ULL;
+    C.set = plan->mergeLv[lv + 1] && !plan->overflow && setAt + 8 * MERGE_SLOTS * m <= plan->cap
+                ? (unsigned long long *)(plan->base + setAt)
+                : nullptr;
     T.itemEnd = L.total;
     T.cpl = C.planes;
     T.cstride = C.stride;
     T.ccnt = C.cnt;
     T.croot = C.root;
+    T.cweight = C.weight;
 }
 
 __global__ void __launch_bounds__(SCAN_NT) k_dd_scan_apply(DevPlan *plan, int lv)
@@ -538,6 +574,123 @@ __global__ void k_dd_join(DevPlan *plan, int lv, const u64 *__restrict__ pos48, 
     level_put(C.planes, C.stride, g, b);
     C.cnt[g] = c;
     C.root[g] = id;
+    if (C.weight) C.weight[g] = 1ull;
+}
+
+// ------------------------------------------------- merged transpositions
+// Different move orders reach the same position.  From the third ply below a
+// root on, a level therefore holds many equal nodes (42% of the third ply's
+// children and again 42% of the fourth's in 8-30-ply playouts), and each
+// copy's whole subtree would be searched again.  Before a level is scanned,
+// equal nodes of one root are merged: one of them, the owner, keeps its
+// moves and takes over the others' path weights; the others lose theirs
+// (cnt = 0).  A node's weight is the number of move paths from its root that
+// reach it, children inherit their parent's, and the count-only ply adds
+// weight x moves, so the root's count is the same.  Nodes are merged only
+// when their boards (state included) are equal in all 48 bytes: the hash
+// only picks the slot.
+//
+// The set is open addressed, MERGE_SLOTS 8-byte slots {hash tag, node} per
+// node.  Each root's nodes use the slots at their own place in the set, so a
+// batch works on one small region of the set and of the boards at a time
+// and most of its random accesses stay in L2.  Which of several equal nodes
+// becomes the owner depends on timing; the sums do not.
+// Bound by the latency of its chain of dependent accesses (segment, slot,
+// owner's board): one node per thread, and enough CTAs to fill every SM.
+// Measured: 4096 playouts of depths 4-6 1588 -> 671 ms, one middlegame
+// position at depth 7 34.2 -> 6.8 ms, an opening at depth 8 365 -> 35 ms.
+constexpr unsigned long long MERGE_EMPTY = ~0ULL;
+constexpr int MERGE_MAX_PROBES = 64;
+
+struct MergeLevel {
+    const u64 *planes;
+    u64 stride, n;
+    u32 *cnt;
+    const u32 *root;
+    unsigned long long *weight;
+    unsigned long long *set;
+    MergeSeg *segs;
+    const uint8_t *rootDepth;
+    int remaining;  // plies left below the level
+};
+
+__device__ __forceinline__ u64 board_hash(const Board &b)
+{
+    u64 h = b.mine * 0x9E3779B97F4A7C15ULL + b.pawns * 0xC2B2AE3D27D4EB4FULL + b.knights * 0x165667B19E3779F9ULL +
+            b.bq * 0xD6E8FEB86659FD93ULL + b.rq * 0xA0761D6478BD642FULL + b.kings * 0xE7037ED1A0B428DBULL;
+    h ^= h >> 32;
+    h *= 0xD6E8FEB86659FD93ULL;
+    h ^= h >> 29;
+    h *= 0x9E3779B97F4A7C15ULL;
+    return h ^ (h >> 32);
+}
+
+// Clears the set and finds every root's nodes.  Roots fewer than
+// MERGE_MIN_PLIES above the level get an empty segment: nothing to merge.
+__device__ __forceinline__ void merge_prepare(const MergeLevel &M)
+{
+    const u64 t0 = (u64)blockIdx.x * blockDim.x + threadIdx.x, step = (u64)gridDim.x * blockDim.x;
+    ulonglong2 *set2 = reinterpret_cast<ulonglong2 *>(M.set);
+    for (u64 i = t0; i < M.n; i += step) {
+        set2[i] = make_ulonglong2(MERGE_EMPTY, MERGE_EMPTY);
+        const u32 r = M.root[i];
+        const bool deep = M.rootDepth[r] >= M.remaining + MERGE_MIN_PLIES;
+        if (i == 0 || M.root[i - 1] != r) M.segs[r].begin = deep ? (u32)i : 0u;
+        if (i + 1 == M.n || M.root[i + 1] != r) M.segs[r].end = deep ? (u32)(i + 1) : 0u;
+    }
+}
+
+__device__ __forceinline__ void merge_nodes(const MergeLevel &M)
+{
+    const u64 t0 = (u64)blockIdx.x * blockDim.x + threadIdx.x, step = (u64)gridDim.x * blockDim.x;
+    for (u64 i = t0; i < M.n; i += step) {
+        if (M.cnt[i] == 0) continue;  // no moves: nothing below to search
+        const MergeSeg sg = M.segs[M.root[i]];
+        if (sg.end - sg.begin < 2) continue;
+        const Board b = level_get(M.planes, M.stride, i);
+        const u64 h = board_hash(b);
+        const u64 nSlots = MERGE_SLOTS * (u64)(sg.end - sg.begin);
+        unsigned long long *slots = M.set + MERGE_SLOTS * (u64)sg.begin;
+        const unsigned long long mine = (h << 32) | (u32)i;
+        u64 at = __umul64hi(h, nSlots);
+        for (int k = 0; k < MERGE_MAX_PROBES; k++) {
+            unsigned long long v = *(volatile unsigned long long *)(slots + at);
+            if (v == MERGE_EMPTY) {
+                v = atomicCAS(slots + at, MERGE_EMPTY, mine);
+                if (v == MERGE_EMPTY) break;  // this node owns its position
+            }
+            if ((v >> 32) == (u32)h) {
+                const u32 o = (u32)v;
+                const Board ob = level_get(M.planes, M.stride, o);
+                if (((ob.mine ^ b.mine) | (ob.pawns ^ b.pawns) | (ob.knights ^ b.knights) | (ob.bq ^ b.bq) |
+                     (ob.rq ^ b.rq) | (ob.kings ^ b.kings)) == 0) {
+                    atomicAdd(M.weight + o, M.weight[i]);
+                    M.cnt[i] = 0;
+                    break;
+                }
+            }
+            if (++at == nSlots) at = 0;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(256) k_merge_prepare(const MergeLevel M) { merge_prepare(M); }
+__global__ void __launch_bounds__(256) k_merge_nodes(const MergeLevel M) { merge_nodes(M); }
+
+// The same for a device-driven level.
+__device__ __forceinline__ MergeLevel dd_merge_level(const DevPlan *plan, int lv, int remaining)
+{
+    const LevelDesc &C = plan->lv[lv];
+    return MergeLevel{C.planes, C.stride, C.set ? C.n : 0, C.cnt, C.root, C.weight, C.set,
+                      plan->segs, plan->rootDepth, remaining};
+}
+__global__ void __launch_bounds__(256) k_dd_merge_prepare(const DevPlan *plan, int lv, int remaining)
+{
+    merge_prepare(dd_merge_level(plan, lv, remaining));
+}
+__global__ void __launch_bounds__(256) k_dd_merge_nodes(const DevPlan *plan, int lv, int remaining)
+{
+    merge_nodes(dd_merge_level(plan, lv, remaining));
 }
 
 // ------------------------------------------------------------ tile kernel
@@ -595,6 +748,7 @@ __global__ void __launch_bounds__(TILE_NT, TILE_MINB) k_tile(const TileParams Pi
     __shared__ u64 sqEnd[TRACK ? TILE_MAXP : 1];
     __shared__ int sdelta[TRACK ? TILE_MAXP : 1];
     __shared__ u32 sroot[TILE_MAXP];
+    __shared__ unsigned long long sweight[TRACK ? 1 : TILE_MAXP];  // paths that reach each parent
     __shared__ u32 srun[TILE_MAXP];
     __shared__ u32 srunRoot[TILE_MAXP];
     __shared__ unsigned long long sacc[TILE_MAXP];
@@ -644,12 +798,18 @@ __global__ void __launch_bounds__(TILE_NT, TILE_MINB) k_tile(const TileParams Pi
                     skS[tid] = (uint8_t)ctz(pb.kings & pb.mine);
                 }
                 sroot[tid] = P.proot ? P.proot[q] : (u32)q;  // no root array: account to the parent itself
+                if (!TRACK) sweight[tid] = P.pweight ? P.pweight[q] : 1ull;
             }
             const u64 sBeg = max(P.pscan[p], iBeg);
             const u64 sEnd = min(P.pscan[p + nP], iEnd);
             __syncthreads();
 
             int nRuns = 0;
+            // a warp's 32 products of a weight below 2^WEIGHT_BITS and a count
+            // (at most 218) sum below 2^32; windows with larger weights add
+            // each product by itself
+            const bool narrow = TRACK || MODE == MODE_EXPAND || !P.pweight ||
+                                __syncthreads_and(!valid || (sweight[tid] >> WEIGHT_BITS) == 0);
             if (MODE == MODE_LEAF || TRACK) {
                 // parents are ordered by root: number the runs of equal roots.
                 // Usually the whole window belongs to one root, which one
@@ -716,11 +876,19 @@ __global__ void __launch_bounds__(TILE_NT, TILE_MINB) k_tile(const TileParams Pi
                             level_put(P.cpl, P.cstride, g, ch);
                             P.ccnt[g] = cnt;
                             P.croot[g] = sroot[pl];
+                            if (!TRACK && P.cweight) P.cweight[g] = sweight[pl];
                         }
                     } else {
                         atomicOr(P.err, DERR_BAD_ITEM);
                         pl = 0;
                     }
+                }
+                if (MODE == MODE_LEAF && !TRACK) {
+                    if (!narrow) {
+                        if (act) atomicAdd(&sacc[srun[pl]], (unsigned long long)cnt * sweight[pl]);
+                        continue;
+                    }
+                    cnt *= (u32)sweight[pl];  // (idle lanes: 0)
                 }
                 if (PG_ONE_RUN_SUM && MODE == MODE_LEAF && !TRACK && nRuns == 1) {
                     // the whole window belongs to one root: a plain warp sum
@@ -1220,6 +1388,7 @@ struct DeviceLevel {
     u32 *cnt;
     u32 *root;  // root id (no TT) or parent index in the previous level (TT)
     u64 n;
+    unsigned long long *weight = nullptr;  // merged runs: paths that reach each node
     // transposition-table runs only
     u64 *hash = nullptr;   // slot key
     u64 *hash2 = nullptr;  // verification key
@@ -1312,7 +1481,7 @@ private:
         return arena + a;
     }
     u64 arena_free() const { return arenaCap > arenaTop ? arenaCap - arenaTop : 0; }
-    bool alloc_level(DeviceLevel &L, u64 n);
+    bool alloc_level(DeviceLevel &L, u64 n, bool weighted = false);
     int scan(const u32 *cnt, u64 n, int remaining, u64 *&scanOut, u32 *&tileFirst, u64 &total, int &capLog2);
     int launch_tile(int mode, int remaining, const DeviceLevel &parents, const u64 *pscan, const u32 *tileFirst,
                     int capLog2, u64 itemBase, u64 itemEnd, DeviceLevel *children, unsigned long long *rootCounts);
@@ -1323,7 +1492,14 @@ private:
         const u64 *dPos = nullptr;
         const u32 *ids[21] = {};
         u32 n[21] = {};
+        // merged runs (else null): every root's depth, and its nodes in the level being merged
+        const uint8_t *depths = nullptr;
+        MergeSeg *segs = nullptr;
+        int maxDepth = 0;
     };
+    int merge_level(const Joiners &J, const DeviceLevel &C, int remaining);
+    int run_levels(const u64 *dPos, const uint8_t *depths, u32 n, unsigned long long *rootCounts, bool merge);
+    bool mergeEnabled = true;
     int process_level(const DeviceLevel &L, int remaining, unsigned long long *rootCounts,
                       const Joiners *join = nullptr);
     int init_joiners(const Joiners &J, int depth, DeviceLevel &C, u64 at, unsigned long long *rootCounts);
@@ -1591,6 +1767,7 @@ int Engine::init(const perft_config &cfg)
             if (v >= 1 && v <= (long)SMALL_LIST_CAP) smallListCap = (u32)v;
         }
     }
+    mergeEnabled = !(getenv("PERFT_NO_MERGE") && getenv("PERFT_NO_MERGE")[0] == '1');
     ddEnabled = !(getenv("PERFT_NO_GRAPHS") && getenv("PERFT_NO_GRAPHS")[0] == '1');
     ddForce = getenv("PERFT_DD_FORCE") && getenv("PERFT_DD_FORCE")[0] == '1';
     ddMaxBytes = DD_MAX_BYTES_DEFAULT;
@@ -1645,14 +1822,31 @@ void Engine::shutdown()
     ready = false;
 }
 
-bool Engine::alloc_level(DeviceLevel &L, u64 n)
+bool Engine::alloc_level(DeviceLevel &L, u64 n, bool weighted)
 {
     L.n = n;
     L.stride = (n + 31) & ~31ULL;
     L.planes = (u64 *)alloc(6 * 8 * L.stride);
     L.cnt = (u32 *)alloc(4 * L.stride);
     L.root = (u32 *)alloc(4 * L.stride);
-    return L.planes && L.cnt && L.root;
+    L.weight = weighted ? (unsigned long long *)alloc(8 * L.stride) : nullptr;
+    return L.planes && L.cnt && L.root && (L.weight || !weighted);
+}
+
+// Merges the equal nodes of a level with `remaining` plies left.
+int Engine::merge_level(const Joiners &J, const DeviceLevel &C, int remaining)
+{
+    if (!C.weight || C.n < 2 || J.maxDepth < remaining + MERGE_MIN_PLIES) return PERFT_OK;
+    const u64 mark = arenaTop;
+    unsigned long long *set = (unsigned long long *)alloc(8 * MERGE_SLOTS * C.n);
+    arenaTop = mark;  // free again once the merge has run (stream order)
+    if (!set) return PERFT_OK;  // the level stays unmerged
+    const MergeLevel M{C.planes, C.stride, C.n, C.cnt, C.root, C.weight, set, J.segs, J.depths, remaining};
+    const unsigned grid = (unsigned)std::min<u64>((C.n + 255) / 256, 64ull * nsm);
+    k_merge_prepare<<<grid, 256, 0, stream>>>(M);
+    k_merge_nodes<<<grid, 256, 0, stream>>>(M);
+    stats.other_launches += 2;
+    return check(cudaGetLastError(), "k_merge_nodes");
 }
 
 // `remaining`: remaining depth of the level scanned; its items go to the
@@ -1693,6 +1887,7 @@ int Engine::launch_tile(int mode, int remaining, const DeviceLevel &parents, con
     P.pstride = parents.stride;
     P.pscan = pscan;
     P.proot = parents.root;
+    P.pweight = parents.weight;
     P.nParents = parents.n;
     P.tileFirst = tileFirst;
     P.itemBase = itemBase;
@@ -1704,6 +1899,7 @@ int Engine::launch_tile(int mode, int remaining, const DeviceLevel &parents, con
         P.cstride = children->stride;
         P.ccnt = children->cnt;
         P.croot = children->root;
+        P.cweight = children->weight;
     }
     P.rootCounts = rootCounts;
     P.err = dErr;
@@ -1746,7 +1942,8 @@ int Engine::init_joiners(const Joiners &J, int depth, DeviceLevel &C, u64 at, un
     const u32 nj = J.n[depth];
     if (!nj) return PERFT_OK;
     k_init_roots<<<(nj + 127) / 128, 128, 0, stream>>>(J.dPos, J.ids[depth], nj, C.planes + 2 * at, C.stride,
-                                                        C.cnt + at, C.root + at, depth, rootCounts, dErr);
+                                                        C.cnt + at, C.root + at, C.weight ? C.weight + at : nullptr,
+                                                        depth, rootCounts, dErr);
     stats.other_launches++;
     return check(cudaGetLastError(), "k_init_roots");
 }
@@ -1779,7 +1976,8 @@ int Engine::process_level(const DeviceLevel &L, int remaining, unsigned long lon
     // interior ply: children fit whole, or in tile-aligned chunks
     const u64 slack = std::min<u64>(64ull << 20, arenaCap / 16);
     const u64 freeB = arena_free() > slack ? arena_free() - slack : 0;
-    u64 budgetNodes = freeB / NODE_BYTES;
+    const bool weighted = L.weight != nullptr;
+    u64 budgetNodes = freeB / (weighted ? NODE_BYTES_MERGE : NODE_BYTES);
     if (remaining > 3) budgetNodes /= 2;  // leave room for the plies below
     budgetNodes = budgetNodes > nJoin ? budgetNodes - nJoin : 0;
     // whole level when it fits; otherwise tile-aligned chunks
@@ -1792,13 +1990,17 @@ int Engine::process_level(const DeviceLevel &L, int remaining, unsigned long lon
         const bool last = k + 1 == nChunks;
         const u64 cm = arenaTop;
         DeviceLevel C;
-        if (!alloc_level(C, (hi - lo) + (last ? nJoin : 0))) return PERFT_ERR_OUT_OF_MEMORY;
+        if (!alloc_level(C, (hi - lo) + (last ? nJoin : 0), weighted)) return PERFT_ERR_OUT_OF_MEMORY;
         if (hi > lo) {
             rc = launch_tile(MODE_EXPAND, remaining, L, pscan, tileFirst, capLog2, lo, hi, &C, nullptr);
             if (rc != PERFT_OK) return rc;
         }
         if (last && nJoin) {
             rc = init_joiners(*join, remaining - 1, C, hi - lo, rootCounts);
+            if (rc != PERFT_OK) return rc;
+        }
+        if (join) {
+            rc = merge_level(*join, C, remaining - 1);
             if (rc != PERFT_OK) return rc;
         }
         rc = process_level(C, remaining - 1, rootCounts, join);
@@ -2110,6 +2312,10 @@ int Engine::build_dd(DDGraph &G)
     };
     DevPlan *dPlan = (DevPlan *)place(sizeof(DevPlan));
     u32 *dIds = (u32 *)place(4 * n);
+    // merged transpositions (levels at least MERGE_MIN_PLIES below some root)
+    const bool merge = mergeEnabled && d - 2 >= MERGE_MIN_PLIES;
+    uint8_t *dDepths = merge ? (uint8_t *)place(n) : nullptr;
+    MergeSeg *dSegs = merge ? (MergeSeg *)place(sizeof(MergeSeg) * n) : nullptr;
     const u64 n0 = nAt[d];
     LevelDesc L0{};
     L0.n = n0;
@@ -2118,6 +2324,7 @@ int Engine::build_dd(DDGraph &G)
     L0.planes = (u64 *)place(48 * L0.stride);
     L0.cnt = (u32 *)place(4 * L0.stride);
     L0.root = (u32 *)place(4 * L0.stride);
+    L0.weight = merge ? (unsigned long long *)place(8 * L0.stride) : nullptr;
     L0.pscan = (u64 *)place(8 * (n0 + 1));
     L0.tileFirst = (u32 *)place(4 * ((n0 * MAX_LEGAL_MOVES) / MAX_TILES_PER_NODE_DIV + 2));
     L0.bsum = (u64 *)place(8 * ((n0 + SCAN_CHUNK - 1) / SCAN_CHUNK + 1));
@@ -2130,7 +2337,7 @@ int Engine::build_dd(DDGraph &G)
     if (bump > cap) return PERFT_ERR_OUT_OF_MEMORY;
 
     ENG_TRY(cudaMallocHost(&G.hTemplate, sizeof(DevPlan)));
-    ENG_TRY(cudaMallocHost(&G.hIds, 4 * n));
+    ENG_TRY(cudaMallocHost(&G.hIds, 5 * n));  // root ids, then every root's depth
     ENG_TRY(cudaMallocHost(&G.hFlags, 64));
     ENG_TRY(cudaEventCreate(&G.evLeaf0));
     ENG_TRY(cudaEventCreate(&G.evLeaf1));
@@ -2140,6 +2347,10 @@ int Engine::build_dd(DDGraph &G)
     G.hTemplate->bump = bump;
     G.hTemplate->tileTarget = 2 * gridTile[MODE_LEAF][G.svL];
     G.hTemplate->tileCounter = dCounter;
+    G.hTemplate->weighted = merge;
+    G.hTemplate->segs = dSegs;
+    G.hTemplate->rootDepth = dDepths;
+    for (int lv = MERGE_MIN_PLIES; lv <= d - 2; lv++) G.hTemplate->mergeLv[lv] = merge;
     G.hTemplate->lv[0] = L0;
     for (int dd = 2; dd < d; dd++) {
         G.hTemplate->joinN[d - dd] = nAt[dd];
@@ -2171,21 +2382,24 @@ int Engine::build_dd(DDGraph &G)
         }
     }
     memcpy(G.hIds, order.data(), 4 * n);
+    memcpy(G.hIds + n, G.depths.data(), n);
 
     ENG_TRY(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
     cudaMemcpyAsync(dPlan, G.hTemplate, sizeof(DevPlan), cudaMemcpyHostToDevice, stream);
     cudaMemcpyAsync(dIds, G.hIds, 4 * n, cudaMemcpyHostToDevice, stream);
+    if (merge) cudaMemcpyAsync(dDepths, G.hIds + n, n, cudaMemcpyHostToDevice, stream);
     cudaMemsetAsync(G.dOut, 0, 8 * n, stream);
     cudaMemsetAsync(dErr, 0, 4, stream);
     G.otherLaunches = (nAt[0] ? 1 : 0) + (nAt[1] ? 1 : 0) + (d >= 2 ? 1 : 0);
     for (int dd = 0; dd <= 1; dd++)
         if (nAt[dd])
             k_init_roots<<<(nAt[dd] + 127) / 128, 128, 0, stream>>>(G.dPos, dIds + offAt[dd], nAt[dd], sPlanes,
-                                                                   sStride, sCnt, sRoot, dd,
+                                                                   sStride, sCnt, sRoot, nullptr, dd,
                                                                    (unsigned long long *)G.dOut, dErr);
     if (d >= 2)
         k_init_roots<<<(unsigned)((n0 + 127) / 128), 128, 0, stream>>>(G.dPos, dIds + offAt[d], (u32)n0,
-                                                                      L0.planes, L0.stride, L0.cnt, L0.root, d,
+                                                                      L0.planes, L0.stride, L0.cnt, L0.root,
+                                                                      L0.weight, d,
                                                                       (unsigned long long *)G.dOut, dErr);
     for (int lv = 0; lv <= d - 2; lv++) {
         const int last = lv == d - 2;
@@ -2230,6 +2444,15 @@ int Engine::build_dd(DDGraph &G)
             if (nj) {
                 k_dd_join<<<(nj + 127) / 128, 128, 0, stream>>>(dPlan, lv + 1, G.dPos, dErr);
                 G.otherLaunches += 1;
+            }
+            if (G.hTemplate->mergeLv[lv + 1]) {
+                // grid-stride: any grid is correct, a level predicted small gets a smaller one
+                int mg = 64 * nsm;
+                if ((int)G.predLv.size() > lv + 1)
+                    mg = (int)std::min<double>(mg, std::max<double>(8.0, G.predLv[lv + 1] / 256.0));
+                k_dd_merge_prepare<<<mg, 256, 0, stream>>>(dPlan, lv + 1, d - (lv + 1));
+                k_dd_merge_nodes<<<mg, 256, 0, stream>>>(dPlan, lv + 1, d - (lv + 1));
+                G.otherLaunches += 2;
             }
         }
     }
@@ -2293,8 +2516,9 @@ int Engine::run_dd(const u64 *dPos, const uint8_t *depths, u32 n, u64 *dOut, boo
                 sum += nodes;
                 predLv[join + k] += nodes;
                 nodes *= 32.0;
+                if (mergeEnabled && k >= MERGE_MIN_PLIES) nodes *= MERGE_KEPT;
             }
-            est += sum * 72.0;
+            est += sum * (mergeEnabled && d - 2 >= MERGE_MIN_PLIES ? 88.0 : 72.0);
         }
         if (est > 0.85 * (double)arena_free()) return PERFT_OK;
         if (est > ddMaxBytes) return PERFT_OK;
@@ -2414,6 +2638,57 @@ int Engine::sync_and_check_errors()
     return PERFT_OK;
 }
 
+// Batch without a table, host-driven.  All depth groups share their plies:
+// the deepest roots start, the others join the level of their remaining
+// depth, so the batch takes one launch per ply (chunked only where a level
+// does not fit the arena).  Roots of depth 0 and 1 are answered by
+// k_init_roots alone.  With `merge`, levels from the third ply below a root
+// on are merged.
+int Engine::run_levels(const u64 *dPos, const uint8_t *depths, u32 n, unsigned long long *rootCounts, bool merge)
+{
+    std::map<int, std::vector<u32>, std::greater<int>> groups;
+    for (u32 i = 0; i < n; i++) groups[depths[i]].push_back(i);
+    const int dmax = groups.begin()->first;
+    std::vector<u32> order;
+    order.reserve(n);
+    Joiners J;
+    J.dPos = dPos;
+    u32 *dIds = (u32 *)alloc(4ull * n);
+    if (!dIds) return PERFT_ERR_OUT_OF_MEMORY;
+    for (auto &g : groups) {
+        J.ids[g.first] = dIds + order.size();
+        J.n[g.first] = (u32)g.second.size();
+        order.insert(order.end(), g.second.begin(), g.second.end());
+    }
+    ENG_TRY(cudaMemcpyAsync(dIds, order.data(), 4ull * n, cudaMemcpyHostToDevice, stream));
+    merge = merge && dmax - 2 >= MERGE_MIN_PLIES;
+    if (merge) {
+        uint8_t *dDepths = (uint8_t *)alloc(n);
+        J.segs = (MergeSeg *)alloc(sizeof(MergeSeg) * (u64)n);
+        if (!dDepths || !J.segs) return PERFT_ERR_OUT_OF_MEMORY;
+        ENG_TRY(cudaMemcpyAsync(dDepths, depths, n, cudaMemcpyHostToDevice, stream));
+        J.depths = dDepths;
+        J.maxDepth = dmax;
+    }
+    // the shallow roots (depth 0, 1) in one scratch level each
+    for (int d = 0; d <= 1; d++) {
+        if (!J.n[d]) continue;
+        const u64 gm = arenaTop;
+        DeviceLevel S;
+        if (!alloc_level(S, J.n[d])) return PERFT_ERR_OUT_OF_MEMORY;
+        const int rc = init_joiners(J, d, S, 0, rootCounts);
+        if (rc != PERFT_OK) return rc;
+        arenaTop = gm;
+    }
+    if (dmax < 2) return PERFT_OK;
+    DeviceLevel L0;
+    if (!alloc_level(L0, J.n[dmax], merge)) return PERFT_ERR_OUT_OF_MEMORY;
+    int rc = init_joiners(J, dmax, L0, 0, rootCounts);
+    if (rc == PERFT_OK) rc = sync_and_check_errors();
+    if (rc == PERFT_OK) rc = process_level(L0, dmax, rootCounts, &J);
+    return rc;
+}
+
 int Engine::run_batch(const u64 *dPos, const uint8_t *depths, u32 n, u64 *dOut, bool trySmall)
 {
     ENG_TRY(cudaSetDevice(device));
@@ -2432,73 +2707,40 @@ int Engine::run_batch(const u64 *dPos, const uint8_t *depths, u32 n, u64 *dOut, 
     ENG_TRY(cudaMemsetAsync(rootCounts, 0, 8ull * n, stream));
     ENG_TRY(cudaMemsetAsync(dErr, 0, 4, stream));
 
-    // group roots by depth: every node of a level then has the same remaining depth
-    std::map<int, std::vector<u32>, std::greater<int>> groups;
-    for (u32 i = 0; i < n; i++) groups[depths[i]].push_back(i);
-
     int rc = PERFT_OK;
     if (!tt) {
-        // Without a table all depth groups share their plies: the deepest
-        // roots start, the others join the level of their remaining depth,
-        // so the batch takes one launch per ply (chunked only where a level
-        // does not fit the arena).  Roots of depth 0 and 1 are answered by
-        // k_init_roots alone.
-        std::vector<u32> order;
-        order.reserve(n);
-        Joiners J;
-        J.dPos = dPos;
-        std::vector<std::pair<int, size_t>> offs;
-        for (auto &g : groups) {
-            offs.push_back({g.first, order.size()});
-            order.insert(order.end(), g.second.begin(), g.second.end());
+        rc = run_levels(dPos, depths, n, rootCounts, mergeEnabled);
+        // path weights and the merge set cost memory: an arena too small for
+        // them still runs what it ran without
+        if (rc == PERFT_ERR_OUT_OF_MEMORY && mergeEnabled) {
+            arenaTop = mark0;
+            ENG_TRY(cudaMemsetAsync(rootCounts, 0, 8ull * n, stream));
+            rc = run_levels(dPos, depths, n, rootCounts, false);
         }
-        u32 *dIds = (u32 *)alloc(4ull * n);
-        if (!dIds) rc = PERFT_ERR_OUT_OF_MEMORY;
-        if (rc == PERFT_OK) {
-            ENG_TRY(cudaMemcpyAsync(dIds, order.data(), 4ull * n, cudaMemcpyHostToDevice, stream));
-            for (auto &o : offs) {
-                J.ids[o.first] = dIds + o.second;
-                J.n[o.first] = (u32)groups[o.first].size();
-            }
-            const int dmax = groups.begin()->first;
-            // the shallow roots (depth 0, 1) in one scratch level each
-            for (int d = 0; d <= 1 && rc == PERFT_OK; d++) {
-                if (!J.n[d]) continue;
-                const u64 gm = arenaTop;
-                DeviceLevel S;
-                if (!alloc_level(S, J.n[d])) rc = PERFT_ERR_OUT_OF_MEMORY;
-                else rc = init_joiners(J, d, S, 0, rootCounts);
-                arenaTop = gm;
-            }
-            if (rc == PERFT_OK && dmax >= 2) {
-                DeviceLevel L0;
-                if (!alloc_level(L0, J.n[dmax])) rc = PERFT_ERR_OUT_OF_MEMORY;
-                if (rc == PERFT_OK) rc = init_joiners(J, dmax, L0, 0, rootCounts);
-                if (rc == PERFT_OK) rc = sync_and_check_errors();
-                if (rc == PERFT_OK) rc = process_level(L0, dmax, rootCounts, &J);
-            }
-        }
-        groups.clear();  // done: skip the per-group loop below
     }
+    // with a table, roots are grouped by depth: every node of a level then has the same remaining depth
+    std::map<int, std::vector<u32>, std::greater<int>> groups;
+    if (tt)
+        for (u32 i = 0; i < n; i++) groups[depths[i]].push_back(i);
     for (auto &g : groups) {
         const int depth = g.first;
         const std::vector<u32> &ids = g.second;
         const u64 gm = arenaTop;
         u32 *dIds = (u32 *)alloc(4ull * ids.size());
         DeviceLevel L0;
-        if (!dIds || !(tt ? alloc_level_tt(L0, ids.size()) : alloc_level(L0, ids.size()))) {
+        if (!dIds || !alloc_level_tt(L0, ids.size())) {
             rc = PERFT_ERR_OUT_OF_MEMORY;
             break;
         }
         ENG_TRY(cudaMemcpyAsync(dIds, ids.data(), 4ull * ids.size(), cudaMemcpyHostToDevice, stream));
         const u32 nb = (u32)((ids.size() + 127) / 128);
         k_init_roots<<<nb, 128, 0, stream>>>(dPos, dIds, (u32)ids.size(), L0.planes, L0.stride, L0.cnt,
-                                              L0.root, depth, rootCounts, dErr);
+                                              L0.root, nullptr, depth, rootCounts, dErr);
         stats.other_launches++;
         ENG_TRY(cudaGetLastError());
         rc = sync_and_check_errors();
         if (rc != PERFT_OK) break;
-        if (depth >= 2) rc = tt ? process_level_tt(L0, depth, nullptr, rootCounts) : process_level(L0, depth, rootCounts);
+        if (depth >= 2) rc = process_level_tt(L0, depth, nullptr, rootCounts);
         arenaTop = gm;
         if (rc != PERFT_OK) break;
     }
@@ -2954,7 +3196,7 @@ extern "C" int perft_batch_noalloc(const perft_pos48 *d_pos, const uint8_t *dept
         }
         k_noalloc_group_ids<<<1, 1024, 0, R.st>>>(dDepths, n, depth, dIds, dGroupCount);
         k_init_roots<<<(cnt + 127) / 128, 128, 0, R.st>>>(d_pos->bb, dIds, cnt, L0.planes, L0.stride,
-                                                           L0.cnt, L0.root, depth, rootCounts, R.err);
+                                                           L0.cnt, L0.root, nullptr, depth, rootCounts, R.err);
         if (cudaGetLastError() != cudaSuccess) {
             rc = PERFT_ERR_CUDA;
             break;

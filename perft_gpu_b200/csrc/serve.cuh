@@ -486,7 +486,7 @@ int Server::admit()
             return PERFT_ERR_OUT_OF_MEMORY;
         }
         k_init_roots<<<(unsigned)((cnt + 127) / 128), 128, 0, st>>>(posBySlot, dSlots + i0, (u32)cnt, S->L.planes,
-                                                                     S->L.stride, S->L.cnt, S->L.root, depth,
+                                                                     S->L.stride, S->L.cnt, S->L.root, nullptr, depth,
                                                                      counts, dErr);
         launches++;
         if (depth >= 2) pools[depth].push_back(S);
