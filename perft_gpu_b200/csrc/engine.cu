@@ -185,71 +185,154 @@ __device__ __forceinline__ int block_excl_count(bool flag, int *sw, int &total)
 }
 
 // ------------------------------------------------------------------ scan
-// Exclusive scan of u32 move counts into u64 item offsets (n + 1 entries,
-// the last one the total), plus the first parent of every TILE_CAP tile.
-__global__ void __launch_bounds__(SCAN_NT) k_scan_reduce(const u32 *__restrict__ cnt, u64 n,
-                                                         u64 *__restrict__ bsum)
+// Exclusive scan of u32 move counts into u64 item offsets (the entry after
+// the last parent's is the total), plus the first parent of every tile.
+//
+// With COMPACT only the nodes that have items become parents: `live` lists
+// them in order and the offsets are theirs.  In merged and table levels
+// about 40% of the nodes have none (copies of another node, table hits);
+// left in place they held 40% of the tile kernel's parent slots, so a tile
+// took two staging rounds and generated moves with 40% of its threads idle.
+// Without COMPACT every node is a parent, at its own index.
+// Measured with compaction: depth 7 from a middlegame position 6.7 -> 6.05 ms,
+// the 4096-position batch 5% less; with results staged in shared memory the
+// offsets of 100 M nodes take 0.7 ms instead of 0.94.
+struct ScanSums {
+    u64 items, live;
+};
+
+// A chunk's items and live nodes in one word: at most SCAN_CHUNK nodes of at
+// most MAX_LEGAL_MOVES moves each.
+constexpr int SCAN_LIVE_SHIFT = 32;
+
+__device__ __forceinline__ u64 scan_pack(u32 c) { return (u64)c | ((u64)(c != 0) << SCAN_LIVE_SHIFT); }
+
+// Sums of chunk b into bsum[b].
+__device__ __forceinline__ void scan_reduce_chunk(const u32 *__restrict__ cnt, u64 n, u64 b, ScanSums *bsum, u64 *sw)
 {
-    __shared__ u64 sw[SCAN_NT / 32];
-    const u64 base = (u64)blockIdx.x * SCAN_CHUNK;
+    const u64 base = b * SCAN_CHUNK;
     u64 s = 0;
     for (int i = threadIdx.x; i < SCAN_CHUNK; i += SCAN_NT) {
         const u64 k = base + i;
-        if (k < n) s += cnt[k];
+        if (k < n) s += scan_pack(cnt[k]);
     }
     u64 total;
     block_excl_scan_u64<SCAN_NT>(s, sw, total);
-    if (threadIdx.x == 0) bsum[blockIdx.x] = total;
+    if (threadIdx.x == 0) bsum[b] = ScanSums{(u32)total, total >> SCAN_LIVE_SHIFT};
 }
 
-__global__ void __launch_bounds__(SCAN_TOP_NT) k_scan_top(u64 *__restrict__ bsum, u64 nb,
+// Exclusive scan of the chunk sums in place (one block); returns the totals.
+__device__ __forceinline__ ScanSums scan_top_block(ScanSums *bsum, u64 nb, u64 *sw)
+{
+    const u64 per = (nb + SCAN_TOP_NT - 1) / SCAN_TOP_NT;
+    const u64 b0 = min(per * threadIdx.x, nb), b1 = min(b0 + per, nb);
+    ScanSums s{0, 0}, total;
+    for (u64 i = b0; i < b1; i++) {
+        s.items += bsum[i].items;
+        s.live += bsum[i].live;
+    }
+    ScanSums run;
+    run.items = block_excl_scan_u64<SCAN_TOP_NT>(s.items, sw, total.items);
+    run.live = block_excl_scan_u64<SCAN_TOP_NT>(s.live, sw, total.live);
+    for (u64 i = b0; i < b1; i++) {
+        const ScanSums v = bsum[i];
+        bsum[i] = run;
+        run.items += v.items;
+        run.live += v.live;
+    }
+    return total;
+}
+
+// Marks the tiles whose first item belongs to parent `idx`, whose items are [run, run + c).
+__device__ __forceinline__ void scan_tiles(u32 *tileFirst, int capLog2, u64 run, u32 c, u64 idx)
+{
+    const u64 t0 = (run + (1ull << capLog2) - 1) >> capLog2;
+    const u64 t1 = (run + c - 1) >> capLog2;
+    for (u64 t = t0; t <= t1; t++) tileFirst[t] = (u32)idx;
+}
+
+// Offsets, parent list and tile index of chunk b.  The chunk's results are
+// placed in shared memory first, so that global writes are coalesced.
+struct ScanShared {
+    u32 c[SCAN_CHUNK];    // counts, then the parents' offsets within the chunk
+    uint16_t at[SCAN_CHUNK];  // the parents' places within the chunk
+    u64 sw[SCAN_NT / 32];
+};
+constexpr size_t SCAN_DYN_SMEM = sizeof(ScanShared);
+
+template <bool COMPACT>
+__device__ __forceinline__ void scan_apply_chunk(const u32 *__restrict__ cnt, u64 n, u64 b, const ScanSums *bsum,
+                                                 u64 *__restrict__ scan, u32 *__restrict__ live,
+                                                 u32 *__restrict__ tileFirst, int capLog2, ScanShared &S)
+{
+    const u64 base = b * SCAN_CHUNK;
+    for (int i = threadIdx.x; i < SCAN_CHUNK; i += SCAN_NT) {
+        const u64 k = base + i;
+        S.c[i] = k < n ? cnt[k] : 0u;
+    }
+    __syncthreads();
+    u32 c[SCAN_IPT];
+    u64 local = 0;
+#pragma unroll
+    for (int k = 0; k < SCAN_IPT; k++) {
+        c[k] = S.c[threadIdx.x * SCAN_IPT + k];
+        local += scan_pack(c[k]);
+    }
+    u64 total;
+    const u64 run0 = block_excl_scan_u64<SCAN_NT>(local, S.sw, total);  // (its barriers also end the reads of S.c)
+    const ScanSums B = bsum[b];
+    u32 run = (u32)run0;
+    u32 place = COMPACT ? (u32)(run0 >> SCAN_LIVE_SHIFT) : threadIdx.x * SCAN_IPT;
+    const u64 first = COMPACT ? B.live : base;
+#pragma unroll
+    for (int k = 0; k < SCAN_IPT; k++) {
+        if (!COMPACT || c[k]) {
+            S.c[place] = run;
+            if (COMPACT) S.at[place] = (uint16_t)(threadIdx.x * SCAN_IPT + k);
+            if (c[k]) scan_tiles(tileFirst, capLog2, B.items + run, c[k], first + place);
+            place++;
+        }
+        run += c[k];
+    }
+    __syncthreads();
+    const u32 m = COMPACT ? (u32)(total >> SCAN_LIVE_SHIFT) : (u32)min((u64)SCAN_CHUNK, n - base);
+    for (u32 i = threadIdx.x; i < m; i += SCAN_NT) {
+        scan[first + i] = B.items + S.c[i];
+        if (COMPACT) live[first + i] = (u32)(base + S.at[i]);
+    }
+    __syncthreads();
+}
+
+__global__ void __launch_bounds__(SCAN_NT) k_scan_reduce(const u32 *__restrict__ cnt, u64 n,
+                                                         ScanSums *__restrict__ bsum)
+{
+    __shared__ u64 sw[SCAN_NT / 32];
+    scan_reduce_chunk(cnt, n, blockIdx.x, bsum, sw);
+}
+
+// totalOut[0]: items, totalOut[1]: live nodes.
+__global__ void __launch_bounds__(SCAN_TOP_NT) k_scan_top(ScanSums *__restrict__ bsum, u64 nb,
                                                           u64 *__restrict__ totalOut)
 {
     __shared__ u64 sw[SCAN_TOP_NT / 32];
-    const u64 per = (nb + SCAN_TOP_NT - 1) / SCAN_TOP_NT;
-    const u64 b0 = per * threadIdx.x, b1 = min(b0 + per, nb);
-    u64 s = 0;
-    for (u64 i = b0; i < b1; i++) s += bsum[i];
-    u64 total;
-    u64 run = block_excl_scan_u64<SCAN_TOP_NT>(s, sw, total);
-    for (u64 i = b0; i < b1; i++) {
-        const u64 v = bsum[i];
-        bsum[i] = run;
-        run += v;
+    const ScanSums t = scan_top_block(bsum, nb, sw);
+    if (threadIdx.x == 0) {
+        totalOut[0] = t.items;
+        totalOut[1] = t.live;
     }
-    if (threadIdx.x == 0) *totalOut = total;
 }
 
+template <bool COMPACT>
 __global__ void __launch_bounds__(SCAN_NT) k_scan_apply(const u32 *__restrict__ cnt, u64 n,
-                                                        const u64 *__restrict__ bsum,
-                                                        u64 *__restrict__ scan,
-                                                        u32 *__restrict__ tileFirst, int capLog2)
+                                                        const ScanSums *__restrict__ bsum,
+                                                        const u64 *__restrict__ totals, u64 *__restrict__ scan,
+                                                        u32 *__restrict__ live, u32 *__restrict__ tileFirst,
+                                                        int capLog2)
 {
-    __shared__ u32 s[SCAN_CHUNK];
-    __shared__ u64 sw[SCAN_NT / 32];
-    const u64 base = (u64)blockIdx.x * SCAN_CHUNK;
-    for (int i = threadIdx.x; i < SCAN_CHUNK; i += SCAN_NT) {
-        const u64 k = base + i;
-        s[i] = k < n ? cnt[k] : 0u;
-    }
-    __syncthreads();
-    u64 local = 0;
-#pragma unroll
-    for (int k = 0; k < SCAN_IPT; k++) local += s[threadIdx.x * SCAN_IPT + k];
-    u64 total;
-    u64 run = bsum[blockIdx.x] + block_excl_scan_u64<SCAN_NT>(local, sw, total);
-    for (int k = 0; k < SCAN_IPT; k++) {
-        const u64 idx = base + (u64)threadIdx.x * SCAN_IPT + k;
-        if (idx >= n) break;
-        const u32 c = s[threadIdx.x * SCAN_IPT + k];
-        scan[idx] = run;
-        if (c) {
-            const u64 t0 = (run + (1ull << capLog2) - 1) >> capLog2;
-            const u64 t1 = (run + c - 1) >> capLog2;
-            for (u64 t = t0; t <= t1; t++) tileFirst[t] = (u32)idx;
-        }
-        run += c;
-    }
+    extern __shared__ __align__(16) unsigned char scanShared[];
+    ScanShared &S = *reinterpret_cast<ScanShared *>(scanShared);
+    if (blockIdx.x == 0 && threadIdx.x == 0) scan[COMPACT ? totals[1] : n] = totals[0];
+    scan_apply_chunk<COMPACT>(cnt, n, blockIdx.x, bsum, scan, live, tileFirst, capLog2, S);
 }
 
 // ----------------------------------------------------------------- roots
@@ -297,9 +380,10 @@ struct LevelDesc {
     unsigned long long *set;     // merged levels: the set's slots (transient), null when they do not fit
     u64 n;        // nodes: the previous ply's children, then the roots joining here
     u64 nChild;   // children written by the previous ply's tile kernel
+    u32 *live;  // merged levels: the nodes with items, in order (null: all nodes are parents)
     u64 *pscan;
     u32 *tileFirst;
-    u64 *bsum;
+    ScanSums *bsum;
     u64 total;
     int capLog2;  // tile size of this level's items
 };
@@ -308,6 +392,7 @@ struct TileParams {
     const u64 *ppl;   // parent planes, plane i at ppl + i * pstride
     u64 pstride;
     const u64 *pscan; // nParents + 1 item offsets
+    const u32 *live;  // node index of each parent; null: the parent's own index
     const u32 *proot;  // root id of each parent; null: sums go to the parent's own slot
     const unsigned long long *pweight;  // paths that reach each parent; null: one each
     u64 nParents;
@@ -389,86 +474,98 @@ __global__ void __launch_bounds__(SCAN_NT) k_dd_scan_reduce(DevPlan *plan, int l
     __shared__ u64 sw[SCAN_NT / 32];
     const LevelDesc &L = plan->lv[lv];
     const u64 n = L.n, nb = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
-    for (u64 b = blockIdx.x; b < nb; b += gridDim.x) {
-        const u64 base = b * SCAN_CHUNK;
-        u64 s = 0;
-        for (int i = threadIdx.x; i < SCAN_CHUNK; i += SCAN_NT) {
-            const u64 k = base + i;
-            if (k < n) s += L.cnt[k];
-        }
-        u64 total;
-        block_excl_scan_u64<SCAN_NT>(s, sw, total);
-        if (threadIdx.x == 0) L.bsum[b] = total;
-    }
+    for (u64 b = blockIdx.x; b < nb; b += gridDim.x) scan_reduce_chunk(L.cnt, n, b, L.bsum, sw);
 }
 
-__device__ void dd_plan_level(DevPlan *plan, int lv, int last, u64 total);
+__device__ void dd_plan_level(DevPlan *plan, int lv, int last, ScanSums total);
 
 __global__ void __launch_bounds__(SCAN_TOP_NT) k_dd_scan_top(DevPlan *plan, int lv, int last)
 {
     __shared__ u64 sw[SCAN_TOP_NT / 32];
     LevelDesc &L = plan->lv[lv];
-    const u64 n = L.n, nb = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
-    const u64 per = (nb + SCAN_TOP_NT - 1) / SCAN_TOP_NT;
-    const u64 b0 = per * threadIdx.x, b1 = min(b0 + per, nb);
-    u64 s = 0;
-    for (u64 i = b0; i < b1; i++) s += L.bsum[i];
-    u64 total;
-    u64 run = block_excl_scan_u64<SCAN_TOP_NT>(s, sw, total);
-    for (u64 i = b0; i < b1; i++) {
-        const u64 v = L.bsum[i];
-        L.bsum[i] = run;
-        run += v;
-    }
+    const ScanSums total = scan_top_block(L.bsum, (L.n + SCAN_CHUNK - 1) / SCAN_CHUNK, sw);
     if (threadIdx.x == 0) dd_plan_level(plan, lv, last, total);
 }
 
 // Whole-level scan in one block: the total, the tile size and the next level
-// (dd_plan_level), then the offsets and tile index, 1024 nodes per pass.
+// (dd_plan_level), then the offsets and tile index, 4096 nodes per pass.
 // Used for levels predicted small, where three launches (each with its own
-// latency) would cost more than the work; correct for any size.
+// latency) would cost more than the work; correct for any size.  A level of
+// one pass takes its total from the pass's own scan.
 __global__ void __launch_bounds__(1024) k_dd_scan_small(DevPlan *plan, int lv, int last)
 {
+    constexpr int IPT = 4, PASS = 1024 * IPT;
     __shared__ u64 sw[32];
     __shared__ int sCap;
     LevelDesc &L = plan->lv[lv];
     const u64 n = L.n;
-    u64 s = 0;
-    for (u64 i = threadIdx.x; i < n; i += 1024) s += L.cnt[i];
-    u64 total;
-    block_excl_scan_u64<1024>(s, sw, total);
-    if (threadIdx.x == 0) {
-        dd_plan_level(plan, lv, last, total);
-        sCap = L.capLog2;
+    const u32 *cnt = L.cnt;
+    u32 c[IPT];
+    u64 x, tot;  // this thread's place in the pass's scan, and the pass's sums
+    auto scan_pass = [&](u64 c0) {
+        u64 local = 0;
+#pragma unroll
+        for (int k = 0; k < IPT; k++) {
+            const u64 i = c0 + (u64)threadIdx.x * IPT + k;
+            c[k] = i < n ? cnt[i] : 0u;
+            local += scan_pack(c[k]);
+        }
+        x = block_excl_scan_u64<1024>(local, sw, tot);
+    };
+    if (n > PASS) {
+        u64 s = 0, a = 0;
+        for (u64 i = threadIdx.x; i < n; i += 1024) {
+            const u32 v = cnt[i];
+            s += v;
+            a += v != 0;
+        }
+        ScanSums total;
+        block_excl_scan_u64<1024>(s, sw, total.items);
+        block_excl_scan_u64<1024>(a, sw, total.live);
+        if (threadIdx.x == 0) dd_plan_level(plan, lv, last, total);
+        scan_pass(0);
+    } else {
+        scan_pass(0);
+        if (threadIdx.x == 0) dd_plan_level(plan, lv, last, ScanSums{(u32)tot, tot >> SCAN_LIVE_SHIFT});
     }
+    if (threadIdx.x == 0) sCap = L.capLog2;
     __syncthreads();
     const int cl = sCap;
-    u64 base = 0;
-    for (u64 c0 = 0; c0 < n; c0 += 1024) {
-        const u64 i = c0 + threadIdx.x;
-        const u32 c = i < n ? L.cnt[i] : 0u;
-        u64 tot;
-        const u64 run = base + block_excl_scan_u64<1024>(c, sw, tot);
-        if (i < n) {
-            L.pscan[i] = run;
-            if (c) {
-                const u64 t0 = (run + (1ull << cl) - 1) >> cl;
-                const u64 t1 = (run + c - 1) >> cl;
-                for (u64 t = t0; t <= t1; t++) L.tileFirst[t] = (u32)i;
+    u64 *pscan = L.pscan;
+    u32 *live = L.live;
+    u32 *tileFirst = L.tileFirst;
+    u64 base = 0, place0 = 0;
+    for (u64 c0 = 0;;) {
+        u64 run = base + (u32)x, place = place0 + (x >> SCAN_LIVE_SHIFT);
+#pragma unroll
+        for (int k = 0; k < IPT; k++) {
+            const u64 i = c0 + (u64)threadIdx.x * IPT + k;
+            const u64 at = live ? place : i;
+            if (live ? c[k] != 0 : i < n) {
+                pscan[at] = run;
+                if (live) live[at] = (u32)i;
+                if (c[k]) scan_tiles(tileFirst, cl, run, c[k], at);
             }
+            run += c[k];
+            place += c[k] != 0;
         }
-        base += tot;
+        base += (u32)tot;
+        place0 += tot >> SCAN_LIVE_SHIFT;
+        c0 += PASS;
+        if (c0 >= n) break;
+        scan_pass(c0);
     }
 }
 
 // Top-of-scan bookkeeping of a device-driven level (one thread): the level's
 // total and tile size, then the next level's buffers from the plan's bump
 // allocator (children plus the roots joining there).
-__device__ void dd_plan_level(DevPlan *plan, int lv, int last, u64 total)
+__device__ void dd_plan_level(DevPlan *plan, int lv, int last, ScanSums sums)
 {
     LevelDesc &L = plan->lv[lv];
-    const u64 n = L.n;
-    if (n) L.pscan[n] = total;
+    const u64 total = sums.items;
+    const u64 nParents = L.live ? sums.live : L.n;
+    if (L.n) L.pscan[nParents] = total;
     L.total = plan->overflow ? 0 : total;
     int cap = plan->capMax[lv] ? plan->capMax[lv] : TILE_CAP_LOG2;
     while (cap > TILE_MIN_LOG2 && (total >> cap) < plan->tileTarget) cap--;
@@ -480,7 +577,8 @@ __device__ void dd_plan_level(DevPlan *plan, int lv, int last, u64 total)
     T.pscan = L.pscan;
     T.proot = L.root;
     T.pweight = L.weight;
-    T.nParents = L.n;
+    T.live = L.live;
+    T.nParents = nParents;
     T.tileFirst = L.tileFirst;
     T.itemBase = 0;
     T.itemEnd = L.total;
@@ -496,9 +594,10 @@ __device__ void dd_plan_level(DevPlan *plan, int lv, int last, u64 total)
     C.cnt = (u32 *)dd_take(plan, 4 * C.stride);
     C.root = (u32 *)dd_take(plan, 4 * C.stride);
     C.weight = plan->weighted ? (unsigned long long *)dd_take(plan, 8 * C.stride) : nullptr;
+    C.live = plan->mergeLv[lv + 1] ? (u32 *)dd_take(plan, 4 * C.stride) : nullptr;
     C.pscan = (u64 *)dd_take(plan, 8 * (m + 1));
     C.tileFirst = (u32 *)dd_take(plan, 4 * ((m * MAX_LEGAL_MOVES) / MAX_TILES_PER_NODE_DIV + 2));
-    C.bsum = (u64 *)dd_take(plan, 8 * ((m + SCAN_CHUNK - 1) / SCAN_CHUNK + 1));
+    C.bsum = (ScanSums *)dd_take(plan, sizeof(ScanSums) * ((m + SCAN_CHUNK - 1) / SCAN_CHUNK + 1));
     if (plan->overflow) {
         C.n = 0;
         L.total = 0;  // nothing is expanded into a level that does not exist
@@ -518,39 +617,15 @@ __device__ void dd_plan_level(DevPlan *plan, int lv, int last, u64 total)
     T.cweight = C.weight;
 }
 
+template <bool COMPACT>
 __global__ void __launch_bounds__(SCAN_NT) k_dd_scan_apply(DevPlan *plan, int lv)
 {
-    __shared__ u32 s[SCAN_CHUNK];
-    __shared__ u64 sw[SCAN_NT / 32];
+    extern __shared__ __align__(16) unsigned char scanShared[];
+    ScanShared &S = *reinterpret_cast<ScanShared *>(scanShared);
     const LevelDesc &L = plan->lv[lv];
     const u64 n = L.n, nb = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
-    for (u64 b = blockIdx.x; b < nb; b += gridDim.x) {
-        const u64 base = b * SCAN_CHUNK;
-        for (int i = threadIdx.x; i < SCAN_CHUNK; i += SCAN_NT) {
-            const u64 k = base + i;
-            s[i] = k < n ? L.cnt[k] : 0u;
-        }
-        __syncthreads();
-        u64 local = 0;
-#pragma unroll
-        for (int k = 0; k < SCAN_IPT; k++) local += s[threadIdx.x * SCAN_IPT + k];
-        u64 total;
-        u64 run = L.bsum[b] + block_excl_scan_u64<SCAN_NT>(local, sw, total);
-        for (int k = 0; k < SCAN_IPT; k++) {
-            const u64 idx = base + (u64)threadIdx.x * SCAN_IPT + k;
-            if (idx >= n) break;
-            const u32 c = s[threadIdx.x * SCAN_IPT + k];
-            L.pscan[idx] = run;
-            if (c) {
-                const int cl = L.capLog2;
-                const u64 t0 = (run + (1ull << cl) - 1) >> cl;
-                const u64 t1 = (run + c - 1) >> cl;
-                for (u64 t = t0; t <= t1; t++) L.tileFirst[t] = (u32)idx;
-            }
-            run += c;
-        }
-        __syncthreads();
-    }
+    for (u64 b = blockIdx.x; b < nb; b += gridDim.x)
+        scan_apply_chunk<COMPACT>(L.cnt, n, b, L.bsum, L.pscan, L.live, L.tileFirst, L.capLog2, S);
 }
 
 // Roots joining level lv of a device-driven run: written behind the
@@ -783,9 +858,10 @@ __global__ void __launch_bounds__(TILE_NT, TILE_MINB) k_tile(const TileParams Pi
             if (valid) {
                 qEnd = P.pscan[q + 1];
                 if (TRACK) sqEnd[tid] = qEnd;
+                const u64 node = P.live ? P.live[q] : q;
                 // mirrored staging: the per-parent flips here replace six
                 // byte swaps per child in make-move
-                const Board lb = level_get(P.ppl, P.pstride, q);
+                const Board lb = level_get(P.ppl, P.pstride, node);
                 const Board pb = PG_MIRRORED_STAGE ? flip_board(lb) : lb;
                 sb[0][tid] = pb.mine;
                 sb[1][tid] = pb.pawns;
@@ -797,8 +873,8 @@ __global__ void __launch_bounds__(TILE_NT, TILE_MINB) k_tile(const TileParams Pi
                     skO[tid] = (uint8_t)ctz(pb.kings & ~pb.mine);
                     skS[tid] = (uint8_t)ctz(pb.kings & pb.mine);
                 }
-                sroot[tid] = P.proot ? P.proot[q] : (u32)q;  // no root array: account to the parent itself
-                if (!TRACK) sweight[tid] = P.pweight ? P.pweight[q] : 1ull;
+                sroot[tid] = P.proot ? P.proot[node] : (u32)node;  // no root array: account to the parent itself
+                if (!TRACK) sweight[tid] = P.pweight ? P.pweight[node] : 1ull;
             }
             const u64 sBeg = max(P.pscan[p], iBeg);
             const u64 sEnd = min(P.pscan[p + nP], iEnd);
@@ -1472,6 +1548,14 @@ private:
         tunedMaxR = 3;
     }
 
+    // A scanned level: its parents, their items and the tiles of those.
+    struct ParentIndex {
+        u64 *pscan = nullptr;
+        u32 *live = nullptr;  // null: every node is a parent
+        u32 *tileFirst = nullptr;
+        u64 nParents = 0, total = 0;
+        int capLog2 = TILE_CAP_LOG2;
+    };
     void *alloc(u64 bytes)
     {
         const u64 a = (arenaTop + 255) & ~255ULL;
@@ -1482,9 +1566,9 @@ private:
     }
     u64 arena_free() const { return arenaCap > arenaTop ? arenaCap - arenaTop : 0; }
     bool alloc_level(DeviceLevel &L, u64 n, bool weighted = false);
-    int scan(const u32 *cnt, u64 n, int remaining, u64 *&scanOut, u32 *&tileFirst, u64 &total, int &capLog2);
-    int launch_tile(int mode, int remaining, const DeviceLevel &parents, const u64 *pscan, const u32 *tileFirst,
-                    int capLog2, u64 itemBase, u64 itemEnd, DeviceLevel *children, unsigned long long *rootCounts);
+    int scan(const u32 *cnt, u64 n, int remaining, bool compact, ParentIndex &out);
+    int launch_tile(int mode, int remaining, const DeviceLevel &parents, const ParentIndex &ix, u64 itemBase,
+                    u64 itemEnd, DeviceLevel *children, unsigned long long *rootCounts);
     // Roots that join the search at a given remaining depth: their ids (device
     // array) and count, indexed by depth.  A root of depth d enters the level
     // whose nodes have d plies left, behind that level's children.
@@ -1621,6 +1705,16 @@ int occupancy_grid(int nsm)
     return perSm * nsm;
 }
 
+// Allows the scan's dynamic shared memory (just above 48 KB) on this device.
+int scan_setup()
+{
+    for (auto fn : {(const void *)k_scan_apply<true>, (const void *)k_scan_apply<false>,
+                    (const void *)k_dd_scan_apply<true>, (const void *)k_dd_scan_apply<false>})
+        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SCAN_DYN_SMEM) != cudaSuccess)
+            return PERFT_ERR_CUDA;
+    return PERFT_OK;
+}
+
 template <int MODE>
 void launch_tile_variant(int sv, int grid, cudaStream_t st, const TileParams &P)
 {
@@ -1660,7 +1754,7 @@ const char *slider_name(int sv)
 
 int Engine::init(const perft_config &cfg)
 {
-    int ndev = 0;
+    int ndev = 0, rc0 = PERFT_OK;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev <= 0) return PERFT_ERR_NO_DEVICE;
     if (cfg.device < 0 || cfg.device >= ndev) return PERFT_ERR_INVALID_ARG;
     device = cfg.device;
@@ -1746,6 +1840,7 @@ int Engine::init(const perft_config &cfg)
                     (const void *)k_tile<MODE_EXPAND, SV_KOGGE, false, DD_SHARED>,
                     (const void *)k_tile<MODE_EXPAND, SV_KOGGE_SPLIT, false, DD_SHARED>})
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TILE_DYN_SMEM);
+    if ((rc0 = scan_setup()) != PERFT_OK) return rc0;
     ddGridScan = 4 * nsm;
     {
         ENG_TRY(cudaMalloc(&dSmall, sizeof(SmallState)));
@@ -1851,45 +1946,54 @@ int Engine::merge_level(const Joiners &J, const DeviceLevel &C, int remaining)
 
 // `remaining`: remaining depth of the level scanned; its items go to the
 // count-only ply when it is 2, to an interior ply otherwise.
-int Engine::scan(const u32 *cnt, u64 n, int remaining, u64 *&scanOut, u32 *&tileFirst, u64 &total, int &capLog2)
+int Engine::scan(const u32 *cnt, u64 n, int remaining, bool compact, ParentIndex &ix)
 {
     const u64 nb = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
     const u64 maxTiles = (n * MAX_LEGAL_MOVES) / MAX_TILES_PER_NODE_DIV + 2;
-    scanOut = (u64 *)alloc(8 * (n + 1));
-    tileFirst = (u32 *)alloc(4 * maxTiles);
-    u64 *bsum = (u64 *)alloc(8 * (nb + 1));
-    if (!scanOut || !tileFirst || !bsum) return PERFT_ERR_OUT_OF_MEMORY;
+    ix.pscan = (u64 *)alloc(8 * (n + 1));
+    ix.live = compact ? (u32 *)alloc(4 * n) : nullptr;
+    ix.tileFirst = (u32 *)alloc(4 * maxTiles);
+    ScanSums *bsum = (ScanSums *)alloc(sizeof(ScanSums) * (nb + 1));
+    if (!ix.pscan || !ix.tileFirst || !bsum || (compact && !ix.live)) return PERFT_ERR_OUT_OF_MEMORY;
+    u64 *totals = (u64 *)(bsum + nb);
     k_scan_reduce<<<(unsigned)nb, SCAN_NT, 0, stream>>>(cnt, n, bsum);
-    k_scan_top<<<1, SCAN_TOP_NT, 0, stream>>>(bsum, nb, scanOut + n);
+    k_scan_top<<<1, SCAN_TOP_NT, 0, stream>>>(bsum, nb, totals);
     ENG_TRY(cudaGetLastError());
-    ENG_TRY(cudaMemcpyAsync(hPinned, scanOut + n, 8, cudaMemcpyDeviceToHost, stream));
+    ENG_TRY(cudaMemcpyAsync(hPinned, totals, 16, cudaMemcpyDeviceToHost, stream));
     ENG_TRY(cudaStreamSynchronize(stream));
-    total = hPinned[0];
+    ix.total = hPinned[0];
+    ix.nParents = compact ? hPinned[1] : n;
     // tile size: the tuned largest tile for this ply, made smaller while some
     // resident CTA would get no second tile
     const int mode = remaining == 2 ? MODE_LEAF : MODE_EXPAND;
     const TuneCfg &tc = cfg_for(mode, remaining);
-    capLog2 = tc.cap;
-    while (capLog2 > TILE_MIN_LOG2 && (total >> capLog2) < 2ull * grid_for(mode, tc)) capLog2--;
-    k_scan_apply<<<(unsigned)nb, SCAN_NT, 0, stream>>>(cnt, n, bsum, scanOut, tileFirst, capLog2);
+    ix.capLog2 = tc.cap;
+    while (ix.capLog2 > TILE_MIN_LOG2 && (ix.total >> ix.capLog2) < 2ull * grid_for(mode, tc)) ix.capLog2--;
+    if (compact)
+        k_scan_apply<true><<<(unsigned)nb, SCAN_NT, SCAN_DYN_SMEM, stream>>>(cnt, n, bsum, totals, ix.pscan, ix.live,
+                                                                            ix.tileFirst, ix.capLog2);
+    else
+        k_scan_apply<false><<<(unsigned)nb, SCAN_NT, SCAN_DYN_SMEM, stream>>>(cnt, n, bsum, totals, ix.pscan, nullptr,
+                                                                             ix.tileFirst, ix.capLog2);
     stats.other_launches += 3;
     ENG_TRY(cudaGetLastError());
     return PERFT_OK;
 }
 
-int Engine::launch_tile(int mode, int remaining, const DeviceLevel &parents, const u64 *pscan, const u32 *tileFirst,
-                        int capLog2, u64 itemBase, u64 itemEnd, DeviceLevel *children,
-                        unsigned long long *rootCounts)
+int Engine::launch_tile(int mode, int remaining, const DeviceLevel &parents, const ParentIndex &ix, u64 itemBase,
+                        u64 itemEnd, DeviceLevel *children, unsigned long long *rootCounts)
 {
+    const int capLog2 = ix.capLog2;
     TileParams P;
     memset(&P, 0, sizeof P);
     P.ppl = parents.planes;
     P.pstride = parents.stride;
-    P.pscan = pscan;
+    P.pscan = ix.pscan;
+    P.live = ix.live;
     P.proot = parents.root;
     P.pweight = parents.weight;
-    P.nParents = parents.n;
-    P.tileFirst = tileFirst;
+    P.nParents = ix.nParents;
+    P.tileFirst = ix.tileFirst;
     P.itemBase = itemBase;
     P.itemEnd = itemEnd;
     P.capLog2 = capLog2;
@@ -1919,13 +2023,13 @@ int Engine::launch_tile(int mode, int remaining, const DeviceLevel &parents, con
     ENG_TRY(cudaEventElapsedTime(&ms, ev0, ev1));
     if (trace)
         fprintf(stderr, "perft-trace %s sv=%s parents=%llu items=%llu..%llu grid=%d ms=%.4f\n",
-                mode == MODE_LEAF ? "leaf" : "expand", slider_name(sv), (unsigned long long)parents.n,
+                mode == MODE_LEAF ? "leaf" : "expand", slider_name(sv), (unsigned long long)ix.nParents,
                 (unsigned long long)itemBase, (unsigned long long)itemEnd, grid, ms);
     if (tuning) tuneAccMs[mode][mode == MODE_LEAF ? 2 : std::min(remaining, (int)TUNE_MAX_R)] += ms;
     if (mode == MODE_LEAF) {
         stats.leaf_launches++;
         stats.leaf_items += itemEnd - itemBase;
-        stats.leaf_parents += parents.n;
+        stats.leaf_parents += ix.nParents;
         stats.leaf_ms += ms;
     } else {
         stats.expand_launches++;
@@ -1958,14 +2062,13 @@ int Engine::process_level(const DeviceLevel &L, int remaining, unsigned long lon
     const u32 nJoin = (join && remaining - 1 >= 2) ? join->n[remaining - 1] : 0;
     if (L.n == 0 && nJoin == 0) return PERFT_OK;
     const u64 mark = arenaTop;
-    u64 *pscan = nullptr;
-    u32 *tileFirst = nullptr;
-    u64 total = 0;
-    int capLog2 = TILE_CAP_LOG2;
-    int rc = L.n ? scan(L.cnt, L.n, remaining, pscan, tileFirst, total, capLog2) : PERFT_OK;
+    ParentIndex ix;
+    const bool merged = L.weight && join && join->maxDepth >= remaining + MERGE_MIN_PLIES;
+    int rc = L.n ? scan(L.cnt, L.n, remaining, merged, ix) : PERFT_OK;
     if (rc != PERFT_OK) return rc;
+    const u64 total = ix.total;
     if (remaining == 2) {
-        if (total) rc = launch_tile(MODE_LEAF, 2, L, pscan, tileFirst, capLog2, 0, total, nullptr, rootCounts);
+        if (total) rc = launch_tile(MODE_LEAF, 2, L, ix, 0, total, nullptr, rootCounts);
         arenaTop = mark;
         return rc;
     }
@@ -1992,7 +2095,7 @@ int Engine::process_level(const DeviceLevel &L, int remaining, unsigned long lon
         DeviceLevel C;
         if (!alloc_level(C, (hi - lo) + (last ? nJoin : 0), weighted)) return PERFT_ERR_OUT_OF_MEMORY;
         if (hi > lo) {
-            rc = launch_tile(MODE_EXPAND, remaining, L, pscan, tileFirst, capLog2, lo, hi, &C, nullptr);
+            rc = launch_tile(MODE_EXPAND, remaining, L, ix, lo, hi, &C, nullptr);
             if (rc != PERFT_OK) return rc;
         }
         if (last && nJoin) {
@@ -2220,17 +2323,15 @@ int Engine::process_level_tt(const DeviceLevel &L, int remaining, unsigned long 
     ENG_TRY(cudaGetLastError());
     arenaTop = mark;  // the de-duplication set is no longer needed
 
-    u64 *pscan = nullptr;
-    u32 *tileFirst = nullptr;
-    u64 total = 0;
-    int capLog2 = TILE_CAP_LOG2;
-    int rc = scan(L.cnt, L.n, remaining, pscan, tileFirst, total, capLog2);
+    ParentIndex ix;
+    int rc = scan(L.cnt, L.n, remaining, true, ix);
     if (rc != PERFT_OK) return rc;
+    const u64 total = ix.total;
     DeviceLevel self = L;
     self.root = nullptr;  // tile sums and child links point at the parent itself
     if (total > 0) {
         if (remaining == 2) {
-            rc = launch_tile(MODE_LEAF, 2, self, pscan, tileFirst, capLog2, 0, total, nullptr, L.acc);
+            rc = launch_tile(MODE_LEAF, 2, self, ix, 0, total, nullptr, L.acc);
             if (rc != PERFT_OK) return rc;
         } else {
             const u64 slack = std::min<u64>(64ull << 20, arenaCap / 16);
@@ -2245,7 +2346,7 @@ int Engine::process_level_tt(const DeviceLevel &L, int remaining, unsigned long 
                 const u64 cm = arenaTop;
                 DeviceLevel C;
                 if (!alloc_level_tt(C, hi - lo)) return PERFT_ERR_OUT_OF_MEMORY;
-                rc = launch_tile(MODE_EXPAND, remaining, self, pscan, tileFirst, capLog2, lo, hi, &C, nullptr);
+                rc = launch_tile(MODE_EXPAND, remaining, self, ix, lo, hi, &C, nullptr);
                 if (rc != PERFT_OK) return rc;
                 rc = process_level_tt(C, remaining - 1, L.acc, nullptr);
                 if (rc != PERFT_OK) return rc;
@@ -2327,7 +2428,7 @@ int Engine::build_dd(DDGraph &G)
     L0.weight = merge ? (unsigned long long *)place(8 * L0.stride) : nullptr;
     L0.pscan = (u64 *)place(8 * (n0 + 1));
     L0.tileFirst = (u32 *)place(4 * ((n0 * MAX_LEGAL_MOVES) / MAX_TILES_PER_NODE_DIV + 2));
-    L0.bsum = (u64 *)place(8 * ((n0 + SCAN_CHUNK - 1) / SCAN_CHUNK + 1));
+    L0.bsum = (ScanSums *)place(sizeof(ScanSums) * ((n0 + SCAN_CHUNK - 1) / SCAN_CHUNK + 1));
     // scratch level for the roots of depth 0 and 1 (counts only)
     const u64 nShallow = std::max<u64>(nAt[0], nAt[1]);
     const u64 sStride = (nShallow + 31) & ~31ULL;
@@ -2416,7 +2517,8 @@ int Engine::build_dd(DDGraph &G)
             k_dd_scan_reduce<<<sg, SCAN_NT, 0, stream>>>(dPlan, lv);
             G.otherLaunches += 3;
             k_dd_scan_top<<<1, SCAN_TOP_NT, 0, stream>>>(dPlan, lv, last);
-            k_dd_scan_apply<<<sg, SCAN_NT, 0, stream>>>(dPlan, lv);
+            if (G.hTemplate->mergeLv[lv]) k_dd_scan_apply<true><<<sg, SCAN_NT, SCAN_DYN_SMEM, stream>>>(dPlan, lv);
+            else k_dd_scan_apply<false><<<sg, SCAN_NT, SCAN_DYN_SMEM, stream>>>(dPlan, lv);
         }
         // (the scan reset the tile cursor)
         // Large plies read their launch parameters (completed by the scan)
@@ -2460,7 +2562,7 @@ int Engine::build_dd(DDGraph &G)
     cudaMemcpyAsync(&G.hFlags[1], dErr, 4, cudaMemcpyDeviceToHost, stream);
     if (d >= 2) {
         cudaMemcpyAsync(&G.hFlags[2], &dPlan->lv[d - 2].total, 8, cudaMemcpyDeviceToHost, stream);
-        cudaMemcpyAsync(&G.hFlags[3], &dPlan->lv[d - 2].n, 8, cudaMemcpyDeviceToHost, stream);
+        cudaMemcpyAsync(&G.hFlags[3], &dPlan->tp[d - 2].nParents, 8, cudaMemcpyDeviceToHost, stream);
     }
     const cudaError_t ce = cudaStreamEndCapture(stream, &G.graph);
     if (ce != cudaSuccess) {
@@ -2518,7 +2620,7 @@ int Engine::run_dd(const u64 *dPos, const uint8_t *depths, u32 n, u64 *dOut, boo
                 nodes *= 32.0;
                 if (mergeEnabled && k >= MERGE_MIN_PLIES) nodes *= MERGE_KEPT;
             }
-            est += sum * (mergeEnabled && d - 2 >= MERGE_MIN_PLIES ? 88.0 : 72.0);
+            est += sum * (mergeEnabled && d - 2 >= MERGE_MIN_PLIES ? 92.0 : 72.0);
         }
         if (est > 0.85 * (double)arena_free()) return PERFT_OK;
         if (est > ddMaxBytes) return PERFT_OK;
@@ -3042,6 +3144,7 @@ int noalloc_setup(int dev)
     D.scratch = (unsigned char *)p;
     D.gridLeaf = occupancy_grid<MODE_LEAF, SV_KOGGE>(prop.multiProcessorCount);
     D.gridExpand = occupancy_grid<MODE_EXPAND, SV_KOGGE>(prop.multiProcessorCount);
+    if (scan_setup() != PERFT_OK) return PERFT_ERR_CUDA;
     D.ready = true;
     return PERFT_OK;
 }
@@ -3085,11 +3188,15 @@ struct NoallocRun {
         const u64 maxTiles = (n * MAX_LEGAL_MOVES + TILE_CAP - 1) / TILE_CAP + 1;
         scanOut = (u64 *)take(8 * (n + 1));
         tileFirst = (u32 *)take(4 * maxTiles);
-        u64 *bsum = (u64 *)take(8 * (nb + 1));
+        const u64 mark = top;
+        ScanSums *bsum = (ScanSums *)take(sizeof(ScanSums) * (nb + 1));
         if (!scanOut || !tileFirst || !bsum) return PERFT_ERR_OUT_OF_MEMORY;
+        top = mark;  // the block sums are done with before the next level is written (stream order)
+        u64 *totals = (u64 *)(bsum + nb);
         k_scan_reduce<<<(unsigned)nb, SCAN_NT, 0, st>>>(cnt, n, bsum);
-        k_scan_top<<<1, SCAN_TOP_NT, 0, st>>>(bsum, nb, scanOut + n);
-        k_scan_apply<<<(unsigned)nb, SCAN_NT, 0, st>>>(cnt, n, bsum, scanOut, tileFirst, TILE_CAP_LOG2);
+        k_scan_top<<<1, SCAN_TOP_NT, 0, st>>>(bsum, nb, totals);
+        k_scan_apply<false><<<(unsigned)nb, SCAN_NT, SCAN_DYN_SMEM, st>>>(cnt, n, bsum, totals, scanOut, nullptr,
+                                                                        tileFirst, TILE_CAP_LOG2);
         if (cudaGetLastError() != cudaSuccess) return PERFT_ERR_CUDA;
         return read_u64(scanOut + n, total);
     }
@@ -3165,12 +3272,13 @@ extern "C" int perft_batch_noalloc(const perft_pos48 *d_pos, const uint8_t *dept
     R.st = (cudaStream_t)stream;
     R.gridLeaf = g_noallocDev[dev].gridLeaf;
     R.gridExpand = g_noallocDev[dev].gridExpand;
-    R.counter = (u32 *)R.take(4);
-    R.err = (u32 *)R.take(4);
+    u32 *words = (u32 *)R.take(12);  // tile cursor, error flags, group size
+    R.counter = words;
+    R.err = words + 1;
     u32 *dIds = (u32 *)R.take(4ull * n);
     uint8_t *dDepths = (uint8_t *)R.take(n);
-    u32 *dGroupCount = (u32 *)R.take(4);
-    if (!R.counter || !R.err || !dIds || !dDepths || !dGroupCount) return PERFT_ERR_OUT_OF_MEMORY;
+    u32 *dGroupCount = words + 2;
+    if (!words || !dIds || !dDepths) return PERFT_ERR_OUT_OF_MEMORY;
 
     // From the first queued operation on, every return goes through the
     // stream synchronisation at the end, so the call never returns with work

@@ -586,14 +586,16 @@ int Server::scan_level(ServeLevel &S)
     S.pscan = (u64 *)take(8 * (n + 1), S.mem);
     S.tileFirst = (u32 *)take(4 * maxTiles, S.mem);
     std::vector<std::pair<u64, u64>> tmp;
-    u64 *bsum = (u64 *)take(8 * (nb + 1), tmp);
+    ScanSums *bsum = (ScanSums *)take(sizeof(ScanSums) * (nb + 1), tmp);
     if (!S.pscan || !S.tileFirst || !bsum) {
         give_back(tmp);
         return PERFT_ERR_OUT_OF_MEMORY;
     }
     k_scan_reduce<<<(unsigned)nb, SCAN_NT, 0, st>>>(S.L.cnt, n, bsum);
-    k_scan_top<<<1, SCAN_TOP_NT, 0, st>>>(bsum, nb, S.pscan + n);
-    k_scan_apply<<<(unsigned)nb, SCAN_NT, 0, st>>>(S.L.cnt, n, bsum, S.pscan, S.tileFirst, TILE_CAP_LOG2);
+    u64 *totals = (u64 *)(bsum + nb);
+    k_scan_top<<<1, SCAN_TOP_NT, 0, st>>>(bsum, nb, totals);
+    k_scan_apply<false><<<(unsigned)nb, SCAN_NT, SCAN_DYN_SMEM, st>>>(S.L.cnt, n, bsum, totals, S.pscan, nullptr,
+                                                                    S.tileFirst, TILE_CAP_LOG2);
     launches += 3;
     // a table level's nodes leave the pending count in its finish pass
     if (!S.tt) {
