@@ -165,6 +165,20 @@ __device__ __forceinline__ u64 block_excl_scan_u64(u64 v, u64 *sw, u64 &total)
     return warpOff + x - v;
 }
 
+// Adds every thread's v to a statistics counter: one atomic per block.  Every
+// thread of the block must call it.
+__device__ __forceinline__ void block_add_stat(unsigned long long *ctr, u32 v)
+{
+    __shared__ u32 sCount;
+    if (threadIdx.x == 0) sCount = 0;
+    __syncthreads();
+    const u32 sum = __reduce_add_sync(0xffffffffu, v);
+    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(&sCount, sum);
+    __syncthreads();
+    if (threadIdx.x == 0 && sCount) atomicAdd(ctr, (unsigned long long)sCount);
+    __syncthreads();
+}
+
 // Exclusive count of set flags over the block; total returned in *total.
 template <int NT>
 __device__ __forceinline__ int block_excl_count(bool flag, int *sw, int &total)
@@ -687,7 +701,18 @@ struct MergeLevel {
     MergeSeg *segs;
     const uint8_t *rootDepth;
     int remaining;  // plies left below the level
+    // linked levels (below): each node's owner, and the subtree sums to clear
+    u32 *alias;
+    unsigned long long *acc;
+    unsigned long long *merged;  // statistics: nodes merged
 };
+
+// Owner links.  Levels whose subtree sums flow up node by node (with a
+// transposition table, or with related roots) are merged over all roots: a
+// copy remembers its owner in `alias` and takes the owner's sum when the
+// level is finished (k_tt_finish), instead of handing over its weight.
+constexpr u32 ALIAS_HIT = 0xFFFFFFFFu;     // final value in acc: from the table, or no moves
+constexpr u32 ALIAS_NOSLOT = 0xFFFFFFFEu;  // searched by itself (no slot found in the set)
 
 __device__ __forceinline__ u64 board_hash(const Board &b)
 {
@@ -715,49 +740,64 @@ __device__ __forceinline__ void merge_prepare(const MergeLevel &M)
     }
 }
 
+template <bool LINKED>
 __device__ __forceinline__ void merge_nodes(const MergeLevel &M)
 {
     const u64 t0 = (u64)blockIdx.x * blockDim.x + threadIdx.x, step = (u64)gridDim.x * blockDim.x;
+    u32 nMerged = 0;
     for (u64 i = t0; i < M.n; i += step) {
-        if (M.cnt[i] == 0) continue;  // no moves: nothing below to search
-        const MergeSeg sg = M.segs[M.root[i]];
-        if (sg.end - sg.begin < 2) continue;
-        const Board b = level_get(M.planes, M.stride, i);
-        const u64 h = board_hash(b);
-        const u64 nSlots = MERGE_SLOTS * (u64)(sg.end - sg.begin);
-        unsigned long long *slots = M.set + MERGE_SLOTS * (u64)sg.begin;
-        const unsigned long long mine = (h << 32) | (u32)i;
-        u64 at = __umul64hi(h, nSlots);
-        for (int k = 0; k < MERGE_MAX_PROBES; k++) {
-            unsigned long long v = *(volatile unsigned long long *)(slots + at);
-            if (v == MERGE_EMPTY) {
-                v = atomicCAS(slots + at, MERGE_EMPTY, mine);
-                if (v == MERGE_EMPTY) break;  // this node owns its position
-            }
-            if ((v >> 32) == (u32)h) {
-                const u32 o = (u32)v;
-                const Board ob = level_get(M.planes, M.stride, o);
-                if (((ob.mine ^ b.mine) | (ob.pawns ^ b.pawns) | (ob.knights ^ b.knights) | (ob.bq ^ b.bq) |
-                     (ob.rq ^ b.rq) | (ob.kings ^ b.kings)) == 0) {
-                    atomicAdd(M.weight + o, M.weight[i]);
-                    M.cnt[i] = 0;
-                    break;
+        u32 link = ALIAS_HIT;
+        if (LINKED) M.acc[i] = 0;
+        if (M.cnt[i]) {  // (no moves: nothing below to search)
+            link = ALIAS_NOSLOT;
+            MergeSeg sg{0, (u32)M.n};
+            if (!LINKED) sg = M.segs[M.root[i]];
+            if (!LINKED && sg.end - sg.begin < 2) continue;
+            const Board b = level_get(M.planes, M.stride, i);
+            const u64 h = board_hash(b);
+            const u64 nSlots = MERGE_SLOTS * (u64)(sg.end - sg.begin);
+            unsigned long long *slots = M.set + MERGE_SLOTS * (u64)sg.begin;
+            const unsigned long long mine = (h << 32) | (u32)i;
+            u64 at = __umul64hi(h, nSlots);
+            for (int k = 0; k < MERGE_MAX_PROBES; k++) {
+                unsigned long long v = *(volatile unsigned long long *)(slots + at);
+                if (v == MERGE_EMPTY) {
+                    v = atomicCAS(slots + at, MERGE_EMPTY, mine);
+                    if (v == MERGE_EMPTY) {  // this node owns its position
+                        link = (u32)i;
+                        break;
+                    }
                 }
+                if ((v >> 32) == (u32)h) {
+                    const u32 o = (u32)v;
+                    const Board ob = level_get(M.planes, M.stride, o);
+                    if (((ob.mine ^ b.mine) | (ob.pawns ^ b.pawns) | (ob.knights ^ b.knights) | (ob.bq ^ b.bq) |
+                         (ob.rq ^ b.rq) | (ob.kings ^ b.kings)) == 0) {
+                        if (!LINKED) atomicAdd(M.weight + o, M.weight[i]);
+                        M.cnt[i] = 0;
+                        link = o;
+                        nMerged++;
+                        break;
+                    }
+                }
+                if (++at == nSlots) at = 0;
             }
-            if (++at == nSlots) at = 0;
         }
+        if (LINKED) M.alias[i] = link;
     }
+    if (LINKED) block_add_stat(M.merged, nMerged);
 }
 
 __global__ void __launch_bounds__(256) k_merge_prepare(const MergeLevel M) { merge_prepare(M); }
-__global__ void __launch_bounds__(256) k_merge_nodes(const MergeLevel M) { merge_nodes(M); }
+__global__ void __launch_bounds__(256) k_merge_nodes(const MergeLevel M) { merge_nodes<false>(M); }
+__global__ void __launch_bounds__(256) k_merge_linked(const MergeLevel M) { merge_nodes<true>(M); }
 
 // The same for a device-driven level.
 __device__ __forceinline__ MergeLevel dd_merge_level(const DevPlan *plan, int lv, int remaining)
 {
     const LevelDesc &C = plan->lv[lv];
     return MergeLevel{C.planes, C.stride, C.set ? C.n : 0, C.cnt, C.root, C.weight, C.set,
-                      plan->segs, plan->rootDepth, remaining};
+                      plan->segs, plan->rootDepth, remaining, nullptr, nullptr, nullptr};
 }
 __global__ void __launch_bounds__(256) k_dd_merge_prepare(const DevPlan *plan, int lv, int remaining)
 {
@@ -765,7 +805,7 @@ __global__ void __launch_bounds__(256) k_dd_merge_prepare(const DevPlan *plan, i
 }
 __global__ void __launch_bounds__(256) k_dd_merge_nodes(const DevPlan *plan, int lv, int remaining)
 {
-    merge_nodes(dd_merge_level(plan, lv, remaining));
+    merge_nodes<false>(dd_merge_level(plan, lv, remaining));
 }
 
 // ------------------------------------------------------------ tile kernel
@@ -1257,31 +1297,26 @@ __global__ void __launch_bounds__(SMALL_NT, SMALL_MINB) k_small_tree(const u64 *
 // colour mirror, so a position and its mirror may share an entry.
 constexpr int ZOB_KEYS = 781;
 constexpr int ZOB_DEPTH_KEYS = 32;
-// Two independent key sets (x, y): the x hash picks the table slot and the
-// de-duplication slot, the y hash verifies.  A verification key that shares
+// Two independent key sets (x, y): the x hash picks the table slot, the y
+// hash verifies.  A verification key that shares
 // no bits with the index keeps false hits at 2^-64 per probe; with one 64-bit
 // hash doing both, only the bits above the index are checked, and searches
 // with ~1e12 probes (perft 12 of the initial position) did see false hits.
 __device__ ulonglong2 d_zobrist[ZOB_KEYS + ZOB_DEPTH_KEYS];
 
-constexpr u32 ALIAS_HIT = 0xFFFFFFFFu;     // value came from the table
-constexpr u32 ALIAS_NOSLOT = 0xFFFFFFFEu;  // not de-duplicated (set full)
-constexpr u64 DEDUP_EMPTY = ~0ULL;
-constexpr int DEDUP_MAX_PROBES = 64;
-
 struct TTStats {
     unsigned long long probes, hits, aliases, stores;
 };
 
-__device__ __forceinline__ void zx(ulonglong2 &h, int k)
+__device__ __forceinline__ void zx(ulonglong2 &h, const ulonglong2 &z)
 {
-    const ulonglong2 z = __ldg(&d_zobrist[k]);
     h.x ^= z.x;
     h.y ^= z.y;
 }
 
-// Both Zobrist hashes of a side-relative board (one 16-byte key load per piece).
-__device__ __forceinline__ ulonglong2 zobrist_rel(const Board &b)
+// Both Zobrist hashes of a side-relative board (one 16-byte key read from
+// shared memory per piece).
+__device__ __forceinline__ ulonglong2 zobrist_rel(const Board &b, const ulonglong2 *keys)
 {
     const u64 pawns = b.pawns & RANKS2TO7;
     const u64 occ = pawns | b.knights | b.bq | b.rq | b.kings;
@@ -1290,22 +1325,14 @@ __device__ __forceinline__ ulonglong2 zobrist_rel(const Board &b)
     ulonglong2 h = make_ulonglong2(0, 0);
 #pragma unroll
     for (int pc = 0; pc < 6; pc++) {
-        u64 m = sets[pc] & b.mine;
-        while (m) {
-            zx(h, pc * 64 + ctz(m));
-            m &= m - 1;
-        }
-        u64 t = sets[pc] & theirs;
-        while (t) {
-            zx(h, (6 + pc) * 64 + ctz(t));
-            t &= t - 1;
-        }
+        for_each_bit(sets[pc] & b.mine, [&](int sq) { zx(h, keys[pc * 64 + sq]); });
+        for_each_bit(sets[pc] & theirs, [&](int sq) { zx(h, keys[(6 + pc) * 64 + sq]); });
     }
     const u32 st = (u32)(b.pawns & 0xFF);
 #pragma unroll
     for (int k = 0; k < 4; k++)
-        if (st & (1u << k)) zx(h, 768 + k);
-    if (st >> 4) zx(h, 772 + (st >> 4) - 1);
+        if (st & (1u << k)) zx(h, keys[768 + k]);
+    if (st >> 4) zx(h, keys[772 + (st >> 4) - 1]);
     return h;
 }
 
@@ -1324,86 +1351,44 @@ __device__ __forceinline__ void count_stat(unsigned long long *ctr, bool hit)
     if (threadIdx.x == 0 && sCount) atomicAdd(ctr, (unsigned long long)sCount);
 }
 
-// Hash every node, probe the table, and insert misses into the level's
-// de-duplication set (lowest index wins).  Hits get their value and no
-// children; their alias is ALIAS_HIT.  Misses keep the set slot in alias.
+// Hashes and probes the nodes that stand for themselves after the level was
+// merged (owners, and nodes the set had no slot for).  Hits take the table's
+// value and lose their children; their alias is ALIAS_HIT.
+// The keys are read from shared memory: a warp's 32 scattered 16-byte reads
+// per piece took one L1 pass each from global memory and bound the kernel.
+// Persistent blocks, so that the 13 KB of keys are loaded once per block.
+// Merging first (exact, by the boards) halves the nodes hashed.  Two table
+// positions at depth 8: 261 -> 255 ms.
 __global__ void __launch_bounds__(256) k_tt_probe(const u64 *__restrict__ planes, u64 stride, u64 n, int remaining,
-                                                  bool probe, u64 keyMask, u32 *__restrict__ cnt,
-                                                  u64 *__restrict__ hash, u64 *__restrict__ hash2,
-                                                  unsigned long long *__restrict__ acc, u32 *__restrict__ alias,
-                                                  const ulonglong2 *tt, u64 ttMask, u64 *__restrict__ dkey,
-                                                  u32 *__restrict__ downer, u64 dMask, TTStats *ts)
-{
-    const u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-    bool hit = false;
-    if (i < n) {
-        const Board b = level_get(planes, stride, i);
-        ulonglong2 z = zobrist_rel(b);
-        zx(z, ZOB_KEYS + remaining);
-        const u64 h = z.x & keyMask;  // slot key (table index, de-duplication set)
-        const u64 g = z.y;            // verification key
-        hash[i] = h;
-        hash2[i] = g;
-        acc[i] = 0;
-        if (probe) {
-            const ulonglong2 e = tt[h & ttMask];
-            if ((e.x ^ e.y) == g) {
-                hit = true;
-                acc[i] = e.y;
-                cnt[i] = 0;
-                alias[i] = ALIAS_HIT;
-            }
-        }
-        if (!hit) {
-            u32 placed = ALIAS_NOSLOT;
-            if (h != DEDUP_EMPTY) {
-                u64 slot = (h * 0x9E3779B97F4A7C15ULL >> 17) & dMask;
-                for (int k = 0; k < DEDUP_MAX_PROBES; k++) {
-                    const unsigned long long old =
-                        atomicCAS((unsigned long long *)&dkey[slot], (unsigned long long)DEDUP_EMPTY,
-                                  (unsigned long long)h);
-                    if (old == DEDUP_EMPTY || old == h) {
-                        atomicMin(&downer[slot], (u32)i);
-                        placed = (u32)slot;
-                        break;
-                    }
-                    slot = (slot + 1) & dMask;
-                }
-            }
-            alias[i] = placed;
-        }
-    }
-    if (probe) {
-        count_stat(&ts->probes, i < n);
-        count_stat(&ts->hits, hit);
-    }
-}
-
-// Turns set slots into owner indices; duplicates lose their children.  A
-// node shares its owner's slot key; it is a duplicate only if the
-// verification keys match too, otherwise it is searched on its own.
-__global__ void __launch_bounds__(256) k_tt_dedup(u64 n, u32 *__restrict__ cnt, u32 *__restrict__ alias,
-                                                  const u32 *__restrict__ downer, const u64 *__restrict__ hash2,
+                                                  u64 keyMask, u32 *__restrict__ cnt, u64 *__restrict__ hash,
+                                                  u64 *__restrict__ hash2, unsigned long long *__restrict__ acc,
+                                                  u32 *__restrict__ alias, const ulonglong2 *tt, u64 ttMask,
                                                   TTStats *ts)
 {
-    const u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-    bool dup = false;
-    if (i < n) {
+    __shared__ ulonglong2 keys[ZOB_KEYS];
+    for (int k = threadIdx.x; k < ZOB_KEYS; k += 256) keys[k] = d_zobrist[k];
+    const ulonglong2 depthKey = d_zobrist[ZOB_KEYS + remaining];
+    __syncthreads();
+    u32 probes = 0, hits = 0;
+    for (u64 i = (u64)blockIdx.x * 256 + threadIdx.x; i < n; i += (u64)gridDim.x * 256) {
         const u32 a = alias[i];
-        if (a != ALIAS_HIT && a != ALIAS_NOSLOT) {
-            const u32 o = downer[a];
-            if (o == (u32)i) {
-                alias[i] = o;
-            } else if (hash2[o] == hash2[i]) {
-                alias[i] = o;
-                cnt[i] = 0;
-                dup = true;
-            } else {
-                alias[i] = ALIAS_NOSLOT;
-            }
+        if (a != (u32)i && a != ALIAS_NOSLOT) continue;
+        ulonglong2 z = zobrist_rel(level_get(planes, stride, i), keys);
+        zx(z, depthKey);
+        const u64 h = z.x & keyMask;  // slot key (table index)
+        hash[i] = h;
+        hash2[i] = z.y;               // verification key
+        const ulonglong2 e = tt[h & ttMask];
+        probes++;
+        if ((e.x ^ e.y) == z.y) {
+            hits++;
+            acc[i] = e.y;
+            cnt[i] = 0;
+            alias[i] = ALIAS_HIT;
         }
     }
-    count_stat(&ts->aliases, dup);
+    block_add_stat(&ts->probes, probes);
+    block_add_stat(&ts->hits, hits);
 }
 
 // After a level's subtrees are summed into acc: copy owners' values into
@@ -1473,9 +1458,11 @@ struct DeviceLevel {
 };
 
 // Bytes of one TT level node: the plain node plus two hashes, subtree sum, alias,
-// and the transient de-duplication set (at most 2.5 slots of 12 bytes per
-// node; it is released before the scan, so this over-counts slightly).
+// and the transient merge set (it is released before the scan, so this
+// over-counts).
 constexpr u64 NODE_BYTES_TT = NODE_BYTES + 8 + 8 + 8 + 4 + 30;
+// Without a table (related roots): the plain node plus sum, alias and set.
+constexpr u64 NODE_BYTES_LINKED = NODE_BYTES + 8 + 4 + 8 * MERGE_SLOTS;
 
 class Engine {
 public:
@@ -1795,8 +1782,8 @@ int Engine::init(const perft_config &cfg)
         for (int k = 0; k < ZOB_KEYS + ZOB_DEPTH_KEYS; k++) keys[k].y = next();
         ENG_TRY(cudaMemcpyToSymbol(d_zobrist, keys, sizeof keys));
         // PERFT_TT_INDEX_KEY_BITS=b keeps only the low b bits of the slot key:
-        // a test setting that makes different positions share table and
-        // de-duplication slots, which the verification key must then tell apart
+        // a test setting that makes different positions share table slots,
+        // which the verification key must then tell apart
         ttKeyMask = ~0ULL;
         if (const char *kb = getenv("PERFT_TT_INDEX_KEY_BITS")) {
             const int bits = atoi(kb);
@@ -1936,7 +1923,8 @@ int Engine::merge_level(const Joiners &J, const DeviceLevel &C, int remaining)
     unsigned long long *set = (unsigned long long *)alloc(8 * MERGE_SLOTS * C.n);
     arenaTop = mark;  // free again once the merge has run (stream order)
     if (!set) return PERFT_OK;  // the level stays unmerged
-    const MergeLevel M{C.planes, C.stride, C.n, C.cnt, C.root, C.weight, set, J.segs, J.depths, remaining};
+    const MergeLevel M{C.planes, C.stride, C.n,       C.cnt,     C.root,  C.weight, set,
+                       J.segs,   J.depths, remaining, nullptr, nullptr, nullptr};
     const unsigned grid = (unsigned)std::min<u64>((C.n + 255) / 256, 64ull * nsm);
     k_merge_prepare<<<grid, 256, 0, stream>>>(M);
     k_merge_nodes<<<grid, 256, 0, stream>>>(M);
@@ -2279,11 +2267,14 @@ int Engine::autotune(bool leaf, bool expand)
 bool Engine::alloc_level_tt(DeviceLevel &L, u64 n)
 {
     if (!alloc_level(L, n)) return false;
-    L.hash = (u64 *)alloc(8 * L.stride);
-    L.hash2 = (u64 *)alloc(8 * L.stride);
+    if (tt) {
+        L.hash = (u64 *)alloc(8 * L.stride);
+        L.hash2 = (u64 *)alloc(8 * L.stride);
+        if (!L.hash || !L.hash2) return false;
+    }
     L.acc = (unsigned long long *)alloc(8 * L.stride);
     L.alias = (u32 *)alloc(4 * L.stride);
-    return L.hash && L.hash2 && L.acc && L.alias;
+    return L.acc && L.alias;
 }
 
 int Engine::tt_clear()
@@ -2294,9 +2285,9 @@ int Engine::tt_clear()
     return PERFT_OK;
 }
 
-// Transposition-table version of process_level.  Every node of L (remaining
-// plies `remaining`) is hashed and probed; hits and same-level duplicates
-// are not expanded.  Subtree sums accumulate in L.acc: directly from the
+// Transposition-table version of process_level.  L (remaining plies
+// `remaining`) is merged over all its roots, and the nodes that stay are
+// hashed and probed; hits and copies are not expanded.  Subtree sums accumulate in L.acc: directly from the
 // count-only last ply, or from the child levels' finish pass.  When L is
 // done, owners are stored, duplicates copy their owner's value, and the
 // values are added into parentAcc (or written to the roots' results).
@@ -2306,22 +2297,21 @@ int Engine::process_level_tt(const DeviceLevel &L, int remaining, unsigned long 
     if (L.n == 0) return PERFT_OK;
     const u64 mark = arenaTop;
     const unsigned nb = (unsigned)((L.n + 255) / 256);
-    const bool useTT = remaining >= ttMinDepth;
+    const bool useTT = tt != nullptr && remaining >= ttMinDepth;
 
-    u64 dsize = 1024;
-    while (dsize < L.n + L.n / 4) dsize <<= 1;  // load <= 80%; unplaced nodes are simply not de-duplicated
-    u64 *dkey = (u64 *)alloc(8 * dsize);
-    u32 *downer = (u32 *)alloc(4 * dsize);
-    if (!dkey || !downer) return PERFT_ERR_OUT_OF_MEMORY;
-    ENG_TRY(cudaMemsetAsync(dkey, 0xFF, 8 * dsize, stream));
-    ENG_TRY(cudaMemsetAsync(downer, 0xFF, 4 * dsize, stream));
-    k_tt_probe<<<nb, 256, 0, stream>>>(L.planes, L.stride, L.n, remaining, useTT, ttKeyMask, L.cnt, L.hash, L.hash2,
-                                       L.acc, L.alias,
-                                       tt, ttMask, dkey, downer, dsize - 1, dTTStats);
-    k_tt_dedup<<<nb, 256, 0, stream>>>(L.n, L.cnt, L.alias, downer, L.hash2, dTTStats);
-    stats.other_launches += 2;
+    unsigned long long *set = (unsigned long long *)alloc(8 * MERGE_SLOTS * L.n);
+    if (!set) return PERFT_ERR_OUT_OF_MEMORY;
+    ENG_TRY(cudaMemsetAsync(set, 0xFF, 8 * MERGE_SLOTS * L.n, stream));
+    const MergeLevel M{L.planes, L.stride, L.n,     L.cnt, nullptr, nullptr, set,
+                       nullptr,  nullptr,  remaining, L.alias, L.acc,   &dTTStats->aliases};
+    k_merge_linked<<<(unsigned)std::min<u64>(nb, 64ull * nsm), 256, 0, stream>>>(M);
+    if (useTT)
+        k_tt_probe<<<(unsigned)std::min<u64>(nb, 8ull * nsm), 256, 0, stream>>>(
+            L.planes, L.stride, L.n, remaining, ttKeyMask, L.cnt, L.hash, L.hash2, L.acc, L.alias, tt, ttMask,
+            dTTStats);
+    stats.other_launches += 1 + useTT;
     ENG_TRY(cudaGetLastError());
-    arenaTop = mark;  // the de-duplication set is no longer needed
+    arenaTop = mark;  // the set is no longer needed
 
     ParentIndex ix;
     int rc = scan(L.cnt, L.n, remaining, true, ix);
@@ -2336,7 +2326,7 @@ int Engine::process_level_tt(const DeviceLevel &L, int remaining, unsigned long 
         } else {
             const u64 slack = std::min<u64>(64ull << 20, arenaCap / 16);
             const u64 freeB = arena_free() > slack ? arena_free() - slack : 0;
-            u64 budgetNodes = freeB / NODE_BYTES_TT;
+            u64 budgetNodes = freeB / (tt ? NODE_BYTES_TT : NODE_BYTES_LINKED);
             if (remaining > 3) budgetNodes /= 2;
             const u64 chunk = total <= budgetNodes ? total : (budgetNodes & ~(u64)(TILE_CAP - 1));
             if (chunk == 0) return PERFT_ERR_OUT_OF_MEMORY;
@@ -2355,7 +2345,7 @@ int Engine::process_level_tt(const DeviceLevel &L, int remaining, unsigned long 
         }
     }
     arenaTop = mark;
-    k_tt_finish<<<nb, 256, 0, stream>>>(L.n, useTT && tt != nullptr, L.hash, L.hash2, L.acc, L.alias, L.root,
+    k_tt_finish<<<nb, 256, 0, stream>>>(L.n, useTT, L.hash, L.hash2, L.acc, L.alias, L.root,
                                         parentAcc, tt,
                                         ttMask, dTTStats);
     stats.other_launches++;

@@ -194,6 +194,7 @@ private:
     u32 maxInFlight = 0, inFlight = 0, maxSlotUsed = 0;
     int gridLeaf = 0, gridExpand = 0, gridLeafAcc = 0, gridExpandTT = 0;
     bool leafSplit = false;
+    unsigned nsm = 1;
     // the engine's transposition table, when the server uses it
     ulonglong2 *tt = nullptr;
     u64 ttMask = 0, ttKeyMask = ~0ULL;
@@ -284,6 +285,7 @@ int Server::start(const perft_serve_config &cfg, char *block, u64 bytes, int dev
     memset(hostTTStats, 0, sizeof(TTStats));
     cudaDeviceProp prop;
     if (cudaGetDeviceProperties(&prop, dev) != cudaSuccess) return PERFT_ERR_CUDA;
+    nsm = (unsigned)prop.multiProcessorCount;
     cudaFuncSetAttribute(k_tile<MODE_LEAF, SV_KOGGE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)TILE_DYN_SMEM);
     cudaFuncSetAttribute(k_tile<MODE_LEAF, SV_KOGGE_SPLIT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -510,23 +512,20 @@ int Server::probe_level(ServeLevel &S)
     S.L.hash2 = (u64 *)take(8 * S.L.stride, S.ttMem);
     S.L.acc = (unsigned long long *)take(8 * S.L.stride, S.ttMem);
     S.L.alias = (u32 *)take(4 * S.L.stride, S.ttMem);
-    u64 dsize = 1024;
-    while (dsize < n + n / 4) dsize <<= 1;
     std::vector<std::pair<u64, u64>> tmp;
-    u64 *dkey = (u64 *)take(8 * dsize, tmp);
-    u32 *downer = (u32 *)take(4 * dsize, tmp);
-    if (!S.L.hash || !S.L.hash2 || !S.L.acc || !S.L.alias || !dkey || !downer) {
+    unsigned long long *set = (unsigned long long *)take(8 * MERGE_SLOTS * n, tmp);
+    if (!S.L.hash || !S.L.hash2 || !S.L.acc || !S.L.alias || !set) {
         give_back(tmp);
         give_back(S.ttMem);  // the next iteration retries from scratch
         return PERFT_ERR_OUT_OF_MEMORY;
     }
     const unsigned nb = (unsigned)((n + 255) / 256);
-    if (cudaMemsetAsync(dkey, 0xFF, 8 * dsize, st) != cudaSuccess ||
-        cudaMemsetAsync(downer, 0xFF, 4 * dsize, st) != cudaSuccess)
-        return PERFT_ERR_CUDA;
-    k_tt_probe<<<nb, 256, 0, st>>>(S.L.planes, S.L.stride, n, S.r, true, ttKeyMask, S.L.cnt, S.L.hash, S.L.hash2,
-                                   S.L.acc, S.L.alias, tt, ttMask, dkey, downer, dsize - 1, dTTStats);
-    k_tt_dedup<<<nb, 256, 0, st>>>(n, S.L.cnt, S.L.alias, downer, S.L.hash2, dTTStats);
+    if (cudaMemsetAsync(set, 0xFF, 8 * MERGE_SLOTS * n, st) != cudaSuccess) return PERFT_ERR_CUDA;
+    const MergeLevel M{S.L.planes, S.L.stride, n,   S.L.cnt,   nullptr, nullptr, set,
+                       nullptr,    nullptr,    S.r, S.L.alias, S.L.acc, &dTTStats->aliases};
+    k_merge_linked<<<std::min(nb, 64u * nsm), 256, 0, st>>>(M);
+    k_tt_probe<<<std::min(nb, 8u * nsm), 256, 0, st>>>(S.L.planes, S.L.stride, n, S.r, ttKeyMask, S.L.cnt, S.L.hash,
+                                                       S.L.hash2, S.L.acc, S.L.alias, tt, ttMask, dTTStats);
     launches += 2;
     give_back(tmp);  // reused only by later launches on this stream
     S.tt = true;
