@@ -62,6 +62,25 @@ def test_uneven_batch(both_paths, oracle):
     assert np.array_equal(both_paths.perft_batch(pos, depths), oracle.perft_batch_mt(pos, depths))
 
 
+def test_related_roots(engine, oracle):
+    """Roots a few moves apart are searched as one tree: the children of one
+    position, repeated roots, and roots that differ only in the real side to
+    move; one root out of place sends the batch down the ordinary path."""
+    start = engine.fen_to_pos(engine.START_FEN)
+    mid = engine.random_playouts(seed=83, n=1, min_plies=16, max_plies=16)[0]
+    black = start.copy()
+    black[1] |= np.uint64(1 << 63)
+    batches = [np.stack([engine.apply_move(p, m) for m in engine.legal_moves(p)] * k) for p, k in ((mid, 2), (start, 2))]
+    batches.append(np.stack([start, black] * 16))
+    batches.append(np.concatenate([batches[1], mid[None]]))
+    for pos in batches:
+        engine.reset_stats()
+        got = engine.perft_batch(pos, 5)
+        linked = engine.stats()["tt_duplicates"] > 0
+        assert linked == (pos is not batches[3])
+        assert np.array_equal(got, oracle.perft_batch_mt(pos, 5))
+
+
 def test_fewer_items_than_paths(both_paths):
     """The count-only ply looks at each position once per root: initial
     position, depth 6, whose 197,281 four-ply paths reach 72,078 positions."""
