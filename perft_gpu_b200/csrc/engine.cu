@@ -1043,40 +1043,87 @@ __global__ void __launch_bounds__(TILE_NT, TILE_MINB) k_tile(const TileParams Pi
 }
 
 // ============================================================ small trees
-// One position of depth 2..5 in one launch, with no level buffers.  The level
-// pipeline spends such a tree's time on per-ply latency: a scan and a tile
-// launch per ply, each a few microseconds on a handful of busy SMs.  Here
-// each CTA takes whole subtrees rooted `depth - r` plies below the position
-// (r = 3, or 2 at depth 2) and counts each one in shared memory:
-//   1. thread 0 generates the subtree root's moves;
-//   2. one thread per move makes the child and counts the child's moves (at
-//      r = 2 these counts are the subtree's perft);
-//   3. a block scan of those counts places the grandchildren, and one thread
-//      per child generates the child's moves into a window of the item list;
-//   4. every thread takes items: make the grandchild, count its moves, sum.
-// Every CTA lists the subtree roots for itself (the position's moves, and at
-// depth 5 its children's moves), so no CTA waits for another; the last CTA
-// to finish sums the per-CTA partial counts.  The move generator, make-move
-// and count are the level pipeline's own functions.
-#ifndef PG_SMALL_NT
-#define PG_SMALL_NT 128
-#endif
-constexpr int SMALL_NT = PG_SMALL_NT;  // threads per CTA: small CTAs put more subtrees in flight
-constexpr int SMALL_MINB = 512 / SMALL_NT;
+// Positions of small depth in one launch, with no level buffers: one position
+// of depth 2..5, or a batch of up to SMALL_BATCH positions of depth 0..4.
+// The level pipeline spends such trees' time on per-ply latency: a scan and a
+// tile launch per ply, each a few microseconds on a handful of busy SMs.  Here
+// each position has some CTAs (its slices), and each CTA counts whole subtrees
+// rooted `depth - 3` plies below the position in shared memory.  Two steps
+// alternate, each with a whole CTA's threads on it:
+//   * small_process: one thread per move makes the child and counts the
+//     child's moves; the count also yields what the child's moves depend on
+//     (MoveCtx);
+//   * small_list: the moves of some positions into the CTA's item list, each
+//     warp taking one part of the generation (gen_part) of 32 positions, so
+//     that no thread generates a whole position and no warp diverges by part.
+// Bound by latency, not throughput: a handful of dependent steps per ply.
+// The steps replace one thread generating a position's moves from scratch
+// while the CTA waits (5-6.5 us each, three in a row at depth 5).  Both steps
+// are single out-of-line functions, since every further inlined copy is
+// fetched cold on every launch.
+// Tried: a thread per (position, piece) and the n-th move found by a search in
+// the scanned move counts instead of a list.  As fast for one position, but
+// 32 positions took 8-20 us against 4: every thread paid for all eight slider
+// directions.
+// Measured per call, before and after: opening at depth 5 84 -> 62 us, depth 3
+// 52 -> 26 us (the kernel 12 us of it), 61 positions of depths 1-4 217 -> 88 us
+// (as a replayed graph of the level pipeline before; on new depths 500 -> 94).
+// Every CTA finds its subtree roots for itself, so no CTA waits for another;
+// the last CTA to finish hands the sums over and clears them for the next
+// launch.  The make-move and count are the level pipeline's own functions.
+constexpr int SMALL_NT = 128;  // threads per CTA: small CTAs put more subtrees in flight
+constexpr int SMALL_MINB = 4;
 constexpr int SMALL_MAX_DEPTH = 5;
-constexpr u32 SMALL_LIST_CAP = 4096;  // subtree roots one CTA can list (depth 5)
-constexpr u32 SMALL_WIN = 2048;       // items per window of a subtree's last ply
-constexpr size_t SMALL_DYN_SMEM = sizeof(u32) * (SMALL_LIST_CAP + SMALL_WIN);
-constexpr int SMALL_MAX_GRID = 1024;
-constexpr u32 SMALL_OVERFLOW = 1u << 8;  // more subtree roots than the list holds: not counted
+constexpr int SMALL_BATCH = 64;
+constexpr int SMALL_BATCH_DEPTH = 4;
+constexpr u32 SMALL_LIST_CAP = 4096;  // most subtree roots of a depth-5 position (larger trees: level pipeline)
+constexpr u32 SMALL_PART = 256;
+constexpr u32 SMALL_ITEMS = 2048 + MAX_LEGAL_MOVES;  // the item list: whole positions up to 2048 moves and one more
+constexpr int SMALL_SLICES = 48;      // subtree roots of a depth-4 position handled at the same time (few positions have more moves)
+constexpr u32 SMALL_OVERFLOW = 1u << 8;  // not counted: too many subtree roots, moves or pieces
 
-struct SmallState {
-    unsigned long long partial[SMALL_MAX_GRID];  // per CTA
-    unsigned long long count;                    // the last CTA's sum
-    u32 flags;    // 0, SMALL_OVERFLOW or DERR_BAD_POSITION (written by the last CTA)
-    u32 done;     // CTAs finished; atomicInc wraps it back to 0 for the next launch
-    u32 flagAcc;  // flags raised by any CTA; the last CTA reads and clears it
+// The launch's parameters, positions included, so that host positions need no copy.
+template <int N>
+struct SmallParams {
+    const u64 *dPos;  // positions on the device; null: pos below
+    u64 *dOut;        // device results (may be null)
+    struct SmallResult *host;  // mapped host memory
+    struct SmallState *state;
+    u32 n, listCap;
+    uint16_t unit0[N + 1];  // first CTA of each position
+    uint8_t depth[N];
+    uint8_t split[N];  // CTAs that share one subtree
+    u64 pos[6 * N];
 };
+struct SmallResult {
+    u64 count[SMALL_BATCH];
+    u32 flags;  // 0, SMALL_OVERFLOW or DERR_BAD_POSITION
+};
+struct SmallState {  // all zero between launches
+    unsigned long long sum[SMALL_BATCH];
+    u32 done;   // CTAs finished
+    u32 flags;  // raised by any CTA
+};
+
+// Places of the positions a CTA holds.
+constexpr int SMALL_CHILD0 = 0;                     // the current subtree root's children
+constexpr int SMALL_SUB = MAX_LEGAL_MOVES;          // the current subtree root
+constexpr int SMALL_ROOT = SMALL_SUB + 1;           // the CTA's position
+constexpr int SMALL_FIRST0 = SMALL_ROOT + 1;        // its children
+constexpr int SMALL_PLACES = SMALL_FIRST0 + MAX_LEGAL_MOVES;
+struct SmallShared {
+    Board b[SMALL_PLACES];
+    MoveCtx c[SMALL_PLACES];
+    u32 items[SMALL_ITEMS];  // (place << 16) | move
+    u32 nItems;
+    u32 nPart[GEN_PARTS];  // one position's list: its parts' moves, each part at its own SMALL_PART items
+    u32 first[MAX_LEGAL_MOVES];  // first item below each child of the position, or of the subtree root
+    uint8_t cnt[SMALL_PLACES];  // move counts (at most MAX_LEGAL_MOVES, else flagged)
+    u32 sw[SMALL_NT / 32];
+    u32 flags;
+    bool last;
+};
+constexpr size_t SMALL_DYN_SMEM = sizeof(SmallShared);
 
 // Exclusive block sum of one u32 per thread; `total` gets the block's sum.
 template <int NT>
@@ -1102,191 +1149,240 @@ __device__ __forceinline__ u32 block_excl_sum(u32 v, u32 *sw, u32 &total)
     return off + inc - v;
 }
 
-// The kernel's phases: the generator into a window, make-and-count, make.
-// PG_SMALL_NOINLINE 1 calls one out-of-line copy of each instead of inlining
-// them at every call site (a tuning build; it measured no faster).
-#ifndef PG_SMALL_NOINLINE
-#define PG_SMALL_NOINLINE 0
-#endif
-#if PG_SMALL_NOINLINE
-#define PG_SMALL_FN __device__ __noinline__
-#else
-#define PG_SMALL_FN __device__ __forceinline__
-#endif
-// Generates b's moves into items[rel0 ..] (those inside [0, n), tagged);
-// returns rel0 plus the number of moves.  PG_SMALL_GEN_SV: the generator's
-// slider variant here.  Kogge-Stone fills (0): one thread generating on a
-// fresh launch waits on every table lookup, and the fills need none; the
-// initial position at depth 5 took 68 us with them against 74 us with the
-// generator's default magic lookups (-1).
-#ifndef PG_SMALL_GEN_SV
-#define PG_SMALL_GEN_SV 0
-#endif
-template <int SV>
-PG_SMALL_FN int small_gen(Board b, u32 *items, int rel0, u32 n, u32 tag)
+// Exclusive sums of the move counts at places p0 .. p0 + n - 1 into S.first
+// (n <= MAX_LEGAL_MOVES); returns the total.
+__device__ __forceinline__ u32 small_first(SmallShared &S, int p0, int n)
 {
-    WindowSink sink{items, rel0, n, tag};
-    gen_moves<SV, false, PG_SMALL_GEN_SV>(b, sink);
-    return sink.rel;
-}
-
-template <int SV>
-PG_SMALL_FN u32 small_make_count(Board parent, u32 mv, Board *child)
-{
-    const Board c = make_child<false>(parent, mv);
-    if (child) *child = c;
-    return count_moves<SV>(c);
-}
-
-template <int SV>
-PG_SMALL_FN Board small_make(Board parent, u32 mv)
-{
-    return make_child<false>(parent, mv);
-}
-
-// Exclusive offsets of the counts c[0..n) (n <= MAX_LEGAL_MOVES) into
-// off[0..n); returns their total.  Each thread scans SMALL_PER consecutive
-// entries.
-template <int NT>
-__device__ __forceinline__ u32 small_scan(const u32 *c, u32 *off, u32 n, u32 *sw)
-{
-    constexpr int PER = (MAX_LEGAL_MOVES + NT - 1) / NT;
-    const u32 t0 = threadIdx.x * PER;
-    u32 v = 0;
-#pragma unroll
-    for (int k = 0; k < PER; k++) v += (t0 + k < n) ? c[t0 + k] : 0u;
+    static_assert(2 * SMALL_NT >= MAX_LEGAL_MOVES, "two positions per thread");
+    const int t = 2 * threadIdx.x;
+    const u32 a = t < n ? S.cnt[p0 + t] : 0u, b = t + 1 < n ? S.cnt[p0 + t + 1] : 0u;
     u32 total;
-    u32 base = block_excl_sum<NT>(v, sw, total);
-#pragma unroll
-    for (int k = 0; k < PER; k++)
-        if (t0 + k < n) {
-            off[t0 + k] = base;
-            base += c[t0 + k];
-        }
+    const u32 x = block_excl_sum<SMALL_NT>(a + b, S.sw, total);
+    if (t < n) S.first[t] = x;
+    if (t + 1 < n) S.first[t + 1] = x + a;
     __syncthreads();
     return total;
 }
 
-// listCap: subtree roots a CTA may list, at most SMALL_LIST_CAP.
-template <int SV>
-__global__ void __launch_bounds__(SMALL_NT, SMALL_MINB) k_small_tree(const u64 *__restrict__ pos48, int depth,
-                                                                     u32 listCap, u64 *__restrict__ out,
-                                                                     SmallState *S)
+// Lists run by run at the list's cursor, or (one position) part by part.
+template <bool SHARED>
+struct SmallSink {
+    SmallShared &S;
+    u32 at, tag;
+    __device__ __forceinline__ void room(int n)
+    {
+        if (SHARED && n) at = atomicAdd(&S.nItems, (u32)n);
+    }
+    __device__ __forceinline__ void operator()(u32 m)
+    {
+        if (at < SMALL_ITEMS) S.items[at] = tag | m;
+        at++;
+    }
+};
+
+// Lists the moves of the positions at places p0 .. p0 + w - 1.  One
+// position's list has the same order in every CTA (slices pick their moves by
+// number); a list of several positions is in no particular order.
+__device__ __noinline__ void small_list(SmallShared &S, int p0, int w)
 {
-    __shared__ Board sB1[MAX_LEGAL_MOVES];  // the position's children (depth 5)
-    __shared__ Board sX[MAX_LEGAL_MOVES];   // the current subtree root's children
-    __shared__ u32 sM1[MAX_LEGAL_MOVES];    // the position's moves
-    __shared__ u32 sMR[MAX_LEGAL_MOVES];    // the current subtree root's moves
-    __shared__ u32 sC[MAX_LEGAL_MOVES];     // children's move counts
-    __shared__ u32 sOff[MAX_LEGAL_MOVES];   // and their exclusive offsets
-    __shared__ u32 swarp[SMALL_NT / 32];
-    __shared__ u32 sN;
-    __shared__ unsigned long long sSum[SMALL_NT / 32];
-    __shared__ bool sLast;
-    extern __shared__ __align__(16) u32 sdyn[];
-    u32 *sList = sdyn;                   // depth 5: subtree roots as (child << 16) | move
-    u32 *sItems = sdyn + SMALL_LIST_CAP;  // grandchildren as (child << 16) | move
+    static_assert(SMALL_NT == 32 * GEN_PARTS, "a warp per part");
+    const int part = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) S.nItems = 0;
+    __syncthreads();
+    if (w == 1) {
+        if (lane == 0) {
+            SmallSink<false> sink{S, (u32)part * SMALL_PART, (u32)p0 << 16};
+            gen_part(S.b[p0], S.c[p0], part, sink);
+            S.nPart[part] = sink.at - (u32)part * SMALL_PART;
+        }
+        __syncthreads();
+        return;
+    }
+    for (int p = p0 + lane; p < p0 + w; p += 32) {
+        if (!S.cnt[p]) continue;
+        SmallSink<true> sink{S, 0u, (u32)p << 16};
+        gen_part(S.b[p], S.c[p], part, sink);
+    }
+    __syncthreads();
+    if (threadIdx.x < GEN_PARTS) S.nPart[threadIdx.x] = threadIdx.x ? 0u : min(S.nItems, SMALL_ITEMS);
+    __syncthreads();
+}
 
+// Makes the listed moves j0, j0 + step, ... below j1 (one per thread) and
+// counts the children's moves; keeps the children at places keep, keep + 1,
+// ... when keep >= 0 (at most MAX_LEGAL_MOVES of them).  Returns this
+// thread's sum of counts.  A kept position with more moves than any game's
+// flags the tree.
+__device__ __noinline__ u32 small_process(SmallShared &S, u32 j0, u32 j1, u32 step, int keep)
+{
+    u32 sum = 0;
+    const u32 c0 = S.nPart[0], c1 = S.nPart[1], c2 = S.nPart[2], c3 = S.nPart[3];
+    j1 = min(j1, c0 + c1 + c2 + c3);
+    for (u32 i = threadIdx.x; j0 + i * step < j1; i += SMALL_NT) {
+        u32 j = j0 + i * step;
+        if (j >= c0) {  // (a list of several positions is all in the first part)
+            j -= c0;
+            u32 at = SMALL_PART;
+            if (j >= c1) {
+                j -= c1;
+                at += SMALL_PART;
+                if (j >= c2) {
+                    j -= c2;
+                    at += SMALL_PART;
+                }
+            }
+            j += at;
+        }
+        const u32 it = S.items[j];
+        const Board b = make_child<false>(S.b[it >> 16], it & 0xFFFFu);
+        MoveCtx c;
+        const u32 n = count_moves_fused<SV_KOGGE>(b, -1, -1, 0, 0, &c);
+        sum += n;
+        if (keep >= 0) {
+            S.b[keep + i] = b;
+            S.c[keep + i] = c;
+            S.cnt[keep + i] = (uint8_t)n;
+            if (n > (u32)MAX_LEGAL_MOVES) atomicOr(&S.flags, SMALL_OVERFLOW);
+        }
+    }
+    return sum;
+}
+
+template <int N>
+__global__ void __launch_bounds__(SMALL_NT, SMALL_MINB) k_small_trees(const __grid_constant__ SmallParams<N> P)
+{
+    extern __shared__ __align__(16) unsigned char smallShared[];
+    SmallShared &S = *reinterpret_cast<SmallShared *>(smallShared);
     const int tid = threadIdx.x, lane = tid & 31;
-    u64 p[6];
+
+    // this CTA's position, and its slice of it
+    int lo = 0, hi = N == 1 ? 1 : (int)P.n;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (P.unit0[mid] <= blockIdx.x) lo = mid;
+        else hi = mid;
+    }
+    const int at = lo;
+    const int depth = P.depth[at];
+    const u32 split = P.split[at], unit = blockIdx.x - P.unit0[at];
+    const u32 nSlices = (u32)(P.unit0[at + 1] - P.unit0[at]) / split;
+    const u32 slice = unit / split, part = unit % split;
+
+    if (tid == 0) S.flags = 0;
+    __syncthreads();
+    // the position's count and its check at the same time
+    if (tid == 0 || tid == 32) {
+        u64 p[6];
 #pragma unroll
-    for (int k = 0; k < 6; k++) p[k] = pos48[k];
-    const Board root = from_pos48(p);
-    const int r = depth >= 3 ? 3 : 2;
-    const int pre = depth - r;  // plies from the position to the subtree roots: 0, 1 or 2
-    u32 flags = validate_pos48(p) != 0 ? DERR_BAD_POSITION : 0u;
-    u32 nRoots = 1;
-    if (!flags && pre >= 1) {
-        if (tid == 0) sN = (u32)small_gen<SV>(root, sM1, 0, MAX_LEGAL_MOVES, 0u);
-        __syncthreads();
-        const u32 n1 = sN;
-        nRoots = n1;
-        if (n1 > (u32)MAX_LEGAL_MOVES) flags = SMALL_OVERFLOW;
-        if (!flags && pre == 2) {
-            for (u32 t = tid; t < n1; t += SMALL_NT) sC[t] = small_make_count<SV>(root, sM1[t], &sB1[t]);
-            __syncthreads();
-            const u32 total = small_scan<SMALL_NT>(sC, sOff, n1, swarp);
-            if (total > listCap) {
-                flags = SMALL_OVERFLOW;
-            } else {
-                for (u32 t = tid; t < n1; t += SMALL_NT)
-                    if (sC[t]) small_gen<SV>(sB1[t], sList, (int)sOff[t], listCap, t << 16);
-                nRoots = total;
-            }
+        for (int k = 0; k < 6; k++) p[k] = P.dPos ? P.dPos[6 * at + k] : P.pos[6 * at + k];
+        if (tid == 32) {
+            if (validate_pos48(p) != 0) atomicOr(&S.flags, DERR_BAD_POSITION);
+        } else {
+            const Board b = from_pos48(p);
+            MoveCtx c;
+            const u32 n = count_moves_fused<SV_KOGGE>(b, -1, -1, 0, 0, &c);
+            S.b[SMALL_ROOT] = b;
+            S.c[SMALL_ROOT] = c;
+            S.cnt[SMALL_ROOT] = (uint8_t)n;
+            if (n > (u32)MAX_LEGAL_MOVES && depth >= 2) atomicOr(&S.flags, SMALL_OVERFLOW);
+            S.nItems = n;
         }
-        __syncthreads();  // every thread has read sN and the lists before the loop rewrites them
     }
-
+    __syncthreads();
     unsigned long long acc = 0;
-    for (u32 s = blockIdx.x; !flags && s < nRoots; s += gridDim.x) {
-        Board R = root;
-        if (pre == 1) R = small_make<SV>(root, sM1[s]);
-        if (pre == 2) {
-            const u32 e = sList[s];
-            R = small_make<SV>(sB1[e >> 16], e & 0xFFFFu);
-        }
-        if (tid == 0) sN = (u32)small_gen<SV>(R, sMR, 0, MAX_LEGAL_MOVES, 0u);
-        __syncthreads();
-        const u32 nA = sN;
-        if (nA > (u32)MAX_LEGAL_MOVES) {
-            flags = SMALL_OVERFLOW;
-            break;
-        }
-        for (u32 t = tid; t < nA; t += SMALL_NT) {
-            const u32 c = small_make_count<SV>(R, sMR[t], &sX[t]);
-            sC[t] = c;
-            if (r == 2) acc += c;
-        }
-        __syncthreads();
-        if (r == 2) continue;  // sMR, sC and sN are rewritten only after this barrier
-        const u32 T = small_scan<SMALL_NT>(sC, sOff, nA, swarp);
-        for (u32 w0 = 0; w0 < T; w0 += SMALL_WIN) {
-            const u32 wn = min(SMALL_WIN, T - w0);
-            for (u32 t = tid; t < nA; t += SMALL_NT) {
-                const u32 c = sC[t], off = sOff[t];
-                if (c && off + c > w0 && off < w0 + wn)
-                    small_gen<SV>(sX[t], sItems, (int)((long long)off - (long long)w0), wn, t << 16);
-            }
+    const u32 n1 = S.nItems;
+    if (!S.flags && tid == 0 && depth < 2) acc = depth == 0 ? 1u : n1;
+    if (depth >= 2 && !S.flags && n1) {
+        // the subtrees: this CTA's share of them
+        u32 s = slice, nSub = 1;
+        __syncthreads();  // every thread has read S.nItems and S.flags
+        small_list(S, SMALL_ROOT, 1);
+        if (depth == 4) {  // roots: the position's children
+            nSub = n1;
+            small_process(S, slice, n1, nSlices, SMALL_FIRST0);
             __syncthreads();
-            for (u32 j = tid; j < wn; j += SMALL_NT) {
-                const u32 it = sItems[j];
-                acc += small_make_count<SV>(sX[it >> 16], it & 0xFFFFu, nullptr);
-            }
+        } else if (depth == 5) {  // roots: its grandchildren
+            small_process(S, 0, n1, 1, SMALL_FIRST0);
             __syncthreads();
+            nSub = small_first(S, SMALL_FIRST0, (int)n1);
+            if (tid == 0 && nSub > P.listCap) S.flags |= SMALL_OVERFLOW;
+            __syncthreads();
+        }
+        // (flags are only read between two barriers with no position stored
+        // in between, so that every thread sees the same)
+        for (; s < nSub; s += nSlices) {
+            const bool stop = S.flags != 0;
+            __syncthreads();
+            if (stop) break;
+            int sub = SMALL_ROOT;
+            if (depth == 4) sub = SMALL_FIRST0 + (int)((s - slice) / nSlices);
+            if (depth == 5) {
+                // the s-th grandchild: the child it is below, and that child's moves
+                if (s != slice) small_first(S, SMALL_FIRST0, (int)n1);  // (the last subtree used the array)
+                int c = 0, e = (int)n1;
+                while (e - c > 1) {
+                    const int mid = (c + e) >> 1;
+                    if (S.first[mid] <= s) c = mid;
+                    else e = mid;
+                }
+                const u32 k = s - S.first[c];
+                small_list(S, SMALL_FIRST0 + c, 1);
+                small_process(S, k, k + 1, 1, SMALL_SUB);
+                __syncthreads();
+                if (S.flags) break;  // (the next position is stored behind small_list's barriers)
+                sub = SMALL_SUB;
+            }
+            const u32 T = sub == SMALL_ROOT ? n1 : S.cnt[sub];
+            if (sub != SMALL_ROOT) small_list(S, sub, 1);
+            if (depth == 2) {
+                acc += small_process(S, 0, T, 1, -1);
+                continue;
+            }
+            const u32 lo3 = part * T / split, hi3 = (part + 1) * T / split;
+            small_process(S, lo3, hi3, 1, SMALL_CHILD0);
+            __syncthreads();
+            // the children's moves, as many whole children at a time as the list holds
+            const int nC = (int)(hi3 - lo3);
+            const u32 all = small_first(S, SMALL_CHILD0, nC);
+            for (int w0 = 0; w0 < nC;) {
+                int w = nC - w0;
+                if (all - S.first[w0] > SMALL_ITEMS) {
+                    w = 1;
+                    while (S.first[w0 + w] + S.cnt[SMALL_CHILD0 + w0 + w] - S.first[w0] <= SMALL_ITEMS) w++;
+                }
+                small_list(S, SMALL_CHILD0 + w0, w);
+                acc += small_process(S, 0, ~0u, 1, -1);
+                __syncthreads();
+                w0 += w;
+            }
         }
     }
 
-    // per-CTA sum, then the last CTA to finish adds them up
+    // the CTA's sum into its position's; the last CTA hands everything over
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-    if (lane == 0) sSum[tid >> 5] = acc;
+    if (lane == 0 && acc) atomicAdd(&P.state->sum[at], acc);
     __syncthreads();
     if (tid == 0) {
-        unsigned long long t = 0;
-#pragma unroll
-        for (int i = 0; i < SMALL_NT / 32; i++) t += sSum[i];
-        S->partial[blockIdx.x] = t;
-        if (flags) atomicOr(&S->flagAcc, flags);
+        if (S.flags) atomicOr(&P.state->flags, S.flags);
         __threadfence();
-        sLast = atomicInc(&S->done, gridDim.x - 1) == gridDim.x - 1;
+        S.last = atomicAdd(&P.state->done, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (!sLast) return;
+    if (!S.last) return;
     __threadfence();
-    unsigned long long t = 0;
-    for (u32 i = tid; i < gridDim.x; i += SMALL_NT) t += __ldcg(&S->partial[i]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
-    if (lane == 0) sSum[tid >> 5] = t;
+    const u32 flags = __ldcg(&P.state->flags);
+    for (int i = tid; i < (int)P.n; i += SMALL_NT) {
+        const u64 c = __ldcg(&P.state->sum[i]);
+        P.host->count[i] = c;
+        if (P.dOut && !flags) P.dOut[i] = c;
+        P.state->sum[i] = 0;
+    }
     __syncthreads();
     if (tid == 0) {
-        unsigned long long sum = 0;
-#pragma unroll
-        for (int i = 0; i < SMALL_NT / 32; i++) sum += sSum[i];
-        const u32 all = atomicExch(&S->flagAcc, 0u) | flags;
-        S->count = all ? 0ull : sum;
-        S->flags = all;
-        if (!all) out[0] = sum;
+        P.host->flags = flags;
+        P.state->flags = 0;
+        P.state->done = 0;
     }
 }
 
@@ -1472,8 +1568,8 @@ class Engine {
 public:
     int init(const perft_config &cfg);
     void shutdown();
-    // trySmall: a single position of depth 2..5 tries the one-launch
-    // small-tree kernel first (false when the caller already tried it)
+    // trySmall: small trees try the one-launch kernel first (false when the
+    // caller already tried it)
     // related: the roots are a few moves apart from each other (related_roots)
     int run_batch(const u64 *dPos, const uint8_t *depths, u32 n, u64 *dOut, bool trySmall = true,
                   bool related = false);
@@ -1652,12 +1748,20 @@ private:
         u64 *hFlags = nullptr;         // pinned: overflow, device error, leaf items
     };
     std::vector<DDGraph> ddCache;
-    // one-launch small trees (k_small_tree)
+    // one-launch small trees (k_small_trees)
     SmallState *dSmall = nullptr;
+    SmallResult *hSmall = nullptr;  // mapped
     int smallGrid = 0;
     bool smallEnabled = true;
     u32 smallListCap = SMALL_LIST_CAP;
-    int run_small(const u64 *dPos, int depth, u64 *dOut, u64 *hOut, bool &handled);
+    // batches replay one captured launch whose parameters each call sets
+    SmallParams<SMALL_BATCH> smallBatch;
+    cudaGraph_t smallGraph = nullptr;
+    cudaGraphExec_t smallExec = nullptr;
+    cudaGraphNode_t smallNode = nullptr;
+    int run_small(const u64 *dPos, const u64 *pos, const uint8_t *depths, u32 n, u64 *dOut, u64 *hOut, bool &handled);
+    template <int N>
+    u32 small_params(SmallParams<N> &P, const u64 *dPos, const u64 *pos, const uint8_t *depths, u32 n, u64 *dOut);
     bool ddEnabled = true;
     bool ddForce = false;  // PERFT_DD_FORCE=1: skip the size estimate (tests the overflow fallback)
     double ddMaxBytes = DD_MAX_BYTES_DEFAULT;
@@ -1838,14 +1942,28 @@ int Engine::init(const perft_config &cfg)
     {
         ENG_TRY(cudaMalloc(&dSmall, sizeof(SmallState)));
         ENG_TRY(cudaMemset(dSmall, 0, sizeof(SmallState)));
-        ENG_TRY(cudaFuncSetAttribute(k_small_tree<SV_KOGGE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        ENG_TRY(cudaHostAlloc(&hSmall, sizeof(SmallResult), cudaHostAllocMapped));
+        ENG_TRY(cudaFuncSetAttribute(k_small_trees<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)SMALL_DYN_SMEM));
+        ENG_TRY(cudaFuncSetAttribute(k_small_trees<SMALL_BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)SMALL_DYN_SMEM));
         int perSm = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_small_tree<SV_KOGGE>, SMALL_NT, SMALL_DYN_SMEM) !=
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_small_trees<1>, SMALL_NT, SMALL_DYN_SMEM) !=
                 cudaSuccess ||
             perSm < 1)
             perSm = 1;
-        smallGrid = std::min(SMALL_MAX_GRID, perSm * nsm);
+        smallGrid = perSm * nsm;
+        ENG_TRY(cudaGraphCreate(&smallGraph, 0));
+        cudaKernelNodeParams kp = {};
+        void *args[] = {&smallBatch};
+        memset(&smallBatch, 0, sizeof smallBatch);
+        kp.func = (void *)k_small_trees<SMALL_BATCH>;
+        kp.gridDim = dim3(1);
+        kp.blockDim = dim3(SMALL_NT);
+        kp.sharedMemBytes = (unsigned)SMALL_DYN_SMEM;
+        kp.kernelParams = args;
+        ENG_TRY(cudaGraphAddKernelNode(&smallNode, smallGraph, nullptr, 0, &kp));
+        ENG_TRY(cudaGraphInstantiate(&smallExec, smallGraph, 0));
         smallEnabled = !(getenv("PERFT_SMALL_TREE") && getenv("PERFT_SMALL_TREE")[0] == '0');
         // PERFT_SMALL_LIST_CAP=k lists at most k depth-5 subtree roots per CTA:
         // a test setting that sends ordinary positions down the fallback
@@ -1900,8 +2018,14 @@ void Engine::shutdown()
     dTTStats = nullptr;
     cudaFree(dCounter);
     cudaFree(dErr);
+    if (smallExec) cudaGraphExecDestroy(smallExec);
+    if (smallGraph) cudaGraphDestroy(smallGraph);
+    smallExec = nullptr;
+    smallGraph = nullptr;
     if (dSmall) cudaFree(dSmall);
     dSmall = nullptr;
+    if (hSmall) cudaFreeHost(hSmall);
+    hSmall = nullptr;
     cudaFreeHost(hPinned);
     cudaEventDestroy(ev0);
     cudaEventDestroy(ev1);
@@ -2675,25 +2799,81 @@ int Engine::run_dd(const u64 *dPos, const uint8_t *depths, u32 n, u64 *dOut, boo
     return PERFT_OK;
 }
 
-// One position of depth 2..5: the whole tree in one k_small_tree launch and
-// one 16-byte read-back (count and flags).  Not handled (the level pipeline
-// runs it) when disabled, outside those depths, or when the position has more
-// depth-5 subtree roots than a CTA can list.  With hOut the count is also
-// returned to the host from the same read-back.
-int Engine::run_small(const u64 *dPos, int depth, u64 *dOut, u64 *hOut, bool &handled)
+// Fills the launch's parameters; returns the grid.  A depth-4 position has
+// SMALL_SLICES CTAs' worth of subtree roots and a depth-5 position fills the
+// device; subtrees are shared by more CTAs while the grid stays one wave.
+template <int N>
+u32 Engine::small_params(SmallParams<N> &P, const u64 *dPos, const u64 *pos, const uint8_t *depths, u32 n, u64 *dOut)
+{
+    P.dPos = dPos;
+    P.dOut = dOut;
+    P.host = hSmall;
+    P.state = dSmall;
+    P.n = n;
+    P.listCap = smallListCap;
+    u32 base = 0, n3 = 0, n4 = 0;
+    for (u32 i = 0; i < n; i++) {
+        n3 += depths[i] == 3;
+        n4 += depths[i] == 4;
+        base += depths[i] < 3;
+    }
+    auto total = [&](u32 k) { return base + n3 * k + n4 * k * SMALL_SLICES; };
+    u32 split = 1;
+    while (split < 8 && total(2 * split) <= (u32)smallGrid) split *= 2;
+    u32 grid = 0;
+    for (u32 i = 0; i < n; i++) {
+        P.unit0[i] = (uint16_t)grid;
+        P.depth[i] = depths[i];
+        P.split[i] = (uint8_t)(depths[i] == 3 || depths[i] == 4 ? split : 1);
+        grid += depths[i] == 5 ? (u32)smallGrid : depths[i] == 4 ? split * SMALL_SLICES : depths[i] == 3 ? split : 1;
+    }
+    P.unit0[n] = (uint16_t)grid;
+    if (!dPos) memcpy(P.pos, pos, 48ull * n);
+    return grid;
+}
+
+// One position of depth 2..5, or a batch of small ones: all trees in one
+// k_small_trees launch, positions passed as launch parameters when they are
+// on the host (dPos null), counts and flags written to mapped host memory.
+// Not handled (the level pipeline runs it) when disabled, when depths or
+// sizes are outside that, or when a position has more depth-5 subtree roots,
+// moves or pieces than the kernel holds.
+int Engine::run_small(const u64 *dPos, const u64 *pos, const uint8_t *depths, u32 n, u64 *dOut, u64 *hOut,
+                      bool &handled)
 {
     handled = false;
-    if (!smallEnabled || depth < 2 || depth > SMALL_MAX_DEPTH) return PERFT_OK;
-    k_small_tree<SV_KOGGE><<<smallGrid, SMALL_NT, SMALL_DYN_SMEM, stream>>>(dPos, depth, smallListCap, dOut,
-                                                                            dSmall);
-    ENG_TRY(cudaGetLastError());
-    ENG_TRY(cudaMemcpyAsync(hPinned + 4, &dSmall->count, 16, cudaMemcpyDeviceToHost, stream));
+    if (!smallEnabled) return PERFT_OK;
+    if (n == 1) {
+        if (depths[0] < 2 || depths[0] > SMALL_MAX_DEPTH) return PERFT_OK;
+        SmallParams<1> P;
+        const u32 grid = small_params(P, dPos, pos, depths, 1, dOut);
+        k_small_trees<1><<<grid, SMALL_NT, SMALL_DYN_SMEM, stream>>>(P);
+        ENG_TRY(cudaGetLastError());
+    } else {
+        if (n > (u32)SMALL_BATCH || tt || !ddEnabled) return PERFT_OK;
+        for (u32 i = 0; i < n; i++)
+            if (depths[i] > SMALL_BATCH_DEPTH) return PERFT_OK;
+        cudaKernelNodeParams kp = {};
+        void *args[] = {&smallBatch};
+        kp.func = (void *)k_small_trees<SMALL_BATCH>;
+        kp.gridDim = dim3(small_params(smallBatch, dPos, pos, depths, n, dOut));
+        kp.blockDim = dim3(SMALL_NT);
+        kp.sharedMemBytes = (unsigned)SMALL_DYN_SMEM;
+        kp.kernelParams = args;
+        ENG_TRY(cudaGraphExecKernelNodeSetParams(smallExec, smallNode, &kp));
+        ENG_TRY(cudaGraphLaunch(smallExec, stream));
+    }
     ENG_TRY(cudaStreamSynchronize(stream));
-    const u32 flags = (u32)hPinned[5];
+    const u32 flags = hSmall->flags;
     if (flags & DERR_BAD_POSITION) return PERFT_ERR_INVALID_ARG;
-    if (flags) return PERFT_OK;  // too many subtree roots for one CTA's list
-    if (hOut) *hOut = hPinned[4];
-    stats.small_launches += 1;
+    if (flags) return PERFT_OK;
+    if (hOut) memcpy(hOut, hSmall->count, 8ull * n);
+    if (n == 1) {
+        stats.small_launches += 1;
+    } else {
+        stats.graph_launches += 1;
+        stats.leaf_launches += 1;
+    }
     handled = true;
     return PERFT_OK;
 }
@@ -2727,6 +2907,9 @@ bool related_roots(const u64 *pos, const uint8_t *depths, u32 n)
 int Engine::run_batch_host(const u64 *pos, const uint8_t *depths, u32 n, u64 *out)
 {
     ENG_TRY(cudaSetDevice(device));  // the staging buffers and the stream belong to the engine's device
+    bool handled = false;
+    const int rcSmall = run_small(nullptr, pos, depths, n, nullptr, out, handled);
+    if (rcSmall != PERFT_OK || handled) return rcSmall;
     if (n > ioCap) {
         if (ioPos) cudaFree(ioPos);
         if (ioOut) cudaFree(ioOut);
@@ -2740,11 +2923,6 @@ int Engine::run_batch_host(const u64 *pos, const uint8_t *depths, u32 n, u64 *ou
         drop_dd();
     }
     ENG_TRY(cudaMemcpyAsync(ioPos, pos, 48ull * n, cudaMemcpyHostToDevice, stream));
-    if (n == 1) {
-        bool handled = false;
-        const int rc = run_small(ioPos, depths[0], ioOut, out, handled);
-        if (rc != PERFT_OK || handled) return rc;
-    }
     const int rc = run_batch(ioPos, depths, n, ioOut, false, related_roots(pos, depths, n));
     if (rc != PERFT_OK) return rc;
     ENG_TRY(cudaMemcpyAsync(out, ioOut, 8ull * n, cudaMemcpyDeviceToHost, stream));
@@ -2816,9 +2994,9 @@ int Engine::run_levels(const u64 *dPos, const uint8_t *depths, u32 n, unsigned l
 int Engine::run_batch(const u64 *dPos, const uint8_t *depths, u32 n, u64 *dOut, bool trySmall, bool related)
 {
     ENG_TRY(cudaSetDevice(device));
-    if (n == 1 && trySmall) {
+    if (trySmall) {
         bool handled = false;
-        const int rc = run_small(dPos, depths[0], dOut, nullptr, handled);
+        const int rc = run_small(dPos, nullptr, depths, n, dOut, nullptr, handled);
         if (rc != PERFT_OK || handled) return rc;
     }
     related = related && mergeEnabled;

@@ -672,6 +672,13 @@ PG_HD void rank_pair(u64 eGen, u64 oGen, u64 os, u64 targets, u64 &attacked, u32
     }
 }
 
+// What a count learned about its position that its moves depend on.
+struct MoveCtx {
+    u64 pinned;    // own pieces pinned to the king
+    u64 check;     // check mask: all squares when not in check, none in double check
+    u64 attacked;  // squares the king may not step to (own king transparent to a checker)
+};
+
 // countMoves for the Kogge-Stone variants, fused:
 //  * checkers come first, straight from the king square (pawn, knight and
 //    two slider lookups), so the check mask is known before any move count;
@@ -687,7 +694,8 @@ PG_HD void rank_pair(u64 eGen, u64 oGen, u64 os, u64 targets, u64 &attacked, u32
 // With OCC, occIn / theirsIn are the board's occupancy and the opponent's
 // pieces, which make-move already has.
 template <int SV, bool OCC = false>
-PG_HD u32 count_moves_fused(const Board &b, int ksqIn = -1, int tksqIn = -1, u64 occIn = 0, u64 theirsIn = 0)
+PG_HD u32 count_moves_fused(const Board &b, int ksqIn = -1, int tksqIn = -1, u64 occIn = 0, u64 theirsIn = 0,
+                            MoveCtx *ctx = nullptr)
 {
     constexpr int M = SvTraits<SV>::shift;
     const u64 pawns = b.pawns & RANKS2TO7;
@@ -786,6 +794,8 @@ PG_HD u32 count_moves_fused(const Board &b, int ksqIn = -1, int tksqIn = -1, u64
 #endif
     }
     attacked |= pawn_att_down(tP) | knight_set_att(tN) | PG_TAB(king[tksqIn >= 0 ? tksqIn : ctz(b.kings & theirs)]);
+
+    if (ctx) *ctx = MoveCtx{pinned, cm, attacked | xray};
 
     // king
     n = add_popc(n, PG_TAB(king[ksq]) & notMine & ~(attacked | xray));
@@ -1088,6 +1098,96 @@ PG_HD void gen_moves(const Board &b, Sink &out)
                 const bool ok = (s & pinned) ? (!inCheck && (PG_TAB(line[ctz(s)][c.ksq]) & target) != 0)
                                              : !ep_exposes_king(c, s, captured);
                 if (ok) out(encode_move(ctz(s) | mvP, 39 + epf, MF_EP));
+            }
+        }
+    }
+}
+
+// -------------------------------------------------- generation in parts
+// The legal moves of a position in GEN_PARTS parts, given its MoveCtx (which
+// the count of the position yields): parts are independent of each other, so
+// several threads share a position's generation, and none repeats the
+// attack map, the pins or the checkers.  The parts together emit exactly the
+// moves of gen_moves.  Before emitting n moves a part calls out.room(n): the
+// sink may place each run of moves where it likes.
+constexpr int GEN_PARTS = 4;
+enum GenPart : int { GP_LEAPERS = 0, GP_DIAGONAL, GP_ORTHOGONAL, GP_PAWNS };
+
+template <class Sink>
+PG_HD void gen_part(const Board &b, const MoveCtx &c, int part, Sink &out)
+{
+    const u64 pawns = b.pawns & RANKS2TO7;
+    const u64 occ = pawns | b.knights | b.bq | b.rq | b.kings;
+    const u64 mine = b.mine, theirs = occ ^ mine, empty = ~occ;
+    const u64 myK = b.kings & mine;
+    const u64 targets = ~mine & c.check;
+    const bool inCheck = c.check != ~0ULL;
+    const u32 st = (u32)(b.pawns & 0xFF);
+
+    if (part == GP_LEAPERS) {
+        const int ksq = ctz(myK);
+        const u64 row = myK | sh_e(myK) | sh_w(myK);
+        const u64 t = ((row | sh_n(row) | sh_s(row)) ^ myK) & ~mine & ~c.attacked;
+        const bool castleK = !inCheck && (st & 1) && !((occ | c.attacked) & 0x60ULL);
+        const bool castleQ = !inCheck && (st & 2) && !(occ & 0x0EULL) && !(c.attacked & 0x0CULL);
+        out.room(popc(t) + castleK + castleQ);
+        emit_targets(out, ksq, t);
+        if (castleK) out(encode_move(4, 6, MF_KING_CASTLE));
+        if (castleQ) out(encode_move(4, 2, MF_QUEEN_CASTLE));
+        for_each_bit(b.knights & mine & ~c.pinned, [&](int s) {
+            const u64 k = knight_set_att(1ULL << s) & targets;
+            out.room(popc(k));
+            emit_targets(out, s, k);
+        });
+    } else if (part != GP_PAWNS) {
+        // a pinned slider moves along its pin line, and never resolves a check
+        const bool diag = part == GP_DIAGONAL;
+        for_each_bit((diag ? b.bq : b.rq) & mine & (inCheck ? ~c.pinned : ~0ULL), [&](int s) {
+            const u64 bit = 1ULL << s;
+            u64 t = (diag ? ks_diag(bit, empty) : ks_orth(bit, empty)) & targets;
+            if (bit & c.pinned) t &= PG_TAB(line[s][ctz(myK)]);
+            out.room(popc(t));
+            emit_targets(out, s, t);
+        });
+    } else if (c.check) {
+        const u64 P = pawns & mine & ~c.pinned;
+        const u64 p1 = sh_n(P) & empty, push = p1 & c.check;
+        const u64 dbl = sh_n(p1 & RANK3) & empty & c.check;
+        const u64 capT = theirs & c.check;
+        const u64 cl = sh_nw(P) & capT, cr = sh_ne(P) & capT;
+        out.room(popc(push) + popc(dbl) + popc(cl) + popc(cr) + 3 * (popc_byte7(push) + popc_byte7(cl) + popc_byte7(cr)));
+        for_each_bit(push, [&](int to) { emit_pawn(out, to - 8, to, MF_QUIET); });
+        for_each_bit(dbl, [&](int to) { out(encode_move(to - 16, to, MF_DOUBLE_PUSH)); });
+        for_each_bit(cl, [&](int to) { emit_pawn(out, to - 7, to, MF_CAPTURE); });
+        for_each_bit(cr, [&](int to) { emit_pawn(out, to - 9, to, MF_CAPTURE); });
+        for_each_bit(inCheck ? 0 : pawns & mine & c.pinned, [&](int s) {
+            const u64 bit = 1ULL << s, line = PG_TAB(line[s][ctz(myK)]);
+            const u64 q1 = sh_n(bit) & empty & line;
+            const u64 q2 = sh_n(q1 & RANK3) & empty;
+            const u64 cap = pawn_att_up(bit) & theirs & line;  // the pinner
+            out.room(popc(q1) + popc(q2) + popc(cap) + 3 * popc_byte7(cap));
+            if (q1) out(encode_move(s, s + 8, MF_QUIET));
+            if (q2) out(encode_move(s, s + 16, MF_DOUBLE_PUSH));
+            if (cap) emit_pawn(out, s, ctz(cap), MF_CAPTURE);
+        });
+        const u32 epf = st >> 4;
+        if (epf) {
+            const u64 target = 1ULL << (39 + epf), captured = sh_s(target);
+            if (!inCheck || (captured & c.check)) {
+                for (u64 srcs = pawn_att_down(target) & pawns & mine; srcs; srcs &= srcs - 1) {
+                    const u64 sb = srcs & (0 - srcs);
+                    bool ok = true;
+                    if (sb & c.pinned) {
+                        ok = !inCheck && (PG_TAB(line[ctz(sb)][ctz(myK)]) & target) != 0;
+                    } else if (myK & RANK5) {
+                        const u64 pro = empty | sb | captured;
+                        ok = !((ks_east(myK, pro) | ks_west(myK, pro)) & b.rq & theirs);
+                    }
+                    if (ok) {
+                        out.room(1);
+                        out(encode_move(ctz(sb), 39 + epf, MF_EP));
+                    }
+                }
             }
         }
     }

@@ -1,0 +1,43 @@
+"""Batches of small trees in one launch (k_small_trees)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [2, 3, 31, 63, 64, 65])
+@pytest.mark.parametrize("depths", [(0, 4), (4, 4), (1, 3), (0, 0)])
+def test_small_batches_equal_oracle(engine, oracle, n, depths):
+    """Sizes around the largest batch of the one-launch kernel, depths 0-4,
+    host and device buffers."""
+    import torch
+    pos = engine.random_playouts(seed=300 + n, n=n, min_plies=0, max_plies=90)
+    d = np.random.default_rng(n).integers(depths[0], depths[1] + 1, size=n).astype(np.uint8)
+    want = oracle.perft_batch_mt(pos, d)
+    assert np.array_equal(engine.perft_batch(pos, d), want)
+    d_pos = torch.from_numpy(pos.view(np.int64)).cuda()
+    d_out = torch.full((n,), -1, dtype=torch.int64, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(2):
+        engine.perft_batch_device(d_pos.data_ptr(), d, n, d_out.data_ptr())
+        assert np.array_equal(d_out.cpu().numpy().view(np.uint64), want)
+
+
+def test_positions_the_kernel_cannot_hold(engine, oracle):
+    """A position with more pieces than move groups (and one with more moves
+    than any game's) goes to the level pipeline, alone and in a batch; an
+    invalid one is refused, and the next call is clean."""
+    queens = engine.fen_to_pos("QQQQQQQQ/QQQQQQQQ/QQQQQQQQ/8/8/8/7p/K6k b - - 0 1")
+    many = engine.fen_to_pos("3Q4/1Q4Q1/4Q3/2Q4R/Q4Q2/3Q4/1Q4Rp/1K1BBNNk w - - 0 1")  # 218 moves
+    start = engine.fen_to_pos(engine.START_FEN)
+    pos = np.stack([start, queens, many])
+    for d in (2, 3):
+        want = [oracle.perft(p, d) for p in pos]
+        assert [engine.perft(p, d) for p in pos] == want
+        assert [int(x) for x in engine.perft_batch(pos, d)] == want
+    bad = start.copy()
+    bad[5] = 0
+    with pytest.raises(engine.PerftError) as ei:
+        engine.perft_batch(np.stack([start, bad]), 3)
+    assert ei.value.status == engine.PERFT_ERR_INVALID_ARG
+    assert [int(x) for x in engine.perft_batch(np.stack([start, start]), 3)] == [8902, 8902]
