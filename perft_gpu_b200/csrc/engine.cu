@@ -699,8 +699,9 @@ struct MergeLevel {
     unsigned long long *weight;
     unsigned long long *set;
     MergeSeg *segs;
-    const uint8_t *rootDepth;
+    const uint8_t *rootDepth;  // null: every root is deep enough
     int remaining;  // plies left below the level
+    bool initWeight;  // the weights are not set yet: one path each
     // linked levels (below): each node's owner, and the subtree sums to clear
     u32 *alias;
     unsigned long long *acc;
@@ -733,8 +734,9 @@ __device__ __forceinline__ void merge_prepare(const MergeLevel &M)
     ulonglong2 *set2 = reinterpret_cast<ulonglong2 *>(M.set);
     for (u64 i = t0; i < M.n; i += step) {
         set2[i] = make_ulonglong2(MERGE_EMPTY, MERGE_EMPTY);
+        if (M.initWeight) M.weight[i] = 1ull;
         const u32 r = M.root[i];
-        const bool deep = M.rootDepth[r] >= M.remaining + MERGE_MIN_PLIES;
+        const bool deep = !M.rootDepth || M.rootDepth[r] >= M.remaining + MERGE_MIN_PLIES;
         if (i == 0 || M.root[i - 1] != r) M.segs[r].begin = deep ? (u32)i : 0u;
         if (i + 1 == M.n || M.root[i + 1] != r) M.segs[r].end = deep ? (u32)(i + 1) : 0u;
     }
@@ -801,7 +803,7 @@ __device__ __forceinline__ MergeLevel dd_merge_level(const DevPlan *plan, int lv
 {
     const LevelDesc &C = plan->lv[lv];
     return MergeLevel{C.planes, C.stride, C.set ? C.n : 0, C.cnt, C.root, C.weight, C.set,
-                      plan->segs, plan->rootDepth, remaining, nullptr, nullptr, nullptr};
+                      plan->segs, plan->rootDepth, remaining, false, nullptr, nullptr, nullptr};
 }
 __global__ void __launch_bounds__(256) k_dd_merge_prepare(const DevPlan *plan, int lv, int remaining)
 {
@@ -867,7 +869,7 @@ __global__ void __launch_bounds__(TILE_NT, TILE_MINB) k_tile(const TileParams Pi
     __shared__ u64 sqEnd[TRACK ? TILE_MAXP : 1];
     __shared__ int sdelta[TRACK ? TILE_MAXP : 1];
     __shared__ u32 sroot[TILE_MAXP];
-    __shared__ unsigned long long sweight[TRACK ? 1 : TILE_MAXP];  // paths that reach each parent
+    __shared__ unsigned long long sweight[TILE_MAXP];  // paths that reach each parent
     __shared__ u32 srun[TILE_MAXP];
     __shared__ u32 srunRoot[TILE_MAXP];
     __shared__ unsigned long long sacc[TILE_MAXP];
@@ -918,7 +920,7 @@ __global__ void __launch_bounds__(TILE_NT, TILE_MINB) k_tile(const TileParams Pi
                     skS[tid] = (uint8_t)ctz(pb.kings & pb.mine);
                 }
                 sroot[tid] = P.proot ? P.proot[node] : (u32)node;  // no root array: account to the parent itself
-                if (!TRACK) sweight[tid] = P.pweight ? P.pweight[node] : 1ull;
+                sweight[tid] = P.pweight ? P.pweight[node] : 1ull;
             }
             const u64 sBeg = max(P.pscan[p], iBeg);
             const u64 sEnd = min(P.pscan[p + nP], iEnd);
@@ -928,7 +930,7 @@ __global__ void __launch_bounds__(TILE_NT, TILE_MINB) k_tile(const TileParams Pi
             // a warp's 32 products of a weight below 2^WEIGHT_BITS and a count
             // (at most 218) sum below 2^32; windows with larger weights add
             // each product by itself
-            const bool narrow = TRACK || MODE == MODE_EXPAND || !P.pweight ||
+            const bool narrow = MODE == MODE_EXPAND || !P.pweight ||
                                 __syncthreads_and(!valid || (sweight[tid] >> WEIGHT_BITS) == 0);
             if (MODE == MODE_LEAF || TRACK) {
                 // parents are ordered by root: number the runs of equal roots.
@@ -996,19 +998,21 @@ __global__ void __launch_bounds__(TILE_NT, TILE_MINB) k_tile(const TileParams Pi
                             level_put(P.cpl, P.cstride, g, ch);
                             P.ccnt[g] = cnt;
                             P.croot[g] = sroot[pl];
-                            if (!TRACK && P.cweight) P.cweight[g] = sweight[pl];
+                            if (P.cweight) P.cweight[g] = sweight[pl];
                         }
                     } else {
                         atomicOr(P.err, DERR_BAD_ITEM);
                         pl = 0;
                     }
                 }
-                if (MODE == MODE_LEAF && !TRACK) {
-                    if (!narrow) {
+                if (MODE == MODE_LEAF) {
+                    if (narrow) {
+                        cnt *= (u32)sweight[pl];  // (idle lanes: 0)
+                    } else {
                         if (act) atomicAdd(&sacc[srun[pl]], (unsigned long long)cnt * sweight[pl]);
-                        continue;
+                        cnt = 0;
+                        if (!TRACK) continue;
                     }
-                    cnt *= (u32)sweight[pl];  // (idle lanes: 0)
                 }
                 if (PG_ONE_RUN_SUM && MODE == MODE_LEAF && !TRACK && nRuns == 1) {
                     // the whole window belongs to one root: a plain warp sum
@@ -1694,6 +1698,7 @@ public:
     u64 free_bytes() const { return arena_free(); }
     int device_id() const { return device; }
     int leaf_sliders() const { return svLeaf; }
+    bool merge_enabled() const { return mergeEnabled; }
     u64 blockMark = 0;
     // The transposition table as the server sees it (null table: none configured).
     struct TTView {
@@ -2054,7 +2059,7 @@ int Engine::merge_level(const Joiners &J, const DeviceLevel &C, int remaining)
     arenaTop = mark;  // free again once the merge has run (stream order)
     if (!set) return PERFT_OK;  // the level stays unmerged
     const MergeLevel M{C.planes, C.stride, C.n,       C.cnt,     C.root,  C.weight, set,
-                       J.segs,   J.depths, remaining, nullptr, nullptr, nullptr};
+                       J.segs,   J.depths, remaining, false,   nullptr, nullptr,  nullptr};
     const unsigned grid = (unsigned)std::min<u64>((C.n + 255) / 256, 64ull * nsm);
     k_merge_prepare<<<grid, 256, 0, stream>>>(M);
     k_merge_nodes<<<grid, 256, 0, stream>>>(M);
@@ -2433,7 +2438,7 @@ int Engine::process_level_tt(const DeviceLevel &L, int remaining, unsigned long 
     if (!set) return PERFT_ERR_OUT_OF_MEMORY;
     ENG_TRY(cudaMemsetAsync(set, 0xFF, 8 * MERGE_SLOTS * L.n, stream));
     const MergeLevel M{L.planes, L.stride, L.n,     L.cnt, nullptr, nullptr, set,
-                       nullptr,  nullptr,  remaining, L.alias, L.acc,   &dTTStats->aliases};
+                       nullptr,  nullptr,  remaining, false, L.alias, L.acc, &dTTStats->aliases};
     k_merge_linked<<<(unsigned)std::min<u64>(nb, 64ull * nsm), 256, 0, stream>>>(M);
     if (useTT)
         k_tt_probe<<<(unsigned)std::min<u64>(nb, 8ull * nsm), 256, 0, stream>>>(

@@ -62,12 +62,18 @@ __global__ void k_serve_admit(const u64 *__restrict__ stagePos, const u32 *__res
     pending[s] = depths[i] >= 2 ? 1ull : 0ull;
 }
 
-// Parents with no legal move end their branch at scan time.
+// Parents without items (no legal move, or merged into an equal node) end
+// their branch at scan time.  One atomic per warp and query: a merged level
+// has hundreds of thousands of them.
 __global__ void k_serve_zero_parents(const u32 *__restrict__ cnt, const u32 *__restrict__ root, u64 n,
                                      unsigned long long *pending)
 {
     const u64 i = (u64)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && cnt[i] == 0) atomicAdd(&pending[root[i]], ~0ull);  // -1
+    const bool zero = i < n && cnt[i] == 0;
+    const u32 key = zero ? root[i] : 0xFFFFFFFFu;
+    const unsigned peers = __match_any_sync(0xffffffffu, key);
+    if (zero && (int)(threadIdx.x & 31) == __ffs(peers) - 1)
+        atomicAdd(&pending[key], (unsigned long long)(-(long long)__popc(peers)));
 }
 
 struct ServeQuery {
@@ -121,7 +127,9 @@ __global__ void __launch_bounds__(256) k_serve_tt_finish(u64 n, const u64 *__res
 struct ServeLevel {
     DeviceLevel L;
     int r = 0;
+    int depth = 0;  // of its queries (a level's queries all have one depth)
     bool scanned = false;
+    bool merged = false;  // merged, or found not worth it
     bool tt = false;  // a table level: per-node sums, finished by k_serve_tt_finish
     // a remaining-depth-2 level expanded from a table level of remaining depth
     // 3: its root array holds parent indices into that level, its counts go
@@ -130,8 +138,9 @@ struct ServeLevel {
     int outstanding = 0;  // (table levels of remaining depth 3) child levels not yet finished
     std::vector<std::pair<u64, u64>> ttMem;  // its hashes, sums and aliases
     u64 *pscan = nullptr;
+    u32 *live = nullptr;  // merged and table levels: the nodes with items
     u32 *tileFirst = nullptr;
-    u64 total = 0, next = 0;
+    u64 nParents = 0, total = 0, next = 0;
     std::vector<std::pair<u64, u64>> mem;  // (offset, bytes) in the server block
 };
 
@@ -165,6 +174,7 @@ private:
     int scan_level(ServeLevel &S);
     int launch(int mode, ServeLevel &S, u64 lo, u64 hi, DeviceLevel *child);
     int probe_level(ServeLevel &S);
+    int merge_level(ServeLevel &S);
     int finish_level(ServeLevel &S);
     int retire(ServeLevel *S);
     std::vector<ServeLevel *> waiting;  // table levels fully expanded, waiting for their child levels
@@ -184,6 +194,8 @@ private:
     u32 *dErr = nullptr, *dCounter = nullptr;
     u64 *posBySlot = nullptr;
     unsigned long long *pending = nullptr, *counts = nullptr;
+    MergeSeg *segs = nullptr;  // per slot: its nodes in the level being merged
+    bool mergeEnabled = true;
     u64 *hostPending = nullptr, *hostCounts = nullptr, *hostTotal = nullptr;  // pinned
     u64 *stagePos = nullptr;   // pinned
     u32 *stageSlots = nullptr; // pinned
@@ -261,10 +273,12 @@ int Server::start(const perft_serve_config &cfg, char *block, u64 bytes, int dev
     posBySlot = (u64 *)take(48ull * SERVE_MAX_SLOTS, fixedMem);
     pending = (unsigned long long *)take(8ull * SERVE_MAX_SLOTS, fixedMem);
     counts = (unsigned long long *)take(8ull * SERVE_MAX_SLOTS, fixedMem);
+    segs = (MergeSeg *)take(sizeof(MergeSeg) * SERVE_MAX_SLOTS, fixedMem);
+    mergeEnabled = g_engine.merge_enabled();
     dCounter = (u32 *)take(256, fixedMem);
     dErr = (u32 *)take(256, fixedMem);
     dTTStats = (TTStats *)take(256, fixedMem);
-    if (!posBySlot || !pending || !counts || !dCounter || !dErr || !dTTStats) return PERFT_ERR_OUT_OF_MEMORY;
+    if (!posBySlot || !pending || !counts || !segs || !dCounter || !dErr || !dTTStats) return PERFT_ERR_OUT_OF_MEMORY;
     if (cudaMemsetAsync(dErr, 0, 4, st) != cudaSuccess) return PERFT_ERR_CUDA;
     if (cudaMemsetAsync(dTTStats, 0, sizeof(TTStats), st) != cudaSuccess) return PERFT_ERR_CUDA;
     {
@@ -474,7 +488,7 @@ int Server::admit()
         u32 i1 = i0;
         while (i1 < n && batch[i1]->depth == depth) i1++;
         ServeLevel *S = new ServeLevel();
-        S->r = (int)depth;
+        S->r = S->depth = (int)depth;
         const u64 cnt = i1 - i0;
         S->L.n = cnt;
         S->L.stride = (cnt + 31) & ~31ULL;
@@ -522,13 +536,50 @@ int Server::probe_level(ServeLevel &S)
     const unsigned nb = (unsigned)((n + 255) / 256);
     if (cudaMemsetAsync(set, 0xFF, 8 * MERGE_SLOTS * n, st) != cudaSuccess) return PERFT_ERR_CUDA;
     const MergeLevel M{S.L.planes, S.L.stride, n,   S.L.cnt,   nullptr, nullptr, set,
-                       nullptr,    nullptr,    S.r, S.L.alias, S.L.acc, &dTTStats->aliases};
+                       nullptr,    nullptr,    S.r, false,     S.L.alias, S.L.acc, &dTTStats->aliases};
     k_merge_linked<<<std::min(nb, 64u * nsm), 256, 0, st>>>(M);
     k_tt_probe<<<std::min(nb, 8u * nsm), 256, 0, st>>>(S.L.planes, S.L.stride, n, S.r, ttKeyMask, S.L.cnt, S.L.hash,
                                                        S.L.hash2, S.L.acc, S.L.alias, tt, ttMask, dTTStats);
     launches += 2;
     give_back(tmp);  // reused only by later launches on this stream
     S.tt = true;
+    return cudaGetLastError() == cudaSuccess ? PERFT_OK : PERFT_ERR_CUDA;
+}
+
+// Merges the equal nodes of each query's part of a level, as the engine's
+// levels do: nodes at least MERGE_MIN_PLIES below their query's position.
+// Small levels stay as they are (two launches would cost more than their
+// copies), and so do levels while less than a quarter of the server's memory
+// is free: weights and set must not displace admitted work.  A server with a
+// table merges its table levels instead (probe_level).
+// 200 queries of depths 3-6 submitted at once: 66.1 -> 28.5 ms.
+constexpr u64 SERVE_MERGE_MIN = 4096;
+int Server::merge_level(ServeLevel &S)
+{
+    const u64 n = S.L.n;
+    if (!mergeEnabled || tt || S.r + MERGE_MIN_PLIES > S.depth || n < SERVE_MERGE_MIN ||
+        blockBytes - inUse < blockBytes / 4)
+        return PERFT_OK;
+    std::vector<std::pair<u64, u64>> tmp, own;
+    const bool init = S.L.weight == nullptr;
+    unsigned long long *weight = init ? (unsigned long long *)take(8 * S.L.stride, own) : S.L.weight;
+    unsigned long long *set = (unsigned long long *)take(8 * MERGE_SLOTS * n, tmp);
+    S.live = (u32 *)take(4 * n, own);
+    if (!weight || !set || !S.live) {
+        S.live = nullptr;
+        give_back(tmp);
+        give_back(own);
+        return PERFT_OK;
+    }
+    S.mem.insert(S.mem.end(), own.begin(), own.end());
+    S.L.weight = weight;
+    const MergeLevel M{S.L.planes, S.L.stride,  n,   S.L.cnt, S.L.root, weight, set,
+                       segs,       nullptr,     S.r, init,    nullptr,  nullptr, nullptr};
+    const unsigned grid = std::min((unsigned)((n + 255) / 256), 64u * nsm);
+    k_merge_prepare<<<grid, 256, 0, st>>>(M);
+    k_merge_nodes<<<grid, 256, 0, st>>>(M);
+    launches += 2;
+    give_back(tmp);  // reused only by later launches on this stream
     return cudaGetLastError() == cudaSuccess ? PERFT_OK : PERFT_ERR_CUDA;
 }
 
@@ -579,6 +630,12 @@ int Server::scan_level(ServeLevel &S)
         const int rc = probe_level(S);
         if (rc != PERFT_OK) return rc;
     }
+    if (!S.merged) {
+        const int rc = merge_level(S);
+        if (rc != PERFT_OK) return rc;
+        S.merged = true;  // (a scan that finds no memory is retried)
+    }
+    if (S.tt && !S.live) S.live = (u32 *)take(4 * S.L.n, S.mem);  // hits and copies make no parents (without: all do)
     const u64 n = S.L.n;
     const u64 nb = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
     const u64 maxTiles = (n * MAX_LEGAL_MOVES) / MAX_TILES_PER_NODE_DIV + 2;
@@ -593,19 +650,23 @@ int Server::scan_level(ServeLevel &S)
     k_scan_reduce<<<(unsigned)nb, SCAN_NT, 0, st>>>(S.L.cnt, n, bsum);
     u64 *totals = (u64 *)(bsum + nb);
     k_scan_top<<<1, SCAN_TOP_NT, 0, st>>>(bsum, nb, totals);
-    k_scan_apply<false><<<(unsigned)nb, SCAN_NT, SCAN_DYN_SMEM, st>>>(S.L.cnt, n, bsum, totals, S.pscan, nullptr,
-                                                                    S.tileFirst, TILE_CAP_LOG2);
+    if (S.live)
+        k_scan_apply<true><<<(unsigned)nb, SCAN_NT, SCAN_DYN_SMEM, st>>>(S.L.cnt, n, bsum, totals, S.pscan, S.live,
+                                                                       S.tileFirst, TILE_CAP_LOG2);
+    else
+        k_scan_apply<false><<<(unsigned)nb, SCAN_NT, SCAN_DYN_SMEM, st>>>(S.L.cnt, n, bsum, totals, S.pscan, nullptr,
+                                                                        S.tileFirst, TILE_CAP_LOG2);
     launches += 3;
     // a table level's nodes leave the pending count in its finish pass
     if (!S.tt) {
         k_serve_zero_parents<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(S.L.cnt, S.L.root, n, pending);
         launches++;
     }
-    give_back(tmp);
-    if (cudaMemcpyAsync(hostTotal, S.pscan + n, 8, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-        cudaStreamSynchronize(st) != cudaSuccess)
-        return PERFT_ERR_CUDA;
+    const bool readOk = cudaMemcpyAsync(hostTotal, totals, 16, cudaMemcpyDeviceToHost, st) == cudaSuccess;
+    give_back(tmp);  // reused only by later launches on this stream
+    if (!readOk || cudaStreamSynchronize(st) != cudaSuccess) return PERFT_ERR_CUDA;
     S.total = hostTotal[0];
+    S.nParents = S.live ? hostTotal[1] : n;
     S.scanned = true;
     return PERFT_OK;
 }
@@ -618,7 +679,9 @@ int Server::launch(int mode, ServeLevel &S, u64 lo, u64 hi, DeviceLevel *child)
     P.pstride = S.L.stride;
     P.pscan = S.pscan;
     P.proot = S.L.root;
-    P.nParents = S.L.n;
+    P.live = S.live;
+    P.pweight = S.L.weight;
+    P.nParents = S.nParents;
     P.tileFirst = S.tileFirst;
     P.itemBase = lo;
     P.itemEnd = hi;
@@ -629,6 +692,7 @@ int Server::launch(int mode, ServeLevel &S, u64 lo, u64 hi, DeviceLevel *child)
         P.cstride = child->stride;
         P.ccnt = child->cnt;
         P.croot = child->root;
+        P.cweight = child->weight;
     }
     P.rootCounts = counts;
     P.pending = pending;
@@ -686,13 +750,15 @@ int Server::advance()
                     for (;;) {  // shrink the step until the children fit
                         C = new ServeLevel();
                         C->r = r - 1;
+                        C->depth = S->depth;
                         const u64 m = hi - lo;
                         C->L.n = m;
                         C->L.stride = (m + 31) & ~31ULL;
                         C->L.planes = (u64 *)take(48 * C->L.stride, C->mem);
                         C->L.cnt = (u32 *)take(4 * C->L.stride, C->mem);
                         C->L.root = (u32 *)take(4 * C->L.stride, C->mem);
-                        if (C->L.planes && C->L.cnt && C->L.root) break;
+                        if (S->L.weight) C->L.weight = (unsigned long long *)take(8 * C->L.stride, C->mem);
+                        if (C->L.planes && C->L.cnt && C->L.root && (C->L.weight || !S->L.weight)) break;
                         give_back(C->mem);
                         delete C;
                         C = nullptr;

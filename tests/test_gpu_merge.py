@@ -105,3 +105,19 @@ def test_arena_without_room_for_the_set(engine, oracle):
                 assert engine.perft(start, 6) == want == 119_060_324
     finally:
         engine.init(device=0, arena_bytes=8 << 30)
+
+
+def test_served_few_pieces(engine):
+    """The server's merged levels: weights beyond the narrow sums' limit, and
+    queries of one level that merge next to each other."""
+    fens = ["4k3/8/8/8/8/8/8/4K3 w - - 0 1", "8/8/3k4/3p4/3P4/3K4/8/8 b - - 0 1", "k7/8/8/8/8/8/8/7K b - - 0 1"]
+    pos = [engine.fen_to_pos(f) for f in fens]
+    memo = {}
+    queries = [(p, d) for d in (6, 9, 13) for p in pos]
+    engine.serve_start()
+    try:
+        tickets = [engine.serve_submit(p, d) for p, d in queries]
+        got = [engine.serve_wait(t, timeout_s=120)[0] for t in tickets]
+    finally:
+        engine.serve_stop()
+    assert got == [_count(engine, p, d, memo) for p, d in queries]
