@@ -23,11 +23,12 @@
 //     and steals tiles from an atomic counter.  Per tile it stages the
 //     parents in shared memory, generates their moves into a compact shared
 //     item list (only the moves inside the tile window), then every thread
-//     takes items: make the move, count the child's legal moves.  Interior
-//     plies write the child (coalesced: item order is child order) and its
-//     count; the last ply only sums counts per root, warp-aggregated with
-//     match/reduce before a shared-memory accumulator and one global atomic
-//     per root run.
+//     takes items: make the move, count the child's legal moves, write the
+//     child (coalesced: item order is child order) and its count.
+//   * The last ply writes nothing: its kernel sums the replies to quiet moves
+//     from the parent alone, makes and counts only the other moves, and sums
+//     per root in a shared-memory accumulator with one global atomic per run.
+//   * Equal nodes of a level are merged before it is expanded.
 //   * When a level does not fit the HBM arena, its item range is split at
 //     tile boundaries and the chunks are expanded depth-first.
 #include <cuda_runtime.h>
@@ -85,6 +86,9 @@ constexpr int TILE_MIN_LOG2 = 10;  // small levels use tiles down to 1024 items 
 constexpr u64 MAX_TILES_PER_NODE_DIV = 1ull << TILE_MIN_LOG2;
 constexpr int TILE_MAXP = TILE_NT;
 constexpr int WEIGHT_BITS = 19;
+// The count-only ply's item list: a tile's parents, whole (the last one may
+// reach past the tile's end; no position has as many moves as the slack).
+constexpr u32 LEAF_ITEMS = TILE_CAP + 512;
 constexpr int TILE_MINB = PG_TILE_MINB;          // resident CTAs per SM the register budget targets
 constexpr int MAX_LEGAL_MOVES = 218;
 
@@ -835,6 +839,25 @@ struct WindowSink {
     }
 };
 
+// Makes an item's move on its (mirrored) parent and counts the child's moves.
+template <int SV>
+__device__ __forceinline__ u32 tile_make_count(const Board &b, u32 it, int kO, int kS, Board &ch)
+{
+    if (PG_KNOWN_KINGS && PG_MIRRORED_STAGE && PG_KNOWN_OCC) {
+        int tk;
+        u64 occ, theirs;
+        ch = make_child_mirrored(b, it, &tk, kS, &occ, &theirs);
+        return count_moves_ko<SV>(ch, kO, tk, occ, theirs);
+    }
+    if (PG_KNOWN_KINGS && PG_MIRRORED_STAGE) {
+        int tk;
+        ch = make_child_mirrored(b, it, &tk, kS);
+        return count_moves_k<SV>(ch, kO, tk);
+    }
+    ch = PG_MIRRORED_STAGE ? make_child_mirrored(b, it) : make_child<PG_MOVER_BITS>(b, it);
+    return count_moves<SV>(ch);
+}
+
 // TRACK (serving): besides the counts, every root run also accumulates the
 // change of its query's pending-node counter: +1 per child written, -1 when
 // a parent's last item is processed.  The counter reaching zero means the
@@ -842,7 +865,7 @@ struct WindowSink {
 // DD: 0 for plain launches (parameters in the parameter bank); DD_SHARED or
 // DD_CONST for the device-driven graph's launches (below).
 enum { DD_NONE = 0, DD_SHARED = 1, DD_CONST = 2 };
-template <int MODE, int SV, bool TRACK = false, int DD = DD_NONE>
+template <int SV, bool TRACK = false, int DD = DD_NONE>
 __global__ void __launch_bounds__(TILE_NT, TILE_MINB) k_tile(const TileParams Pin)
 {
     // Device-driven launches take the level pointers and sizes from the plan:
@@ -870,9 +893,8 @@ __global__ void __launch_bounds__(TILE_NT, TILE_MINB) k_tile(const TileParams Pi
     __shared__ int sdelta[TRACK ? TILE_MAXP : 1];
     __shared__ u32 sroot[TILE_MAXP];
     __shared__ unsigned long long sweight[TILE_MAXP];  // paths that reach each parent
-    __shared__ u32 srun[TILE_MAXP];
-    __shared__ u32 srunRoot[TILE_MAXP];
-    __shared__ unsigned long long sacc[TILE_MAXP];
+    __shared__ u32 srun[TRACK ? TILE_MAXP : 1];
+    __shared__ u32 srunRoot[TRACK ? TILE_MAXP : 1];
     extern __shared__ __align__(16) u32 sitems[];  // TILE_CAP items (dynamic: may exceed 48 KB)
     __shared__ int swarp[TILE_NT / 32];
     __shared__ u32 sTile;
@@ -927,12 +949,7 @@ __global__ void __launch_bounds__(TILE_NT, TILE_MINB) k_tile(const TileParams Pi
             __syncthreads();
 
             int nRuns = 0;
-            // a warp's 32 products of a weight below 2^WEIGHT_BITS and a count
-            // (at most 218) sum below 2^32; windows with larger weights add
-            // each product by itself
-            const bool narrow = MODE == MODE_EXPAND || !P.pweight ||
-                                __syncthreads_and(!valid || (sweight[tid] >> WEIGHT_BITS) == 0);
-            if (MODE == MODE_LEAF || TRACK) {
+            if (TRACK) {
                 // parents are ordered by root: number the runs of equal roots.
                 // Usually the whole window belongs to one root, which one
                 // block vote settles without the two-barrier run count.
@@ -941,8 +958,7 @@ __global__ void __launch_bounds__(TILE_NT, TILE_MINB) k_tile(const TileParams Pi
                     if (valid) srun[tid] = 0;
                     if (tid == 0) {
                         srunRoot[0] = sroot[0];
-                        sacc[0] = 0ull;
-                        if (TRACK) sdelta[0] = 0;
+                        sdelta[0] = 0;
                     }
                 } else {
                     const bool head = valid && (tid == 0 || sroot[tid] != sroot[tid - 1]);
@@ -950,8 +966,7 @@ __global__ void __launch_bounds__(TILE_NT, TILE_MINB) k_tile(const TileParams Pi
                     if (valid) srun[tid] = head ? r : r - 1;
                     if (head) {
                         srunRoot[r] = sroot[tid];
-                        sacc[r] = 0ull;
-                        if (TRACK) sdelta[r] = 0;
+                        sdelta[r] = 0;
                     }
                 }
             }
@@ -967,12 +982,11 @@ __global__ void __launch_bounds__(TILE_NT, TILE_MINB) k_tile(const TileParams Pi
             }
             __syncthreads();
 
-            // ---- every thread takes items: make, count, write or sum
+            // ---- every thread takes items: make, count, write
             const int nItems = (int)(sEnd - sBeg);
             for (int j0 = 0; j0 < nItems; j0 += TILE_NT) {
                 const int j = j0 + tid;
                 const bool act = j < nItems;
-                u32 cnt = 0;
                 int pl = 0;
                 if (act) {
                     const u32 it = sitems[j];  // move (bits 0-15), parent slot (16-23), mover planes (24-28)
@@ -980,66 +994,227 @@ __global__ void __launch_bounds__(TILE_NT, TILE_MINB) k_tile(const TileParams Pi
                     if (pl < nP) {
                         const Board b{sb[0][pl], sb[1][pl], sb[2][pl], sb[3][pl], sb[4][pl], sb[5][pl]};
                         Board ch;
-                        if (PG_KNOWN_KINGS && PG_MIRRORED_STAGE && PG_KNOWN_OCC) {
-                            int tk;
-                            u64 occ, theirs;
-                            ch = make_child_mirrored(b, it, &tk, skS[pl], &occ, &theirs);
-                            cnt = count_moves_ko<SV>(ch, skO[pl], tk, occ, theirs);
-                        } else if (PG_KNOWN_KINGS && PG_MIRRORED_STAGE) {
-                            int tk;
-                            ch = make_child_mirrored(b, it, &tk, skS[pl]);
-                            cnt = count_moves_k<SV>(ch, skO[pl], tk);
-                        } else {
-                            ch = PG_MIRRORED_STAGE ? make_child_mirrored(b, it) : make_child<PG_MOVER_BITS>(b, it);
-                            cnt = count_moves<SV>(ch);
-                        }
-                        if (MODE == MODE_EXPAND) {
-                            const u64 g = sBeg + (u64)j - P.itemBase;
-                            level_put(P.cpl, P.cstride, g, ch);
-                            P.ccnt[g] = cnt;
-                            P.croot[g] = sroot[pl];
-                            if (P.cweight) P.cweight[g] = sweight[pl];
-                        }
+                        const u32 cnt = tile_make_count<SV>(b, it, skO[PG_KNOWN_KINGS ? pl : 0],
+                                                            skS[PG_KNOWN_KINGS ? pl : 0], ch);
+                        const u64 g = sBeg + (u64)j - P.itemBase;
+                        level_put(P.cpl, P.cstride, g, ch);
+                        P.ccnt[g] = cnt;
+                        P.croot[g] = sroot[pl];
+                        if (P.cweight) P.cweight[g] = sweight[pl];
                     } else {
                         atomicOr(P.err, DERR_BAD_ITEM);
                         pl = 0;
                     }
                 }
-                if (MODE == MODE_LEAF) {
-                    if (narrow) {
-                        cnt *= (u32)sweight[pl];  // (idle lanes: 0)
-                    } else {
-                        if (act) atomicAdd(&sacc[srun[pl]], (unsigned long long)cnt * sweight[pl]);
-                        cnt = 0;
-                        if (!TRACK) continue;
-                    }
-                }
-                if (PG_ONE_RUN_SUM && MODE == MODE_LEAF && !TRACK && nRuns == 1) {
-                    // the whole window belongs to one root: a plain warp sum
-                    // (idle lanes hold 0), no grouping by root
-                    const u32 sum = __reduce_add_sync(0xffffffffu, cnt);
-                    if (lane == 0 && sum) atomicAdd(&sacc[0], (unsigned long long)sum);
-                } else if (MODE == MODE_LEAF || TRACK) {
+                if (TRACK) {
                     const u32 key = act ? srun[pl] : 0xFFFFFFFFu;
                     const unsigned peers = __match_any_sync(0xffffffffu, key);
-                    if (MODE == MODE_LEAF) {
-                        const u32 sum = __reduce_add_sync(peers, cnt);
-                        if (act && lane == __ffs(peers) - 1) atomicAdd(&sacc[key], (unsigned long long)sum);
-                    }
-                    if (TRACK) {
-                        const bool lastOfParent = act && (sBeg + (u64)j + 1 == sqEnd[pl]);
-                        const int d = (act && MODE == MODE_EXPAND ? 1 : 0) - (lastOfParent ? 1 : 0);
-                        const int dsum = __reduce_add_sync(peers, d);
-                        if (act && lane == __ffs(peers) - 1 && dsum) atomicAdd(&sdelta[key], dsum);
-                    }
+                    const bool lastOfParent = act && (sBeg + (u64)j + 1 == sqEnd[pl]);
+                    const int d = (act ? 1 : 0) - (lastOfParent ? 1 : 0);
+                    const int dsum = __reduce_add_sync(peers, d);
+                    if (act && lane == __ffs(peers) - 1 && dsum) atomicAdd(&sdelta[key], dsum);
                 }
             }
             __syncthreads();
-            if (MODE == MODE_LEAF && tid < nRuns) atomicAdd(&P.rootCounts[srunRoot[tid]], sacc[tid]);
             if (TRACK && tid < nRuns && sdelta[tid])
                 atomicAdd(&P.pending[srunRoot[tid]], (unsigned long long)(long long)sdelta[tid]);
             if (sEnd >= iEnd || p + nP >= P.nParents) break;
             p += nP;
+            __syncthreads();
+        }
+        __syncthreads();
+    }
+}
+
+// -------------------------------------------------------- count-only last ply
+// Counts the replies to every move of a level's parents (remaining depth 2)
+// and adds weight x replies per root.  One thread generates a parent's moves;
+// the replies to its quiet moves, about two thirds, are summed from the
+// position alone (movegen.cuh, QuietCtx) without making the moves, and only
+// the rest go to the shared item list, where every thread takes items, makes
+// the move and counts.  A parent belongs to the tile that holds its first
+// item, so that no parent is split.
+//
+// Bound by the integer pipes: a counted item issues about 900 thread
+// instructions, a parent's own analysis about 2500 and a set of quiet moves
+// about 60, so counting a third of the 33 items and analysing once is about
+// half of counting all of them.  Measured against making and counting every
+// item: 4096 playouts of depths 4-6 656 -> 452 ms, depth 7 5.98 -> 4.71 ms,
+// opening at depth 8 17.7 -> 11.4 ms.
+struct LeafSink {
+    u32 *items;
+    u32 *count;
+    u32 at, tag, n;
+    __device__ __forceinline__ void room(int k)
+    {
+        at = atomicAdd(count, (u32)k);
+        n += (u32)k;
+    }
+    __device__ __forceinline__ void operator()(u32 m)
+    {
+        if (at < LEAF_ITEMS) items[at] = tag | m;
+        ++at;
+    }
+};
+
+template <int SV, bool TRACK = false, int DD = DD_NONE>
+__global__ void __launch_bounds__(TILE_NT, TILE_MINB) k_leaf(const TileParams Pin)
+{
+    __shared__ TileParams sP;  // (see k_tile)
+    if (DD == DD_SHARED) {
+        if (threadIdx.x == 0) sP = *Pin.planEntry;
+        __syncthreads();
+    }
+    const TileParams &P = DD == DD_CONST ? c_ddTile : (DD == DD_SHARED ? sP : Pin);
+    __shared__ u64 sb[6][TILE_MAXP];
+    __shared__ uint8_t skO[PG_KNOWN_KINGS ? TILE_MAXP : 1], skS[PG_KNOWN_KINGS ? TILE_MAXP : 1];
+    __shared__ u32 sroot[TILE_MAXP];
+    __shared__ unsigned long long sweight[TILE_MAXP];  // paths that reach each parent
+    __shared__ u32 srun[TILE_MAXP];
+    __shared__ u32 srunRoot[TILE_MAXP];
+    __shared__ unsigned long long sacc[TILE_MAXP];
+    __shared__ int sdelta[TRACK ? TILE_MAXP : 1];
+    extern __shared__ __align__(16) u32 sitems[];  // LEAF_ITEMS
+    __shared__ int swarp[TILE_NT / 32];
+    __shared__ u32 sTile, sCount;
+
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int capLog2 = P.capLog2;
+    const u64 tile0 = P.itemBase >> capLog2;
+    const u64 nTiles = (P.itemEnd - P.itemBase + (1ull << capLog2) - 1) >> capLog2;
+
+    for (;;) {
+        if (tid == 0) sTile = atomicAdd(P.tileCounter, 1u);
+        __syncthreads();
+        const u64 tl = sTile;
+        if (tl >= nTiles) break;
+        const u64 iBeg = P.itemBase + (tl << capLog2);
+        const u64 iEnd = min(iBeg + ((u64)1 << capLog2), P.itemEnd);
+        u64 p = P.tileFirst[tile0 + tl];
+        if (P.pscan[p] < iBeg) p++;  // begins in the tile before
+
+        for (;;) {
+            // ---- stage the parents whose first item lies in the tile
+            const u64 q = p + tid;
+            u64 qBeg = 0;
+            bool valid = false;
+            if (q < P.nParents) {
+                qBeg = P.pscan[q];
+                valid = qBeg < iEnd;
+            }
+            const int nP = __syncthreads_count(valid);
+            if (nP == 0) break;
+            u32 nMoves = 0;
+            if (tid == 0) sCount = 0;
+            if (valid) {
+                nMoves = (u32)(P.pscan[q + 1] - qBeg);
+                const u64 node = P.live ? P.live[q] : q;
+                const Board pb = flip_board(level_get(P.ppl, P.pstride, node));  // mirrored (see k_tile)
+                sb[0][tid] = pb.mine;
+                sb[1][tid] = pb.pawns;
+                sb[2][tid] = pb.knights;
+                sb[3][tid] = pb.bq;
+                sb[4][tid] = pb.rq;
+                sb[5][tid] = pb.kings;
+                if (PG_KNOWN_KINGS) {
+                    skO[tid] = (uint8_t)ctz(pb.kings & ~pb.mine);
+                    skS[tid] = (uint8_t)ctz(pb.kings & pb.mine);
+                }
+                sroot[tid] = P.proot ? P.proot[node] : (u32)node;  // no root array: account to the parent itself
+                sweight[tid] = P.pweight ? P.pweight[node] : 1ull;
+            }
+            __syncthreads();
+
+            // ---- the runs of equal roots (parents are ordered by root)
+            int nRuns = 0;
+            if (PG_ONE_RUN_VOTE && __syncthreads_and(!valid || sroot[tid] == sroot[0])) {
+                nRuns = 1;
+                if (valid) srun[tid] = 0;
+                if (tid == 0) {
+                    srunRoot[0] = sroot[0];
+                    sacc[0] = 0ull;
+                    if (TRACK) sdelta[0] = 0;
+                }
+            } else {
+                const bool head = valid && (tid == 0 || sroot[tid] != sroot[tid - 1]);
+                const int r = block_excl_count<TILE_NT>(head, swarp, nRuns);
+                if (valid) srun[tid] = head ? r : r - 1;
+                if (head) {
+                    srunRoot[r] = sroot[tid];
+                    sacc[r] = 0ull;
+                    if (TRACK) sdelta[r] = 0;
+                }
+            }
+            // a warp's 32 products of a weight below 2^WEIGHT_BITS and a count
+            // (at most 218) sum below 2^32; windows with larger weights add
+            // each product by itself
+            const bool narrow = !P.pweight || __syncthreads_and(!valid || (sweight[tid] >> WEIGHT_BITS) == 0);
+
+            // ---- generate: quiet moves are counted here, the rest is listed
+            u32 quietReplies = 0;
+            if (nMoves) {
+                const Board f{sb[0][tid], sb[1][tid], sb[2][tid], sb[3][tid], sb[4][tid], sb[5][tid]};
+                QuietCtx qc;
+                quiet_setup(f, qc);
+                quiet_flip(qc);
+                LeafSink sink{sitems, &sCount, 0u, (u32)tid << 16, 0u};
+                u32 nQuiet = 0;
+                gen_moves_quiet<SV>(flip_board(f), qc, sink, nQuiet, quietReplies);
+                if (nQuiet + sink.n != nMoves) atomicOr(P.err, DERR_GEN_MISMATCH);
+            }
+            __syncthreads();
+            if (sCount > LEAF_ITEMS && tid == 0) atomicOr(P.err, DERR_BAD_ITEM);
+            if (nRuns == 1) {
+                unsigned long long s = quietReplies * (valid ? sweight[tid] : 0ull);
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+                if (lane == 0 && s) atomicAdd(&sacc[0], s);
+                const unsigned done = __ballot_sync(0xffffffffu, nMoves != 0);
+                if (TRACK && lane == 0 && done) atomicAdd(&sdelta[0], -__popc(done));
+            } else {
+                if (quietReplies) atomicAdd(&sacc[srun[tid]], quietReplies * sweight[tid]);
+                if (TRACK && nMoves) atomicAdd(&sdelta[srun[tid]], -1);
+            }
+
+            // ---- every thread takes listed items: make, count, sum
+            const int nItems = (int)min(sCount, LEAF_ITEMS);
+            for (int j0 = 0; j0 < nItems; j0 += TILE_NT) {
+                const int j = j0 + tid;
+                const bool act = j < nItems;
+                u32 cnt = 0;
+                int pl = 0;
+                if (act) {
+                    const u32 it = sitems[j];
+                    pl = (int)((it >> 16) & 0xFFu);
+                    const Board b{sb[0][pl], sb[1][pl], sb[2][pl], sb[3][pl], sb[4][pl], sb[5][pl]};
+                    Board ch;
+                    cnt = tile_make_count<SV>(b, it, skO[PG_KNOWN_KINGS ? pl : 0], skS[PG_KNOWN_KINGS ? pl : 0], ch);
+                }
+                if (!narrow) {
+                    if (act) atomicAdd(&sacc[srun[pl]], (unsigned long long)cnt * sweight[pl]);
+                    continue;
+                }
+                if (act) cnt *= (u32)sweight[pl];
+                if (PG_ONE_RUN_SUM && nRuns == 1) {
+                    // the whole window belongs to one root: a plain warp sum
+                    // (idle lanes hold 0), no grouping by root
+                    const u32 sum = __reduce_add_sync(0xffffffffu, cnt);
+                    if (lane == 0 && sum) atomicAdd(&sacc[0], (unsigned long long)sum);
+                } else {
+                    const u32 key = act ? srun[pl] : 0xFFFFFFFFu;
+                    const unsigned peers = __match_any_sync(0xffffffffu, key);
+                    const u32 sum = __reduce_add_sync(peers, cnt);
+                    if (act && lane == __ffs(peers) - 1) atomicAdd(&sacc[key], (unsigned long long)sum);
+                }
+            }
+            __syncthreads();
+            if (tid < nRuns) {
+                atomicAdd(&P.rootCounts[srunRoot[tid]], sacc[tid]);
+                if (TRACK && sdelta[tid])
+                    atomicAdd(&P.pending[srunRoot[tid]], (unsigned long long)(long long)sdelta[tid]);
+            }
+            if (nP < TILE_MAXP) break;
+            p += TILE_MAXP;
             __syncthreads();
         }
         __syncthreads();
@@ -1792,16 +1967,25 @@ int Engine::check(cudaError_t e, const char *what)
     } while (0)
 
 constexpr size_t TILE_DYN_SMEM = sizeof(u32) * TILE_CAP;
+constexpr size_t LEAF_DYN_SMEM = sizeof(u32) * LEAF_ITEMS;
+constexpr size_t tile_dyn_smem(int mode) { return mode == MODE_LEAF ? LEAF_DYN_SMEM : TILE_DYN_SMEM; }
+
+template <int MODE, int SV, bool TRACK = false, int DD = DD_NONE>
+constexpr void (*tile_kernel())(const TileParams)
+{
+    if constexpr (MODE == MODE_LEAF) return k_leaf<SV, TRACK, DD>;
+    else return k_tile<SV, TRACK, DD>;
+}
 
 // Allows the item list's dynamic shared memory on one instantiation and
 // returns its resident-CTA grid (SMs x CTAs per SM).
-template <int MODE, int SV>
+template <int MODE, int SV, bool TRACK = false>
 int occupancy_grid(int nsm)
 {
-    cudaFuncSetAttribute(k_tile<MODE, SV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TILE_DYN_SMEM);
+    const auto fn = tile_kernel<MODE, SV, TRACK>();
+    cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_dyn_smem(MODE));
     int perSm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_tile<MODE, SV>, TILE_NT, TILE_DYN_SMEM) !=
-            cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, fn, TILE_NT, tile_dyn_smem(MODE)) != cudaSuccess ||
         perSm < 1)
         perSm = 1;
     return perSm * nsm;
@@ -1820,12 +2004,13 @@ int scan_setup()
 template <int MODE>
 void launch_tile_variant(int sv, int grid, cudaStream_t st, const TileParams &P)
 {
+    constexpr size_t smem = tile_dyn_smem(MODE);
     switch (sv) {
-    case SV_MAGIC: k_tile<MODE, SV_MAGIC><<<grid, TILE_NT, TILE_DYN_SMEM, st>>>(P); break;
-    case SV_KOGGE_FMA: k_tile<MODE, SV_KOGGE_FMA><<<grid, TILE_NT, TILE_DYN_SMEM, st>>>(P); break;
-    case SV_KOGGE_SPLIT: k_tile<MODE, SV_KOGGE_SPLIT><<<grid, TILE_NT, TILE_DYN_SMEM, st>>>(P); break;
-    case SV_HYBRID: k_tile<MODE, SV_HYBRID><<<grid, TILE_NT, TILE_DYN_SMEM, st>>>(P); break;
-    default: k_tile<MODE, SV_KOGGE><<<grid, TILE_NT, TILE_DYN_SMEM, st>>>(P); break;
+    case SV_MAGIC: tile_kernel<MODE, SV_MAGIC>()<<<grid, TILE_NT, smem, st>>>(P); break;
+    case SV_KOGGE_FMA: tile_kernel<MODE, SV_KOGGE_FMA>()<<<grid, TILE_NT, smem, st>>>(P); break;
+    case SV_KOGGE_SPLIT: tile_kernel<MODE, SV_KOGGE_SPLIT>()<<<grid, TILE_NT, smem, st>>>(P); break;
+    case SV_HYBRID: tile_kernel<MODE, SV_HYBRID>()<<<grid, TILE_NT, smem, st>>>(P); break;
+    default: tile_kernel<MODE, SV_KOGGE>()<<<grid, TILE_NT, smem, st>>>(P); break;
     }
 }
 
@@ -1835,11 +2020,13 @@ void launch_tile_variant(int sv, int grid, cudaStream_t st, const TileParams &P)
 template <int MODE>
 void launch_dd_tile(int sv, bool constParams, int grid, cudaStream_t st, const TileParams &P)
 {
+    constexpr size_t smem = tile_dyn_smem(MODE);
     const bool split = sv == SV_KOGGE_SPLIT;
-    if (constParams && split) k_tile<MODE, SV_KOGGE_SPLIT, false, DD_CONST><<<grid, TILE_NT, TILE_DYN_SMEM, st>>>(P);
-    else if (constParams) k_tile<MODE, SV_KOGGE, false, DD_CONST><<<grid, TILE_NT, TILE_DYN_SMEM, st>>>(P);
-    else if (split) k_tile<MODE, SV_KOGGE_SPLIT, false, DD_SHARED><<<grid, TILE_NT, TILE_DYN_SMEM, st>>>(P);
-    else k_tile<MODE, SV_KOGGE, false, DD_SHARED><<<grid, TILE_NT, TILE_DYN_SMEM, st>>>(P);
+    if (constParams && split)
+        tile_kernel<MODE, SV_KOGGE_SPLIT, false, DD_CONST>()<<<grid, TILE_NT, smem, st>>>(P);
+    else if (constParams) tile_kernel<MODE, SV_KOGGE, false, DD_CONST>()<<<grid, TILE_NT, smem, st>>>(P);
+    else if (split) tile_kernel<MODE, SV_KOGGE_SPLIT, false, DD_SHARED>()<<<grid, TILE_NT, smem, st>>>(P);
+    else tile_kernel<MODE, SV_KOGGE, false, DD_SHARED>()<<<grid, TILE_NT, smem, st>>>(P);
 }
 
 const char *slider_name(int sv)
@@ -1933,14 +2120,13 @@ int Engine::init(const perft_config &cfg)
     gridTile[MODE_EXPAND][SV_HYBRID] = occupancy_grid<MODE_EXPAND, SV_HYBRID>(nsm);
     gridTile[MODE_LEAF][SV_HYBRID] = occupancy_grid<MODE_LEAF, SV_HYBRID>(nsm);
 
-    for (auto fn : {(const void *)k_tile<MODE_LEAF, SV_KOGGE, false, DD_CONST>,
-                    (const void *)k_tile<MODE_LEAF, SV_KOGGE_SPLIT, false, DD_CONST>,
-                    (const void *)k_tile<MODE_EXPAND, SV_KOGGE, false, DD_CONST>,
-                    (const void *)k_tile<MODE_EXPAND, SV_KOGGE_SPLIT, false, DD_CONST>,
-                    (const void *)k_tile<MODE_LEAF, SV_KOGGE, false, DD_SHARED>,
-                    (const void *)k_tile<MODE_LEAF, SV_KOGGE_SPLIT, false, DD_SHARED>,
-                    (const void *)k_tile<MODE_EXPAND, SV_KOGGE, false, DD_SHARED>,
-                    (const void *)k_tile<MODE_EXPAND, SV_KOGGE_SPLIT, false, DD_SHARED>})
+    for (auto fn : {(const void *)k_leaf<SV_KOGGE, false, DD_CONST>, (const void *)k_leaf<SV_KOGGE_SPLIT, false, DD_CONST>,
+                    (const void *)k_leaf<SV_KOGGE, false, DD_SHARED>,
+                    (const void *)k_leaf<SV_KOGGE_SPLIT, false, DD_SHARED>})
+        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LEAF_DYN_SMEM);
+    for (auto fn : {(const void *)k_tile<SV_KOGGE, false, DD_CONST>, (const void *)k_tile<SV_KOGGE_SPLIT, false, DD_CONST>,
+                    (const void *)k_tile<SV_KOGGE, false, DD_SHARED>,
+                    (const void *)k_tile<SV_KOGGE_SPLIT, false, DD_SHARED>})
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TILE_DYN_SMEM);
     if ((rc0 = scan_setup()) != PERFT_OK) return rc0;
     ddGridScan = 4 * nsm;

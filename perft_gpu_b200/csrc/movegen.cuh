@@ -1338,6 +1338,328 @@ PG_HD Board make_child_mirrored(const Board &f, u32 mv, int *moverKing = nullptr
     return c;
 }
 
+// ------------------------------------------------- quiet moves counted as sets
+// The count-only ply needs, for every move of a position P, the number of
+// replies.  Most moves are quiet and change that number in a way that can be
+// read off the position: with n0 the opponent's moves in P if it were its
+// turn (A moves, B replies),
+//   replies(f -> t) = n0 + F[f] - F[t],
+// where F[s] is what B loses when the square s becomes occupied by A and
+// gains when A's piece leaves it: the squares beyond s on the rays of B's
+// sliders that reach s, and B's pawn pushes through s, less B's pawn captures
+// on s.  F is kept bit-sliced (six planes), so a piece's targets are summed
+// with six population counts.
+//
+// The formula holds when the move changes neither the legality of B's moves
+// nor two squares of one ray or pawn path:
+//   * captures, promotions, castling, en passant and double pushes that can
+//     be taken en passant are left out;
+//   * neither f nor t may change an attack on B's king, its free or
+//     A-occupied neighbour squares or (with castling rights) its castling
+//     squares (the set V), or a pin: squares between an A slider and V with
+//     at most one piece between, the blockers of a slider two pieces away
+//     from the king, V itself and the castling path (`bad`); squares from
+//     which the moving piece attacks V; for sliders every square on a line
+//     with the king;
+//   * a piece that moves along a line may not start on a square that a B
+//     slider attacks (f and t would be on one ray), nor go from one square
+//     to another in front of B's pawns;
+//   * B's pawns on the seventh rank: the squares before them (four moves
+//     each) are left out.
+// About 70% of the moves of 8-34-ply playouts qualify.
+struct QuietCtx {
+    u64 F[6];  // bit planes of F (plus 2 everywhere, which cancels)
+    u64 badP, badN, badB, badR, badK;
+    u64 att;   // squares that unpinned B sliders attack
+    u64 push;  // squares that B's pawn pushes use
+    u32 n0;
+};
+
+// Adds the number with bit planes b0, b1, b2 to F.
+PG_HD void planes_add3(u64 *F, u64 b0, u64 b1, u64 b2)
+{
+    u64 c = F[0] & b0;
+    F[0] ^= b0;
+    u64 x = F[1];
+    F[1] = x ^ b1 ^ c;
+    c = (x & b1) | (c & (x | b1));
+    x = F[2];
+    F[2] = x ^ b2 ^ c;
+    c = (x & b2) | (c & (x | b2));
+    x = F[3];
+    F[3] = x ^ c;
+    c &= x;
+    x = F[4];
+    F[4] = x ^ c;
+    F[5] ^= c & x;
+}
+PG_HD void planes_add1(u64 *F, u64 b)
+{
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+        const u64 c = F[k] & b;
+        F[k] ^= b;
+        b = c;
+    }
+}
+
+// One direction (one step of S squares up or down, `wrap` the squares a step
+// can end on, `from` those it can start on): fills of B's sliders (o), A's
+// sliders (e) and V share one propagator chain.
+template <int S, bool UP>
+PG_HD u64 quiet_step(u64 x)
+{
+    return UP ? x << S : x >> S;
+}
+template <int S, bool UP>
+PG_HD void quiet_dir(QuietCtx &q, u64 o, u64 e, u64 V, u64 empty, u64 notB, u64 wrap, u64 from, u64 *eOut, u64 *vOut)
+{
+    const u64 p0 = empty & wrap;
+    const u64 p1 = p0 & quiet_step<S, UP>(p0);
+    const u64 p2 = p1 & quiet_step<2 * S, UP>(p1);
+    auto fill = [&](u64 g) {
+        g |= p0 & quiet_step<S, UP>(g);
+        g |= p1 & quiet_step<2 * S, UP>(g);
+        g |= p2 & quiet_step<4 * S, UP>(g);
+        return quiet_step<S, UP>(g) & wrap;
+    };
+    const u64 ro = fill(o);
+    *eOut = fill(e);
+    *vOut = fill(V);
+    q.att |= ro;
+    // k[j]: at least j squares beyond that B could move to
+    const u64 k1 = quiet_step<S, !UP>(notB) & from;
+    const u64 k2 = quiet_step<S, !UP>(empty & k1) & from;
+    const u64 k3 = quiet_step<S, !UP>(empty & k2) & from;
+    const u64 k4 = quiet_step<S, !UP>(empty & k3) & from;
+    const u64 k5 = quiet_step<S, !UP>(empty & k4) & from;
+    const u64 k6 = quiet_step<S, !UP>(empty & k5) & from;
+    planes_add3(q.F, (k1 ^ k2 ^ k3 ^ k4 ^ k5 ^ k6) & ro, ((k2 & ~k4) | k6) & ro, k4 & ro);
+}
+
+// f: the parent P, mirrored (the frame of B to move).
+PG_HD void quiet_setup(const Board &f, QuietCtx &q)
+{
+    const u64 pawns = f.pawns & RANKS2TO7;
+    const u64 occ = pawns | f.knights | f.bq | f.rq | f.kings;
+    const u64 A = f.mine, B = occ ^ A, empty = ~occ, notB = ~B;
+    const u32 st = (u32)(f.pawns >> 58) & 3u;  // B's castling rights
+    MoveCtx c;
+    {
+        Board N = f;
+        N.mine = B;
+        N.pawns = pawns | st;
+        q.n0 = count_moves_fused<SV_KOGGE>(N, -1, -1, 0, 0, &c);
+    }
+    const u64 kB = f.kings & B;
+    const int ksq = ctz(kB);
+    u64 V = (PG_TAB(king[ksq]) & notB) | kB;
+    u64 bad = 0;
+    if (st & 1) V |= 0x60ULL;
+    if (st & 2) {
+        V |= 0x0CULL;
+        bad |= 0x0EULL;
+    }
+    const u64 aB = f.bq & A, aR = f.rq & A;
+    const u64 B1 = f.bq & B & ~c.pinned, R1 = f.rq & B & ~c.pinned;
+#pragma unroll
+    for (int k = 0; k < 6; k++) q.F[k] = 0;
+    q.att = 0;
+    const u64 nA = ~FILEA, nH = ~FILEH;
+    u64 e1, e2, v1, v2;
+    quiet_dir<8, true>(q, R1, aR, V, empty, notB, ~0ULL, ~0ULL, &e1, &v1);
+    quiet_dir<8, false>(q, R1, aR, V, empty, notB, ~0ULL, ~0ULL, &e2, &v2);
+    u64 vR = v1 | v2;
+    bad |= (e1 & v2) | (e2 & v1);
+    quiet_dir<1, true>(q, R1, aR, V, empty, notB, nA, nH, &e1, &v1);
+    quiet_dir<1, false>(q, R1, aR, V, empty, notB, nH, nA, &e2, &v2);
+    vR |= v1 | v2;
+    bad |= (e1 & v2) | (e2 & v1);
+    quiet_dir<9, true>(q, B1, aB, V, empty, notB, nA, nH, &e1, &v1);
+    quiet_dir<9, false>(q, B1, aB, V, empty, notB, nH, nA, &e2, &v2);
+    u64 vB = v1 | v2;
+    bad |= (e1 & v2) | (e2 & v1);
+    quiet_dir<7, true>(q, B1, aB, V, empty, notB, nH, nA, &e1, &v1);
+    quiet_dir<7, false>(q, B1, aB, V, empty, notB, nA, nH, &e2, &v2);
+    vB |= v1 | v2;
+    bad |= (e1 & v2) | (e2 & v1) | V;
+    // pins, and sliders one more piece away from a pin
+    const u64 kR = PG_TAB(rookRays[ksq]), kD = PG_TAB(bishopRays[ksq]);
+    for_each_bit((kR & aR) | (kD & aB), [&](int s) {
+        const u64 btw = PG_TAB(between[ksq][s]), blk = btw & occ;
+        const u64 rest = blk & (blk - 1);
+        if (!rest) bad |= btw;
+        else if (!(rest & (rest - 1))) bad |= blk;
+    });
+    // B's pawns: pushes through a square, captures on it
+    const u64 P = pawns & B & ~c.pinned;
+    const u64 n1 = sh_n(P), first = n1 & RANK3;
+    planes_add1(q.F, n1);
+    planes_add1(q.F, first & sh_s(empty));
+    planes_add1(q.F, sh_n(first & empty));
+    planes_add1(q.F, ~sh_nw(P));
+    planes_add1(q.F, ~sh_ne(P));
+    bad |= (n1 | sh_nw(P) | sh_ne(P)) & RANK8;
+    q.push = n1 | sh_n(first);
+    q.badP = bad | pawn_att_up(V);
+    q.badN = bad | knight_set_att(V);
+    q.badB = bad | vB | kD;
+    q.badR = bad | vR | kR;
+    const u64 row = V | sh_e(V) | sh_w(V);
+    q.badK = bad | row | sh_n(row) | sh_s(row);
+}
+
+// F of one square, and summed over a set.
+PG_HD u32 quiet_f(const QuietCtx &q, int s)
+{
+    u32 v = 0;
+#pragma unroll
+    for (int k = 0; k < 6; k++) v |= (u32)((q.F[k] >> s) & 1) << k;
+    return v;
+}
+PG_HD u32 quiet_sum(const QuietCtx &q, u64 set)
+{
+    u32 v = 0;
+#pragma unroll
+    for (int k = 0; k < 6; k++) v += (u32)popc(q.F[k] & set) << k;
+    return v;
+}
+
+// The same masks in the parent's own frame, where its moves are generated.
+PG_HD void quiet_flip(QuietCtx &q)
+{
+#pragma unroll
+    for (int k = 0; k < 6; k++) q.F[k] = flipv(q.F[k]);
+    q.badP = flipv(q.badP);
+    q.badN = flipv(q.badN);
+    q.badB = flipv(q.badB);
+    q.badR = flipv(q.badR);
+    q.badK = flipv(q.badK);
+    q.att = flipv(q.att);
+    q.push = flipv(q.push);
+}
+
+// gen_moves with the quiet moves counted: adds the replies of the moves that
+// the formula covers to `replies` and their number to `n`, and emits the rest
+// (calling out.room(k) before each run of k moves).
+// q is in the parent's frame.
+template <int SV, class Sink>
+PG_HD void gen_moves_quiet(const Board &b, const QuietCtx &q, Sink &out, u32 &n, u32 &replies)
+{
+    constexpr int GEN_SV = PG_GEN_MAGIC ? SV_MAGIC : SV;
+    Ctx c;
+    setup_ctx<PG_GEN_MAGIC_ATTACKS ? GEN_SV : SV>(b, c);
+    const u64 notMine = ~c.mine;
+    // moves of the piece on s to the squares t; `aligned`: it moves along lines
+    auto piece = [&](int s, u64 t, u64 bad, bool aligned) {
+        const u64 bit = 1ULL << s;
+        u64 quiet = 0;
+        if (!(bit & (bad | (aligned ? q.att : 0)))) {
+            quiet = t & c.empty & ~bad;
+            if (bit & q.push) quiet &= ~q.push;
+        }
+        if (quiet) {
+            const u32 k = (u32)popc(quiet);
+            n += k;
+            replies += k * (q.n0 + quiet_f(q, s)) - quiet_sum(q, quiet);
+        }
+        t &= ~quiet;
+        if (t) {
+            out.room(popc(t));
+            emit_targets(out, s, t);
+        }
+    };
+    // pawn moves to the squares t from S squares below
+    auto pawns = [&](u64 t, int S, u32 flags, u64 ok) {
+        const u64 badF = q.badP | q.att;
+        const u64 quiet = t & ok & ~q.badP & ~(badF << S) & ~(q.push & (q.push << S));
+        if (quiet) {
+            const u32 k = (u32)popc(quiet);
+            n += k;
+            replies += k * q.n0 + quiet_sum(q, quiet >> S) - quiet_sum(q, quiet);
+        }
+        t &= ~quiet;
+        if (t) {
+            out.room(popc(t) + 3 * popc_byte7(t));
+            for_each_bit(t, [&](int to) { emit_pawn(out, to - S, to, flags); });
+        }
+    };
+    piece(c.ksq, PG_TAB(king[c.ksq]) & notMine & ~c.attacked, q.badK, true);
+    const u64 cm = check_mask<SV>(c);
+    if (!cm) return;
+    const bool inCheck = cm != ~0ULL;
+    const u64 targets = notMine & cm;
+
+    const bool castleK = !inCheck && (c.st & 1) && !((c.occ | c.attacked) & 0x60ULL);
+    const bool castleQ = !inCheck && (c.st & 2) && !(c.occ & 0x0EULL) && !(c.attacked & 0x0CULL);
+    if (castleK || castleQ) {
+        out.room(castleK + castleQ);
+        if (castleK) out(encode_move(4, 6, MF_KING_CASTLE));
+        if (castleQ) out(encode_move(4, 2, MF_QUEEN_CASTLE));
+    }
+    const u64 pinned = pinned_of(c);
+    auto doubleOk = [&](u64 t) {  // double pushes that leave no en passant
+        return t & ~(sh_e(c.tP) | sh_w(c.tP));
+    };
+    for_each_bit(inCheck ? 0 : pinned, [&](int s) {
+        const u64 p = 1ULL << s;
+        const u64 line = PG_TAB(line[s][c.ksq]);
+        if (p & b.knights) return;
+        if (p & c.pawns) {
+            const u64 p1 = sh_n(p) & c.empty & line;
+            pawns(p1, 8, MF_QUIET, ~RANK8);
+            const u64 p2 = sh_n(p1 & RANK3) & c.empty;
+            pawns(p2, 16, MF_DOUBLE_PUSH, doubleOk(p2));
+            const u64 cap = pawn_att_up(p) & line & c.theirs;
+            if (cap) pawns(cap, ctz(cap) - s, MF_CAPTURE, 0);
+            return;
+        }
+        u64 t = 0, bad = 0;
+        if (p & b.bq) {
+            t |= bishop_att<GEN_SV>(s, c.occ);
+            bad |= q.badB;
+        }
+        if (p & b.rq) {
+            t |= rook_att<GEN_SV>(s, c.occ);
+            bad |= q.badR;
+        }
+        piece(s, t & notMine & line, bad, true);
+    });
+    for_each_bit(b.knights & c.mine & ~pinned, [&](int s) { piece(s, PG_TAB(knight[s]) & targets, q.badN, false); });
+    // (a queen attacks along both kinds of line from wherever it stands)
+    const u64 both = b.bq & b.rq;
+    for_each_bit(b.bq & c.mine & ~pinned, [&](int s) {
+        piece(s, bishop_att<GEN_SV>(s, c.occ) & targets, q.badB | (((both >> s) & 1) ? q.badR : 0), true);
+    });
+    for_each_bit(b.rq & c.mine & ~pinned, [&](int s) {
+        piece(s, rook_att<GEN_SV>(s, c.occ) & targets, q.badR | (((both >> s) & 1) ? q.badB : 0), true);
+    });
+    const u64 P = c.pawns & c.mine & ~pinned;
+    const u64 p1 = sh_n(P) & c.empty;
+    const u64 p2 = sh_n(p1 & RANK3) & c.empty & cm;
+    pawns(p1 & cm, 8, MF_QUIET, ~RANK8);
+    pawns(p2, 16, MF_DOUBLE_PUSH, doubleOk(p2));
+    const u64 capT = c.theirs & cm;
+    pawns(sh_nw(P) & capT, 7, MF_CAPTURE, 0);
+    pawns(sh_ne(P) & capT, 9, MF_CAPTURE, 0);
+    const u32 epf = c.st >> 4;
+    if (epf) {
+        const u64 target = 1ULL << (39 + epf);
+        const u64 captured = sh_s(target);
+        if (!inCheck || (captured & cm)) {
+            for (u64 srcs = pawn_att_down(target) & c.pawns & c.mine; srcs; srcs &= srcs - 1) {
+                const u64 sb = srcs & (0 - srcs);
+                const bool ok = (sb & pinned) ? (!inCheck && (PG_TAB(line[ctz(sb)][c.ksq]) & target) != 0)
+                                              : !ep_exposes_king(c, sb, captured);
+                if (ok) {
+                    out.room(1);
+                    out(encode_move(ctz(sb), 39 + epf, MF_EP));
+                }
+            }
+        }
+    }
+}
+
 // ---------------------------------------------------------- validation
 // 0 when a pos48 board is a position the generator can search: piece planes
 // disjoint (bishop and rook planes overlap only as queens), white pieces

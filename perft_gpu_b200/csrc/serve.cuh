@@ -300,26 +300,12 @@ int Server::start(const perft_serve_config &cfg, char *block, u64 bytes, int dev
     cudaDeviceProp prop;
     if (cudaGetDeviceProperties(&prop, dev) != cudaSuccess) return PERFT_ERR_CUDA;
     nsm = (unsigned)prop.multiProcessorCount;
-    cudaFuncSetAttribute(k_tile<MODE_LEAF, SV_KOGGE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)TILE_DYN_SMEM);
-    cudaFuncSetAttribute(k_tile<MODE_LEAF, SV_KOGGE_SPLIT, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)TILE_DYN_SMEM);
-    cudaFuncSetAttribute(k_tile<MODE_EXPAND, SV_KOGGE, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)TILE_DYN_SMEM);
     // the count-only ply follows the engine's tuned leaf variant when it is
     // the split-shift Kogge-Stone one; every other choice uses plain Kogge-Stone
     leafSplit = g_engine.leaf_sliders() == SV_KOGGE_SPLIT;
-    int perSm = 1;
-    if (leafSplit)
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_tile<MODE_LEAF, SV_KOGGE_SPLIT, true>, TILE_NT,
-                                                      TILE_DYN_SMEM);
-    else
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_tile<MODE_LEAF, SV_KOGGE, true>, TILE_NT,
-                                                      TILE_DYN_SMEM);
-    gridLeaf = std::max(1, perSm) * prop.multiProcessorCount;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, k_tile<MODE_EXPAND, SV_KOGGE, true>, TILE_NT,
-                                                  TILE_DYN_SMEM);
-    gridExpand = std::max(1, perSm) * prop.multiProcessorCount;
+    gridLeaf = leafSplit ? occupancy_grid<MODE_LEAF, SV_KOGGE_SPLIT, true>(prop.multiProcessorCount)
+                         : occupancy_grid<MODE_LEAF, SV_KOGGE, true>(prop.multiProcessorCount);
+    gridExpand = occupancy_grid<MODE_EXPAND, SV_KOGGE, true>(prop.multiProcessorCount);
     // table levels' last ply: the engine's per-node-sum leaf kernel
     gridLeafAcc = leafSplit ? occupancy_grid<MODE_LEAF, SV_KOGGE_SPLIT>(prop.multiProcessorCount)
                             : occupancy_grid<MODE_LEAF, SV_KOGGE>(prop.multiProcessorCount);
@@ -713,12 +699,11 @@ int Server::launch(int mode, ServeLevel &S, u64 lo, u64 hi, DeviceLevel *child)
         P.pending = nullptr;
         launch_tile_variant<MODE_EXPAND>(SV_KOGGE, (int)std::min<u64>(gridExpandTT, nTiles), st, P);
     } else if (mode == MODE_LEAF && leafSplit)
-        k_tile<MODE_LEAF, SV_KOGGE_SPLIT, true>
-            <<<(int)std::min<u64>(gridLeaf, nTiles), TILE_NT, TILE_DYN_SMEM, st>>>(P);
+        k_leaf<SV_KOGGE_SPLIT, true><<<(int)std::min<u64>(gridLeaf, nTiles), TILE_NT, LEAF_DYN_SMEM, st>>>(P);
     else if (mode == MODE_LEAF)
-        k_tile<MODE_LEAF, SV_KOGGE, true><<<(int)std::min<u64>(gridLeaf, nTiles), TILE_NT, TILE_DYN_SMEM, st>>>(P);
+        k_leaf<SV_KOGGE, true><<<(int)std::min<u64>(gridLeaf, nTiles), TILE_NT, LEAF_DYN_SMEM, st>>>(P);
     else
-        k_tile<MODE_EXPAND, SV_KOGGE, true><<<(int)std::min<u64>(gridExpand, nTiles), TILE_NT, TILE_DYN_SMEM, st>>>(P);
+        k_tile<SV_KOGGE, true><<<(int)std::min<u64>(gridExpand, nTiles), TILE_NT, TILE_DYN_SMEM, st>>>(P);
     launches++;
     return cudaGetLastError() == cudaSuccess ? PERFT_OK : PERFT_ERR_CUDA;
 }

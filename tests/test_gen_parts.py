@@ -1,5 +1,6 @@
-"""Generation in parts (movegen.cuh, gen_part), compiled for the host: the moves
-make the children that the oracle makes.  Runs without a GPU."""
+"""Generation in parts and with quiet moves counted as sets (movegen.cuh,
+gen_part and gen_moves_quiet), compiled for the host, against the oracle.
+Runs without a GPU."""
 import ctypes
 import os
 import subprocess
@@ -30,6 +31,7 @@ def gp():
     src = [SRC, os.path.join(ROOT, "perft_gpu_b200", "csrc", "tables.cpp")]
     subprocess.run(["g++", "-O2", "-std=c++20", "-fPIC", "-shared", "-o", LIB] + src, check=True)
     lib = ctypes.CDLL(LIB)
+    lib.gp_replies.restype = ctypes.c_int64
     lib.gp_init()
     return lib
 
@@ -65,3 +67,39 @@ def test_playouts(gp, oracle):
             if not len(kids):
                 break
             p = kids[int(rng.integers(len(kids)))]
+
+
+def _check_replies(gp, oracle, pos):
+    n = ctypes.c_uint32(0)
+    got = gp.gp_replies(P6(*[int(x) for x in pos]), ctypes.byref(n))
+    assert got == oracle.perft(pos, 2), (oracle.pos_to_fen(pos) if hasattr(oracle, "pos_to_fen") else pos, n.value)
+    return n.value
+
+
+def test_quiet_replies_crafted(gp, oracle):
+    """The crafted positions, two plies of each of their trees (pins, checks,
+    castling rights, en passant and promotions on both sides)."""
+    for fen in CRAFTED + list(many_moves_with_mirrors()):
+        p = oracle.fen_to_pos(fen)
+        _check_replies(gp, oracle, p)
+        for k in oracle.children(p):
+            _check_replies(gp, oracle, k)
+            for g in oracle.children(k):
+                _check_replies(gp, oracle, g)
+
+
+@pytest.mark.parametrize("plies", [(0, 12), (8, 34), (40, 160)])
+def test_quiet_replies_playouts(gp, oracle, plies):
+    rng = np.random.default_rng(plies[1])
+    start = oracle.fen_to_pos("rnbqkbnr/pppppppp/8/8/8/8/PPPPPPPP/RNBQKBNR w KQkq - 0 1")
+    quiet = moves = 0
+    for _ in range(200):
+        p = start
+        for _ in range(int(rng.integers(*plies))):
+            kids = oracle.children(p)
+            if not len(kids):
+                break
+            p = kids[int(rng.integers(len(kids)))]
+            quiet += _check_replies(gp, oracle, p)
+            moves += len(kids)
+    assert quiet > moves // 4  # the sets do carry the bulk of the moves
