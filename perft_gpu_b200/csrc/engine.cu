@@ -86,9 +86,25 @@ constexpr int TILE_MIN_LOG2 = 10;  // small levels use tiles down to 1024 items 
 constexpr u64 MAX_TILES_PER_NODE_DIV = 1ull << TILE_MIN_LOG2;
 constexpr int TILE_MAXP = TILE_NT;
 constexpr int WEIGHT_BITS = 19;
-// The count-only ply's item list: a tile's parents, whole (the last one may
-// reach past the tile's end; no position has as many moves as the slack).
-constexpr u32 LEAF_ITEMS = TILE_CAP + 512;
+// The count-only ply: CTA size and resident CTAs, and the item list, which
+// holds the listed moves of LEAF_NT parents (about a third of theirs) or all
+// moves of LEAF_FEW.  Large CTAs in step fetch each instruction for more
+// warps; the L1 that shared memory leaves holds the move tables.
+#ifndef PG_LEAF_NT
+#define PG_LEAF_NT 256
+#endif
+#ifndef PG_LEAF_MINB
+#define PG_LEAF_MINB 3
+#endif
+constexpr int LEAF_NT = PG_LEAF_NT;
+constexpr int LEAF_MINB = PG_LEAF_MINB;
+constexpr u32 LEAF_ITEMS = 24 * LEAF_NT;
+constexpr int LEAF_FEW = LEAF_NT / 64;
+static_assert(LEAF_FEW * 2 * 218 <= LEAF_ITEMS, "a few parents always fit, whatever their pieces");
+// A CTA takes LEAF_NT parents at a time, or fewer (down to this) while some
+// CTA would get none: 100 positions at depth 2 take 95 us with 16, 104 with
+// 32, 110 with 4 or always LEAF_NT.
+constexpr int LEAF_MIN_UNIT = 16;
 constexpr int TILE_MINB = PG_TILE_MINB;          // resident CTAs per SM the register budget targets
 constexpr int MAX_LEGAL_MOVES = 218;
 
@@ -1032,15 +1048,24 @@ __global__ void __launch_bounds__(TILE_NT, TILE_MINB) k_tile(const TileParams Pi
 // the replies to its quiet moves, about two thirds, are summed from the
 // position alone (movegen.cuh, QuietCtx) without making the moves, and only
 // the rest go to the shared item list, where every thread takes items, makes
-// the move and counts.  A parent belongs to the tile that holds its first
-// item, so that no parent is split.
+// the move and counts.  CTAs take LEAF_NT consecutive parents at a time.
 //
-// Bound by the integer pipes: a counted item issues about 900 thread
-// instructions, a parent's own analysis about 2500 and a set of quiet moves
-// about 60, so counting a third of the 33 items and analysing once is about
-// half of counting all of them.  Measured against making and counting every
-// item: 4096 playouts of depths 4-6 656 -> 452 ms, depth 7 5.98 -> 4.71 ms,
-// opening at depth 8 17.7 -> 11.4 ms.
+// Bound by the integer pipes (ALU 74% busy) and by instruction fetch: a
+// counted item issues about 950 thread instructions, a parent's generation
+// and analysis about 5000, so counting a quarter of the 33 items is a third of
+// counting all of them.  Measured against making and counting every item:
+// 4096 playouts of depths 4-6 656 -> 452 ms with two thirds counted as sets,
+// tiles of 8192 items and straight-line analysis; per item of that ply then
+// (depth 7 of a middlegame position / a batch / an opening at depth 8)
+//   straight-line analysis, tiles of 8192 items   23.4 / 22.4 / 19.7 ps
+//   loops over lines, pieces and pawn moves       21.8 / 21.8 / 17.8
+//   units of LEAF_NT parents (a tile of 8192 items had 240-300 parents, the
+//   part beyond 256 in a round of its own)        18.5 / 20.3 / 15.0
+//   attacks told apart by line, exact king lines  16.5 / 18.5 / 14.3
+// Slower: 128-thread CTAs, 6 per SM (26.4 / 25.7 / 22.5 against 21.8 / 21.8 /
+// 17.8) and warps that work by themselves without barriers (34.7 / 37.3 /
+// 29.0): warps at different places fetch each instruction again.  384 threads,
+// 2 per SM: the same within 1%.
 struct LeafSink {
     u32 *items;
     u32 *count;
@@ -1058,7 +1083,7 @@ struct LeafSink {
 };
 
 template <int SV, bool TRACK = false, int DD = DD_NONE>
-__global__ void __launch_bounds__(TILE_NT, TILE_MINB) k_leaf(const TileParams Pin)
+__global__ void __launch_bounds__(LEAF_NT, LEAF_MINB) k_leaf(const TileParams Pin)
 {
     __shared__ TileParams sP;  // (see k_tile)
     if (DD == DD_SHARED) {
@@ -1066,137 +1091,125 @@ __global__ void __launch_bounds__(TILE_NT, TILE_MINB) k_leaf(const TileParams Pi
         __syncthreads();
     }
     const TileParams &P = DD == DD_CONST ? c_ddTile : (DD == DD_SHARED ? sP : Pin);
-    __shared__ u64 sb[6][TILE_MAXP];
-    __shared__ uint8_t skO[PG_KNOWN_KINGS ? TILE_MAXP : 1], skS[PG_KNOWN_KINGS ? TILE_MAXP : 1];
-    __shared__ u32 sroot[TILE_MAXP];
-    __shared__ unsigned long long sweight[TILE_MAXP];  // paths that reach each parent
-    __shared__ u32 srun[TILE_MAXP];
-    __shared__ u32 srunRoot[TILE_MAXP];
-    __shared__ unsigned long long sacc[TILE_MAXP];
-    __shared__ int sdelta[TRACK ? TILE_MAXP : 1];
+    __shared__ u64 sb[6][LEAF_NT];
+    __shared__ uint8_t skO[LEAF_NT], skS[LEAF_NT];  // king squares in the children's frame (see k_tile)
+    __shared__ u32 sroot[LEAF_NT];
+    __shared__ unsigned long long sweight[LEAF_NT];  // paths that reach each parent
+    __shared__ u32 srun[LEAF_NT];
+    __shared__ u32 srunRoot[LEAF_NT];
+    __shared__ unsigned long long sacc[LEAF_NT];
+    __shared__ int sdelta[TRACK ? LEAF_NT : 1];
     extern __shared__ __align__(16) u32 sitems[];  // LEAF_ITEMS
-    __shared__ int swarp[TILE_NT / 32];
-    __shared__ u32 sTile, sCount;
+    __shared__ int swarp[LEAF_NT / 32];
+    __shared__ u32 sUnit, sCount;
 
     const int tid = threadIdx.x, lane = tid & 31;
-    const int capLog2 = P.capLog2;
-    const u64 tile0 = P.itemBase >> capLog2;
-    const u64 nTiles = (P.itemEnd - P.itemBase + (1ull << capLog2) - 1) >> capLog2;
+    // small levels: fewer parents per unit, so that every CTA gets some
+    int perUnit = LEAF_NT;
+    while (perUnit > LEAF_MIN_UNIT && P.nParents < (u64)perUnit * gridDim.x) perUnit >>= 1;
+    const u64 nUnits = (P.nParents + perUnit - 1) / perUnit;
 
     for (;;) {
-        if (tid == 0) sTile = atomicAdd(P.tileCounter, 1u);
+        if (tid == 0) sUnit = atomicAdd(P.tileCounter, 1u);
         __syncthreads();
-        const u64 tl = sTile;
-        if (tl >= nTiles) break;
-        const u64 iBeg = P.itemBase + (tl << capLog2);
-        const u64 iEnd = min(iBeg + ((u64)1 << capLog2), P.itemEnd);
-        u64 p = P.tileFirst[tile0 + tl];
-        if (P.pscan[p] < iBeg) p++;  // begins in the tile before
+        if (sUnit >= nUnits) break;
+        // ---- stage the unit's parents (serving: those whose first item is in the step)
+        const u64 q = (u64)sUnit * perUnit + tid;
+        const bool inUnit = tid < perUnit && q < P.nParents;
+        u32 nMoves = 0;
+        if (tid == 0) sCount = 0;
+        if (inUnit) {
+            const u64 beg = P.pscan[q];
+            if (beg >= P.itemBase && beg < P.itemEnd) nMoves = (u32)(P.pscan[q + 1] - beg);
+            const u64 node = P.live ? P.live[q] : q;
+            sroot[tid] = P.proot ? P.proot[node] : (u32)node;  // no root array: account to the parent itself
+            sweight[tid] = P.pweight ? P.pweight[node] : 1ull;
+            const Board pb = flip_board(level_get(P.ppl, P.pstride, node));  // mirrored (see k_tile)
+            sb[0][tid] = pb.mine;
+            sb[1][tid] = pb.pawns;
+            sb[2][tid] = pb.knights;
+            sb[3][tid] = pb.bq;
+            sb[4][tid] = pb.rq;
+            sb[5][tid] = pb.kings;
+            skO[tid] = (uint8_t)ctz(pb.kings & ~pb.mine);
+            skS[tid] = (uint8_t)ctz(pb.kings & pb.mine);
+        }
+        if (!__syncthreads_or(nMoves)) continue;
 
-        for (;;) {
-            // ---- stage the parents whose first item lies in the tile
-            const u64 q = p + tid;
-            u64 qBeg = 0;
-            bool valid = false;
-            if (q < P.nParents) {
-                qBeg = P.pscan[q];
-                valid = qBeg < iEnd;
+        // ---- the runs of equal roots (parents are ordered by root).  Usually
+        // the whole unit belongs to one root, which one block vote settles.
+        int nRuns = 0;
+        if (__syncthreads_and(!inUnit || sroot[tid] == sroot[0])) {
+            nRuns = 1;
+            srun[tid] = 0;
+            if (tid == 0) {
+                srunRoot[0] = sroot[0];
+                sacc[0] = 0ull;
+                if (TRACK) sdelta[0] = 0;
             }
-            const int nP = __syncthreads_count(valid);
-            if (nP == 0) break;
-            u32 nMoves = 0;
-            if (tid == 0) sCount = 0;
-            if (valid) {
-                nMoves = (u32)(P.pscan[q + 1] - qBeg);
-                const u64 node = P.live ? P.live[q] : q;
-                const Board pb = flip_board(level_get(P.ppl, P.pstride, node));  // mirrored (see k_tile)
-                sb[0][tid] = pb.mine;
-                sb[1][tid] = pb.pawns;
-                sb[2][tid] = pb.knights;
-                sb[3][tid] = pb.bq;
-                sb[4][tid] = pb.rq;
-                sb[5][tid] = pb.kings;
-                if (PG_KNOWN_KINGS) {
-                    skO[tid] = (uint8_t)ctz(pb.kings & ~pb.mine);
-                    skS[tid] = (uint8_t)ctz(pb.kings & pb.mine);
-                }
-                sroot[tid] = P.proot ? P.proot[node] : (u32)node;  // no root array: account to the parent itself
-                sweight[tid] = P.pweight ? P.pweight[node] : 1ull;
+        } else {
+            const bool head = inUnit && (tid == 0 || sroot[tid] != sroot[tid - 1]);
+            const int r = block_excl_count<LEAF_NT>(head, swarp, nRuns);
+            if (inUnit) srun[tid] = head ? r : r - 1;
+            if (head) {
+                srunRoot[r] = sroot[tid];
+                sacc[r] = 0ull;
+                if (TRACK) sdelta[r] = 0;
             }
-            __syncthreads();
+        }
+        // a warp's 32 products of a weight below 2^WEIGHT_BITS and a count
+        // (at most 218) sum below 2^32; units with larger weights add each
+        // product by itself
+        const bool narrow = !P.pweight || __syncthreads_and(!inUnit || (sweight[tid] >> WEIGHT_BITS) == 0);
 
-            // ---- the runs of equal roots (parents are ordered by root)
-            int nRuns = 0;
-            if (PG_ONE_RUN_VOTE && __syncthreads_and(!valid || sroot[tid] == sroot[0])) {
-                nRuns = 1;
-                if (valid) srun[tid] = 0;
-                if (tid == 0) {
-                    srunRoot[0] = sroot[0];
-                    sacc[0] = 0ull;
-                    if (TRACK) sdelta[0] = 0;
-                }
-            } else {
-                const bool head = valid && (tid == 0 || sroot[tid] != sroot[tid - 1]);
-                const int r = block_excl_count<TILE_NT>(head, swarp, nRuns);
-                if (valid) srun[tid] = head ? r : r - 1;
-                if (head) {
-                    srunRoot[r] = sroot[tid];
-                    sacc[r] = 0ull;
-                    if (TRACK) sdelta[r] = 0;
-                }
-            }
-            // a warp's 32 products of a weight below 2^WEIGHT_BITS and a count
-            // (at most 218) sum below 2^32; windows with larger weights add
-            // each product by itself
-            const bool narrow = !P.pweight || __syncthreads_and(!valid || (sweight[tid] >> WEIGHT_BITS) == 0);
-
-            // ---- generate: quiet moves are counted here, the rest is listed
-            u32 quietReplies = 0;
-            if (nMoves) {
+        u32 quietReplies = 0;
+        for (int g = 0, step = LEAF_NT; g < LEAF_NT;) {
+            // ---- generate: quiet moves are counted here, the rest is listed.
+            // Should the list overflow, fewer parents take turns.
+            u32 replies = 0;
+            if (nMoves && tid >= g && tid < g + step) {
                 const Board f{sb[0][tid], sb[1][tid], sb[2][tid], sb[3][tid], sb[4][tid], sb[5][tid]};
                 QuietCtx qc;
                 quiet_setup(f, qc);
                 quiet_flip(qc);
                 LeafSink sink{sitems, &sCount, 0u, (u32)tid << 16, 0u};
                 u32 nQuiet = 0;
-                gen_moves_quiet<SV>(flip_board(f), qc, sink, nQuiet, quietReplies);
+                gen_moves_quiet<SV>(flip_board(f), qc, sink, nQuiet, replies);
                 if (nQuiet + sink.n != nMoves) atomicOr(P.err, DERR_GEN_MISMATCH);
             }
             __syncthreads();
-            if (sCount > LEAF_ITEMS && tid == 0) atomicOr(P.err, DERR_BAD_ITEM);
-            if (nRuns == 1) {
-                unsigned long long s = quietReplies * (valid ? sweight[tid] : 0ull);
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-                if (lane == 0 && s) atomicAdd(&sacc[0], s);
-                const unsigned done = __ballot_sync(0xffffffffu, nMoves != 0);
-                if (TRACK && lane == 0 && done) atomicAdd(&sdelta[0], -__popc(done));
-            } else {
-                if (quietReplies) atomicAdd(&sacc[srun[tid]], quietReplies * sweight[tid]);
-                if (TRACK && nMoves) atomicAdd(&sdelta[srun[tid]], -1);
+            const u32 listed = sCount;
+            if (listed > LEAF_ITEMS && step > LEAF_FEW) {
+                __syncthreads();
+                if (tid == 0) sCount = 0;
+                __syncthreads();
+                step >>= 2;
+                continue;
             }
+            quietReplies += replies;
+            if (listed > LEAF_ITEMS && tid == 0) atomicOr(P.err, DERR_BAD_ITEM);
 
             // ---- every thread takes listed items: make, count, sum
-            const int nItems = (int)min(sCount, LEAF_ITEMS);
-            for (int j0 = 0; j0 < nItems; j0 += TILE_NT) {
+            const int nItems = (int)min(listed, LEAF_ITEMS);
+            for (int j0 = 0; j0 < nItems; j0 += LEAF_NT) {
                 const int j = j0 + tid;
                 const bool act = j < nItems;
                 u32 cnt = 0;
                 int pl = 0;
                 if (act) {
                     const u32 it = sitems[j];
-                    pl = (int)((it >> 16) & 0xFFu);
+                    pl = (int)(it >> 16);
                     const Board b{sb[0][pl], sb[1][pl], sb[2][pl], sb[3][pl], sb[4][pl], sb[5][pl]};
                     Board ch;
-                    cnt = tile_make_count<SV>(b, it, skO[PG_KNOWN_KINGS ? pl : 0], skS[PG_KNOWN_KINGS ? pl : 0], ch);
+                    cnt = tile_make_count<SV>(b, it, skO[pl], skS[pl], ch);
                 }
                 if (!narrow) {
                     if (act) atomicAdd(&sacc[srun[pl]], (unsigned long long)cnt * sweight[pl]);
                     continue;
                 }
                 if (act) cnt *= (u32)sweight[pl];
-                if (PG_ONE_RUN_SUM && nRuns == 1) {
-                    // the whole window belongs to one root: a plain warp sum
+                if (nRuns == 1) {
+                    // the whole unit belongs to one root: a plain warp sum
                     // (idle lanes hold 0), no grouping by root
                     const u32 sum = __reduce_add_sync(0xffffffffu, cnt);
                     if (lane == 0 && sum) atomicAdd(&sacc[0], (unsigned long long)sum);
@@ -1207,15 +1220,30 @@ __global__ void __launch_bounds__(TILE_NT, TILE_MINB) k_leaf(const TileParams Pi
                     if (act && lane == __ffs(peers) - 1) atomicAdd(&sacc[key], (unsigned long long)sum);
                 }
             }
-            __syncthreads();
-            if (tid < nRuns) {
-                atomicAdd(&P.rootCounts[srunRoot[tid]], sacc[tid]);
-                if (TRACK && sdelta[tid])
-                    atomicAdd(&P.pending[srunRoot[tid]], (unsigned long long)(long long)sdelta[tid]);
+            g += step;
+            if (g < LEAF_NT) {
+                __syncthreads();
+                if (tid == 0) sCount = 0;
+                __syncthreads();
             }
-            if (nP < TILE_MAXP) break;
-            p += TILE_MAXP;
-            __syncthreads();
+        }
+
+        if (nRuns == 1) {
+            unsigned long long s = inUnit ? quietReplies * sweight[tid] : 0ull;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+            if (lane == 0 && s) atomicAdd(&sacc[0], s);
+            const unsigned done = __ballot_sync(0xffffffffu, nMoves != 0);
+            if (TRACK && lane == 0 && done) atomicAdd(&sdelta[0], -__popc(done));
+        } else {
+            if (quietReplies) atomicAdd(&sacc[srun[tid]], quietReplies * sweight[tid]);
+            if (TRACK && nMoves) atomicAdd(&sdelta[srun[tid]], -1);
+        }
+        __syncthreads();
+        if (tid < nRuns) {
+            if (sacc[tid]) atomicAdd(&P.rootCounts[srunRoot[tid]], sacc[tid]);
+            if (TRACK && sdelta[tid])
+                atomicAdd(&P.pending[srunRoot[tid]], (unsigned long long)(long long)sdelta[tid]);
         }
         __syncthreads();
     }
@@ -1970,6 +1998,8 @@ constexpr size_t TILE_DYN_SMEM = sizeof(u32) * TILE_CAP;
 constexpr size_t LEAF_DYN_SMEM = sizeof(u32) * LEAF_ITEMS;
 constexpr size_t tile_dyn_smem(int mode) { return mode == MODE_LEAF ? LEAF_DYN_SMEM : TILE_DYN_SMEM; }
 
+constexpr int tile_threads(int mode) { return mode == MODE_LEAF ? LEAF_NT : TILE_NT; }
+
 template <int MODE, int SV, bool TRACK = false, int DD = DD_NONE>
 constexpr void (*tile_kernel())(const TileParams)
 {
@@ -1985,7 +2015,7 @@ int occupancy_grid(int nsm)
     const auto fn = tile_kernel<MODE, SV, TRACK>();
     cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_dyn_smem(MODE));
     int perSm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, fn, TILE_NT, tile_dyn_smem(MODE)) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSm, fn, tile_threads(MODE), tile_dyn_smem(MODE)) != cudaSuccess ||
         perSm < 1)
         perSm = 1;
     return perSm * nsm;
@@ -2006,11 +2036,11 @@ void launch_tile_variant(int sv, int grid, cudaStream_t st, const TileParams &P)
 {
     constexpr size_t smem = tile_dyn_smem(MODE);
     switch (sv) {
-    case SV_MAGIC: tile_kernel<MODE, SV_MAGIC>()<<<grid, TILE_NT, smem, st>>>(P); break;
-    case SV_KOGGE_FMA: tile_kernel<MODE, SV_KOGGE_FMA>()<<<grid, TILE_NT, smem, st>>>(P); break;
-    case SV_KOGGE_SPLIT: tile_kernel<MODE, SV_KOGGE_SPLIT>()<<<grid, TILE_NT, smem, st>>>(P); break;
-    case SV_HYBRID: tile_kernel<MODE, SV_HYBRID>()<<<grid, TILE_NT, smem, st>>>(P); break;
-    default: tile_kernel<MODE, SV_KOGGE>()<<<grid, TILE_NT, smem, st>>>(P); break;
+    case SV_MAGIC: tile_kernel<MODE, SV_MAGIC>()<<<grid, tile_threads(MODE), smem, st>>>(P); break;
+    case SV_KOGGE_FMA: tile_kernel<MODE, SV_KOGGE_FMA>()<<<grid, tile_threads(MODE), smem, st>>>(P); break;
+    case SV_KOGGE_SPLIT: tile_kernel<MODE, SV_KOGGE_SPLIT>()<<<grid, tile_threads(MODE), smem, st>>>(P); break;
+    case SV_HYBRID: tile_kernel<MODE, SV_HYBRID>()<<<grid, tile_threads(MODE), smem, st>>>(P); break;
+    default: tile_kernel<MODE, SV_KOGGE>()<<<grid, tile_threads(MODE), smem, st>>>(P); break;
     }
 }
 
@@ -2023,10 +2053,10 @@ void launch_dd_tile(int sv, bool constParams, int grid, cudaStream_t st, const T
     constexpr size_t smem = tile_dyn_smem(MODE);
     const bool split = sv == SV_KOGGE_SPLIT;
     if (constParams && split)
-        tile_kernel<MODE, SV_KOGGE_SPLIT, false, DD_CONST>()<<<grid, TILE_NT, smem, st>>>(P);
-    else if (constParams) tile_kernel<MODE, SV_KOGGE, false, DD_CONST>()<<<grid, TILE_NT, smem, st>>>(P);
-    else if (split) tile_kernel<MODE, SV_KOGGE_SPLIT, false, DD_SHARED>()<<<grid, TILE_NT, smem, st>>>(P);
-    else tile_kernel<MODE, SV_KOGGE, false, DD_SHARED>()<<<grid, TILE_NT, smem, st>>>(P);
+        tile_kernel<MODE, SV_KOGGE_SPLIT, false, DD_CONST>()<<<grid, tile_threads(MODE), smem, st>>>(P);
+    else if (constParams) tile_kernel<MODE, SV_KOGGE, false, DD_CONST>()<<<grid, tile_threads(MODE), smem, st>>>(P);
+    else if (split) tile_kernel<MODE, SV_KOGGE_SPLIT, false, DD_SHARED>()<<<grid, tile_threads(MODE), smem, st>>>(P);
+    else tile_kernel<MODE, SV_KOGGE, false, DD_SHARED>()<<<grid, tile_threads(MODE), smem, st>>>(P);
 }
 
 const char *slider_name(int sv)

@@ -699,9 +699,9 @@ int Server::launch(int mode, ServeLevel &S, u64 lo, u64 hi, DeviceLevel *child)
         P.pending = nullptr;
         launch_tile_variant<MODE_EXPAND>(SV_KOGGE, (int)std::min<u64>(gridExpandTT, nTiles), st, P);
     } else if (mode == MODE_LEAF && leafSplit)
-        k_leaf<SV_KOGGE_SPLIT, true><<<(int)std::min<u64>(gridLeaf, nTiles), TILE_NT, LEAF_DYN_SMEM, st>>>(P);
+        k_leaf<SV_KOGGE_SPLIT, true><<<(int)std::min<u64>(gridLeaf, nTiles), LEAF_NT, LEAF_DYN_SMEM, st>>>(P);
     else if (mode == MODE_LEAF)
-        k_leaf<SV_KOGGE, true><<<(int)std::min<u64>(gridLeaf, nTiles), TILE_NT, LEAF_DYN_SMEM, st>>>(P);
+        k_leaf<SV_KOGGE, true><<<(int)std::min<u64>(gridLeaf, nTiles), LEAF_NT, LEAF_DYN_SMEM, st>>>(P);
     else
         k_tile<SV_KOGGE, true><<<(int)std::min<u64>(gridExpand, nTiles), TILE_NT, TILE_DYN_SMEM, st>>>(P);
     launches++;
