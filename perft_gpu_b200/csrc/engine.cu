@@ -85,7 +85,6 @@ constexpr int TILE_CAP = 1 << TILE_CAP_LOG2;
 constexpr int TILE_MIN_LOG2 = 10;  // small levels use tiles down to 1024 items to fill every SM
 constexpr u64 MAX_TILES_PER_NODE_DIV = 1ull << TILE_MIN_LOG2;
 constexpr int TILE_MAXP = TILE_NT;
-constexpr int WEIGHT_BITS = 19;
 // The count-only ply: CTA size and resident CTAs, and the item list, which
 // holds the listed moves of LEAF_NT parents (about a third of theirs) or all
 // moves of LEAF_FEW.  Large CTAs in step fetch each instruction for more
@@ -1062,6 +1061,9 @@ __global__ void __launch_bounds__(TILE_NT, TILE_MINB) k_tile(const TileParams Pi
 //   units of LEAF_NT parents (a tile of 8192 items had 240-300 parents, the
 //   part beyond 256 in a round of its own)        18.5 / 20.3 / 15.0
 //   attacks told apart by line, exact king lines  16.5 / 18.5 / 14.3
+//   replies added per parent in shared memory (before: per root, grouped in
+//   each warp, weight by weight)                  15.3 / 17.3 / 13.3
+// and with a sum for every parent (table levels) 22.9 -> 19.3.
 // Slower: 128-thread CTAs, 6 per SM (26.4 / 25.7 / 22.5 against 21.8 / 21.8 /
 // 17.8) and warps that work by themselves without barriers (34.7 / 37.3 /
 // 29.0): warps at different places fetch each instruction again.  384 threads,
@@ -1095,12 +1097,10 @@ __global__ void __launch_bounds__(LEAF_NT, LEAF_MINB) k_leaf(const TileParams Pi
     __shared__ uint8_t skO[LEAF_NT], skS[LEAF_NT];  // king squares in the children's frame (see k_tile)
     __shared__ u32 sroot[LEAF_NT];
     __shared__ unsigned long long sweight[LEAF_NT];  // paths that reach each parent
-    __shared__ u32 srun[LEAF_NT];
-    __shared__ u32 srunRoot[LEAF_NT];
-    __shared__ unsigned long long sacc[LEAF_NT];
-    __shared__ int sdelta[TRACK ? LEAF_NT : 1];
+    __shared__ u32 sreplies[LEAF_NT];  // to each parent's listed moves
+    __shared__ unsigned long long ssum;
+    __shared__ int sdone;
     extern __shared__ __align__(16) u32 sitems[];  // LEAF_ITEMS
-    __shared__ int swarp[LEAF_NT / 32];
     __shared__ u32 sUnit, sCount;
 
     const int tid = threadIdx.x, lane = tid & 31;
@@ -1117,7 +1117,12 @@ __global__ void __launch_bounds__(LEAF_NT, LEAF_MINB) k_leaf(const TileParams Pi
         const u64 q = (u64)sUnit * perUnit + tid;
         const bool inUnit = tid < perUnit && q < P.nParents;
         u32 nMoves = 0;
-        if (tid == 0) sCount = 0;
+        sreplies[tid] = 0;
+        if (tid == 0) {
+            sCount = 0;
+            ssum = 0;
+            sdone = 0;
+        }
         if (inUnit) {
             const u64 beg = P.pscan[q];
             if (beg >= P.itemBase && beg < P.itemEnd) nMoves = (u32)(P.pscan[q + 1] - beg);
@@ -1136,31 +1141,8 @@ __global__ void __launch_bounds__(LEAF_NT, LEAF_MINB) k_leaf(const TileParams Pi
         }
         if (!__syncthreads_or(nMoves)) continue;
 
-        // ---- the runs of equal roots (parents are ordered by root).  Usually
-        // the whole unit belongs to one root, which one block vote settles.
-        int nRuns = 0;
-        if (__syncthreads_and(!inUnit || sroot[tid] == sroot[0])) {
-            nRuns = 1;
-            srun[tid] = 0;
-            if (tid == 0) {
-                srunRoot[0] = sroot[0];
-                sacc[0] = 0ull;
-                if (TRACK) sdelta[0] = 0;
-            }
-        } else {
-            const bool head = inUnit && (tid == 0 || sroot[tid] != sroot[tid - 1]);
-            const int r = block_excl_count<LEAF_NT>(head, swarp, nRuns);
-            if (inUnit) srun[tid] = head ? r : r - 1;
-            if (head) {
-                srunRoot[r] = sroot[tid];
-                sacc[r] = 0ull;
-                if (TRACK) sdelta[r] = 0;
-            }
-        }
-        // a warp's 32 products of a weight below 2^WEIGHT_BITS and a count
-        // (at most 218) sum below 2^32; units with larger weights add each
-        // product by itself
-        const bool narrow = !P.pweight || __syncthreads_and(!inUnit || (sweight[tid] >> WEIGHT_BITS) == 0);
+        // usually the whole unit belongs to one root (parents are ordered by root)
+        const bool oneRoot = __syncthreads_and(!inUnit || sroot[tid] == sroot[0]);
 
         u32 quietReplies = 0;
         for (int g = 0, step = LEAF_NT; g < LEAF_NT;) {
@@ -1189,36 +1171,13 @@ __global__ void __launch_bounds__(LEAF_NT, LEAF_MINB) k_leaf(const TileParams Pi
             quietReplies += replies;
             if (listed > LEAF_ITEMS && tid == 0) atomicOr(P.err, DERR_BAD_ITEM);
 
-            // ---- every thread takes listed items: make, count, sum
-            const int nItems = (int)min(listed, LEAF_ITEMS);
-            for (int j0 = 0; j0 < nItems; j0 += LEAF_NT) {
-                const int j = j0 + tid;
-                const bool act = j < nItems;
-                u32 cnt = 0;
-                int pl = 0;
-                if (act) {
-                    const u32 it = sitems[j];
-                    pl = (int)(it >> 16);
-                    const Board b{sb[0][pl], sb[1][pl], sb[2][pl], sb[3][pl], sb[4][pl], sb[5][pl]};
-                    Board ch;
-                    cnt = tile_make_count<SV>(b, it, skO[pl], skS[pl], ch);
-                }
-                if (!narrow) {
-                    if (act) atomicAdd(&sacc[srun[pl]], (unsigned long long)cnt * sweight[pl]);
-                    continue;
-                }
-                if (act) cnt *= (u32)sweight[pl];
-                if (nRuns == 1) {
-                    // the whole unit belongs to one root: a plain warp sum
-                    // (idle lanes hold 0), no grouping by root
-                    const u32 sum = __reduce_add_sync(0xffffffffu, cnt);
-                    if (lane == 0 && sum) atomicAdd(&sacc[0], (unsigned long long)sum);
-                } else {
-                    const u32 key = act ? srun[pl] : 0xFFFFFFFFu;
-                    const unsigned peers = __match_any_sync(0xffffffffu, key);
-                    const u32 sum = __reduce_add_sync(peers, cnt);
-                    if (act && lane == __ffs(peers) - 1) atomicAdd(&sacc[key], (unsigned long long)sum);
-                }
+            // ---- every thread takes listed items: make, count, add to the parent's
+            for (int j = tid; j < (int)min(listed, LEAF_ITEMS); j += LEAF_NT) {
+                const u32 it = sitems[j];
+                const int pl = (int)(it >> 16);
+                const Board b{sb[0][pl], sb[1][pl], sb[2][pl], sb[3][pl], sb[4][pl], sb[5][pl]};
+                Board ch;
+                atomicAdd(&sreplies[pl], tile_make_count<SV>(b, it, skO[pl], skS[pl], ch));
             }
             g += step;
             if (g < LEAF_NT) {
@@ -1228,22 +1187,35 @@ __global__ void __launch_bounds__(LEAF_NT, LEAF_MINB) k_leaf(const TileParams Pi
             }
         }
 
-        if (nRuns == 1) {
-            unsigned long long s = inUnit ? quietReplies * sweight[tid] : 0ull;
+        __syncthreads();
+        // ---- weight x replies into the roots' sums
+        unsigned long long s = inUnit ? (quietReplies + sreplies[tid]) * sweight[tid] : 0ull;
+        const unsigned done = __ballot_sync(0xffffffffu, nMoves != 0);
+        if (oneRoot) {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-            if (lane == 0 && s) atomicAdd(&sacc[0], s);
-            const unsigned done = __ballot_sync(0xffffffffu, nMoves != 0);
-            if (TRACK && lane == 0 && done) atomicAdd(&sdelta[0], -__popc(done));
+            if (lane == 0 && s) atomicAdd(&ssum, s);
+            if (TRACK && lane == 0 && done) atomicAdd(&sdone, __popc(done));
+            __syncthreads();
+            if (tid == 0) {
+                if (ssum) atomicAdd(&P.rootCounts[sroot[0]], ssum);
+                if (TRACK && sdone) atomicAdd(&P.pending[sroot[0]], (unsigned long long)(-(long long)sdone));
+            }
         } else {
-            if (quietReplies) atomicAdd(&sacc[srun[tid]], quietReplies * sweight[tid]);
-            if (TRACK && nMoves) atomicAdd(&sdelta[srun[tid]], -1);
-        }
-        __syncthreads();
-        if (tid < nRuns) {
-            if (sacc[tid]) atomicAdd(&P.rootCounts[srunRoot[tid]], sacc[tid]);
-            if (TRACK && sdelta[tid])
-                atomicAdd(&P.pending[srunRoot[tid]], (unsigned long long)(long long)sdelta[tid]);
+            // segmented sums over the warp's runs of equal roots
+            const u32 root = inUnit ? sroot[tid] : 0xFFFFFFFFu;
+            const unsigned run = __match_any_sync(0xffffffffu, root);
+            if (P.proot) {
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const unsigned long long y = __shfl_down_sync(0xffffffffu, s, o);
+                    if (lane + o < 32 && ((run >> (lane + o)) & 1)) s += y;
+                }
+            }
+            const bool first = !P.proot || lane == __ffs(run) - 1;
+            if (inUnit && first && s) atomicAdd(&P.rootCounts[root], s);
+            if (TRACK && inUnit && first && (run & done))
+                atomicAdd(&P.pending[root], (unsigned long long)(-(long long)__popc(run & done)));
         }
         __syncthreads();
     }
