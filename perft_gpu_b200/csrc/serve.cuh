@@ -523,7 +523,7 @@ int Server::probe_level(ServeLevel &S)
     if (cudaMemsetAsync(set, 0xFF, 8 * MERGE_SLOTS * n, st) != cudaSuccess) return PERFT_ERR_CUDA;
     const MergeLevel M{S.L.planes, S.L.stride, n,   S.L.cnt,   nullptr, nullptr, set,
                        nullptr,    nullptr,    S.r, false,     S.L.alias, S.L.acc, &dTTStats->aliases};
-    k_merge_linked<<<std::min(nb, 64u * nsm), 256, 0, st>>>(M);
+    k_merge_linked<<<nb, 256, 0, st>>>(M);
     k_tt_probe<<<std::min(nb, 8u * nsm), 256, 0, st>>>(S.L.planes, S.L.stride, n, S.r, ttKeyMask, S.L.cnt, S.L.hash,
                                                        S.L.hash2, S.L.acc, S.L.alias, tt, ttMask, dTTStats);
     launches += 2;
@@ -561,9 +561,9 @@ int Server::merge_level(ServeLevel &S)
     S.L.weight = weight;
     const MergeLevel M{S.L.planes, S.L.stride,  n,   S.L.cnt, S.L.root, weight, set,
                        segs,       nullptr,     S.r, init,    nullptr,  nullptr, nullptr};
-    const unsigned grid = std::min((unsigned)((n + 255) / 256), 64u * nsm);
-    k_merge_prepare<<<grid, 256, 0, st>>>(M);
-    k_merge_nodes<<<grid, 256, 0, st>>>(M);
+    const unsigned blocks = (unsigned)((n + 255) / 256);
+    k_merge_prepare<<<std::min(blocks, 64u * nsm), 256, 0, st>>>(M);
+    k_merge_nodes<<<blocks, 256, 0, st>>>(M);
     launches += 2;
     give_back(tmp);  // reused only by later launches on this stream
     return cudaGetLastError() == cudaSuccess ? PERFT_OK : PERFT_ERR_CUDA;
