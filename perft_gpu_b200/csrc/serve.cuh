@@ -48,6 +48,7 @@ namespace {
 
 constexpr u32 SERVE_MAX_SLOTS = 1u << 16;
 constexpr int SERVE_MAX_R = 21;
+constexpr u64 SERVE_MOVES_PER_PARENT = 32;  // in round numbers: step_items in parents of the count-only ply
 
 __global__ void k_serve_admit(const u64 *__restrict__ stagePos, const u32 *__restrict__ slots,
                               const uint8_t *__restrict__ depths, u32 n, u64 *__restrict__ posBySlot,
@@ -680,10 +681,11 @@ int Server::launch(int mode, ServeLevel &S, u64 lo, u64 hi, DeviceLevel *child)
         P.croot = child->root;
         P.cweight = child->weight;
     }
+    P.uncounted = S.r == 3;
     P.rootCounts = counts;
     P.pending = pending;
     P.err = dErr;
-    const u64 nTiles = (hi - lo + TILE_CAP - 1) / TILE_CAP;
+    const u64 nTiles = mode == MODE_LEAF ? leaf_units(S.nParents) : (hi - lo + TILE_CAP - 1) / TILE_CAP;
     if (cudaMemsetAsync(dCounter, 0, 4, st) != cudaSuccess) return PERFT_ERR_CUDA;
     if (mode == MODE_LEAF && S.tt) {
         // sums per node (the parent's own slot of acc), as the engine's table levels do
@@ -725,7 +727,9 @@ int Server::advance()
                 }
                 if (rc != PERFT_OK) return rc;
             }
-            u64 lo = S->next, hi = std::min(S->total, lo + stepItems);
+            // (the count-only ply's parents count as one item each, see k_tile)
+            const u64 step = r == 2 ? std::max<u64>(stepItems / SERVE_MOVES_PER_PARENT, TILE_CAP) : stepItems;
+            u64 lo = S->next, hi = std::min(S->total, lo + step);
             if (lo < hi) {
                 if (r == 2) {
                     int rc = launch(MODE_LEAF, *S, lo, hi, nullptr);
