@@ -108,7 +108,9 @@ constexpr int TILE_MINB = PG_TILE_MINB;          // resident CTAs per SM the reg
 constexpr int MAX_LEGAL_MOVES = 218;
 
 constexpr int SCAN_NT = 512;
-constexpr int SCAN_IPT = 16;
+// (16 nodes per thread: the same on large levels, but one position at depth 6
+// takes 0.633 ms instead of 0.620, its scans in fewer blocks)
+constexpr int SCAN_IPT = 8;
 constexpr int SCAN_CHUNK = SCAN_NT * SCAN_IPT;
 constexpr int SCAN_TOP_NT = 1024;
 
@@ -276,9 +278,11 @@ __device__ __forceinline__ ScanSums scan_top_block(ScanSums *bsum, u64 nb, u64 *
     return total;
 }
 
-// Marks the tiles whose first item belongs to parent `idx`, whose items are [run, run + c).
+// Marks the tiles whose first item belongs to parent `idx`, whose items are
+// [run, run + c).  The count-only ply has no tiles (null).
 __device__ __forceinline__ void scan_tiles(u32 *tileFirst, int capLog2, u64 run, u32 c, u64 idx)
 {
+    if (!tileFirst) return;
     const u64 t0 = (run + (1ull << capLog2) - 1) >> capLog2;
     const u64 t1 = (run + c - 1) >> capLog2;
     for (u64 t = t0; t <= t1; t++) tileFirst[t] = (u32)idx;
@@ -291,7 +295,6 @@ struct ScanShared {
     uint16_t at[SCAN_CHUNK];  // the parents' places within the chunk
     u64 sw[SCAN_NT / 32];
 };
-constexpr size_t SCAN_DYN_SMEM = sizeof(ScanShared);
 
 template <bool COMPACT>
 __device__ __forceinline__ void scan_apply_chunk(const u32 *__restrict__ cnt, u64 n, u64 b, const ScanSums *bsum,
@@ -362,8 +365,7 @@ __global__ void __launch_bounds__(SCAN_NT) k_scan_apply(const u32 *__restrict__ 
                                                         u32 *__restrict__ live, u32 *__restrict__ tileFirst,
                                                         int capLog2)
 {
-    extern __shared__ __align__(16) unsigned char scanShared[];
-    ScanShared &S = *reinterpret_cast<ScanShared *>(scanShared);
+    __shared__ ScanShared S;
     if (blockIdx.x == 0 && threadIdx.x == 0) scan[COMPACT ? totals[1] : n] = totals[0];
     scan_apply_chunk<COMPACT>(cnt, n, blockIdx.x, bsum, scan, live, tileFirst, capLog2, S);
 }
@@ -476,6 +478,7 @@ struct DevPlan {
     u32 joinN[DD_MAX_LEVELS];
     const u32 *joinIds[DD_MAX_LEVELS];
     int capMax[DD_MAX_LEVELS];  // largest tile (log2 items) for the items of level k
+    int lastLv;                    // the count-only ply's level
     int weighted;                  // levels carry path weights (some level is merged)
     int mergeLv[DD_MAX_LEVELS];    // level k's transpositions are merged
     MergeSeg *segs;                // per root: its nodes in the level being merged
@@ -632,7 +635,9 @@ __device__ void dd_plan_level(DevPlan *plan, int lv, int last, ScanSums sums)
     C.weight = plan->weighted ? (unsigned long long *)dd_take(plan, 8 * C.stride) : nullptr;
     C.live = plan->mergeLv[lv + 1] ? (u32 *)dd_take(plan, 4 * C.stride) : nullptr;
     C.pscan = (u64 *)dd_take(plan, 8 * (m + 1));
-    C.tileFirst = (u32 *)dd_take(plan, 4 * ((m * MAX_LEGAL_MOVES) / MAX_TILES_PER_NODE_DIV + 2));
+    C.tileFirst = lv + 1 < plan->lastLv
+                      ? (u32 *)dd_take(plan, 4 * ((m * MAX_LEGAL_MOVES) / MAX_TILES_PER_NODE_DIV + 2))
+                      : nullptr;
     C.bsum = (ScanSums *)dd_take(plan, sizeof(ScanSums) * ((m + SCAN_CHUNK - 1) / SCAN_CHUNK + 1));
     if (plan->overflow) {
         C.n = 0;
@@ -656,8 +661,7 @@ __device__ void dd_plan_level(DevPlan *plan, int lv, int last, ScanSums sums)
 template <bool COMPACT>
 __global__ void __launch_bounds__(SCAN_NT) k_dd_scan_apply(DevPlan *plan, int lv)
 {
-    extern __shared__ __align__(16) unsigned char scanShared[];
-    ScanShared &S = *reinterpret_cast<ScanShared *>(scanShared);
+    __shared__ ScanShared S;
     const LevelDesc &L = plan->lv[lv];
     const u64 n = L.n, nb = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
     for (u64 b = blockIdx.x; b < nb; b += gridDim.x)
@@ -2016,16 +2020,6 @@ int occupancy_grid(int nsm)
     return perSm * nsm;
 }
 
-// Allows the scan's dynamic shared memory (just above 48 KB) on this device.
-int scan_setup()
-{
-    for (auto fn : {(const void *)k_scan_apply<true>, (const void *)k_scan_apply<false>,
-                    (const void *)k_dd_scan_apply<true>, (const void *)k_dd_scan_apply<false>})
-        if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SCAN_DYN_SMEM) != cudaSuccess)
-            return PERFT_ERR_CUDA;
-    return PERFT_OK;
-}
-
 template <int MODE>
 void launch_tile_variant(int sv, int grid, cudaStream_t st, const TileParams &P)
 {
@@ -2068,7 +2062,7 @@ const char *slider_name(int sv)
 
 int Engine::init(const perft_config &cfg)
 {
-    int ndev = 0, rc0 = PERFT_OK;
+    int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev <= 0) return PERFT_ERR_NO_DEVICE;
     if (cfg.device < 0 || cfg.device >= ndev) return PERFT_ERR_INVALID_ARG;
     device = cfg.device;
@@ -2153,7 +2147,6 @@ int Engine::init(const perft_config &cfg)
                     (const void *)k_tile<SV_KOGGE, false, DD_SHARED>,
                     (const void *)k_tile<SV_KOGGE_SPLIT, false, DD_SHARED>})
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TILE_DYN_SMEM);
-    if ((rc0 = scan_setup()) != PERFT_OK) return rc0;
     ddGridScan = 4 * nsm;
     {
         ENG_TRY(cudaMalloc(&dSmall, sizeof(SmallState)));
@@ -2283,12 +2276,13 @@ int Engine::merge_level(const Joiners &J, const DeviceLevel &C, int remaining)
 int Engine::scan(const u32 *cnt, u64 n, int remaining, bool compact, ParentIndex &ix)
 {
     const u64 nb = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
+    const bool tiles = remaining > 2;
     const u64 maxTiles = (n * MAX_LEGAL_MOVES) / MAX_TILES_PER_NODE_DIV + 2;
     ix.pscan = (u64 *)alloc(8 * (n + 1));
     ix.live = compact ? (u32 *)alloc(4 * n) : nullptr;
-    ix.tileFirst = (u32 *)alloc(4 * maxTiles);
+    ix.tileFirst = tiles ? (u32 *)alloc(4 * maxTiles) : nullptr;
     ScanSums *bsum = (ScanSums *)alloc(sizeof(ScanSums) * (nb + 1));
-    if (!ix.pscan || !ix.tileFirst || !bsum || (compact && !ix.live)) return PERFT_ERR_OUT_OF_MEMORY;
+    if (!ix.pscan || (tiles && !ix.tileFirst) || !bsum || (compact && !ix.live)) return PERFT_ERR_OUT_OF_MEMORY;
     u64 *totals = (u64 *)(bsum + nb);
     k_scan_reduce<<<(unsigned)nb, SCAN_NT, 0, stream>>>(cnt, n, bsum);
     k_scan_top<<<1, SCAN_TOP_NT, 0, stream>>>(bsum, nb, totals);
@@ -2304,10 +2298,10 @@ int Engine::scan(const u32 *cnt, u64 n, int remaining, bool compact, ParentIndex
     ix.capLog2 = tc.cap;
     while (ix.capLog2 > TILE_MIN_LOG2 && (ix.total >> ix.capLog2) < 2ull * grid_for(mode, tc)) ix.capLog2--;
     if (compact)
-        k_scan_apply<true><<<(unsigned)nb, SCAN_NT, SCAN_DYN_SMEM, stream>>>(cnt, n, bsum, totals, ix.pscan, ix.live,
+        k_scan_apply<true><<<(unsigned)nb, SCAN_NT, 0, stream>>>(cnt, n, bsum, totals, ix.pscan, ix.live,
                                                                             ix.tileFirst, ix.capLog2);
     else
-        k_scan_apply<false><<<(unsigned)nb, SCAN_NT, SCAN_DYN_SMEM, stream>>>(cnt, n, bsum, totals, ix.pscan, nullptr,
+        k_scan_apply<false><<<(unsigned)nb, SCAN_NT, 0, stream>>>(cnt, n, bsum, totals, ix.pscan, nullptr,
                                                                              ix.tileFirst, ix.capLog2);
     stats.other_launches += 3;
     ENG_TRY(cudaGetLastError());
@@ -2788,6 +2782,7 @@ int Engine::build_dd(DDGraph &G)
     G.hTemplate->bump = bump;
     G.hTemplate->tileTarget = 2 * gridTile[MODE_LEAF][G.svL];
     G.hTemplate->tileCounter = dCounter;
+    G.hTemplate->lastLv = d - 2;
     G.hTemplate->weighted = merge;
     G.hTemplate->segs = dSegs;
     G.hTemplate->rootDepth = dDepths;
@@ -2859,8 +2854,8 @@ int Engine::build_dd(DDGraph &G)
             k_dd_scan_reduce<<<sg, SCAN_NT, 0, stream>>>(dPlan, lv);
             G.otherLaunches += 3;
             k_dd_scan_top<<<1, SCAN_TOP_NT, 0, stream>>>(dPlan, lv, last);
-            if (G.hTemplate->mergeLv[lv]) k_dd_scan_apply<true><<<sg, SCAN_NT, SCAN_DYN_SMEM, stream>>>(dPlan, lv);
-            else k_dd_scan_apply<false><<<sg, SCAN_NT, SCAN_DYN_SMEM, stream>>>(dPlan, lv);
+            if (G.hTemplate->mergeLv[lv]) k_dd_scan_apply<true><<<sg, SCAN_NT, 0, stream>>>(dPlan, lv);
+            else k_dd_scan_apply<false><<<sg, SCAN_NT, 0, stream>>>(dPlan, lv);
         }
         // (the scan reset the tile cursor)
         // Large plies read their launch parameters (completed by the scan)
@@ -3569,7 +3564,6 @@ int noalloc_setup(int dev)
     D.scratch = (unsigned char *)p;
     D.gridLeaf = occupancy_grid<MODE_LEAF, SV_KOGGE>(prop.multiProcessorCount);
     D.gridExpand = occupancy_grid<MODE_EXPAND, SV_KOGGE>(prop.multiProcessorCount);
-    if (scan_setup() != PERFT_OK) return PERFT_ERR_CUDA;
     D.ready = true;
     return PERFT_OK;
 }
@@ -3607,20 +3601,20 @@ struct NoallocRun {
         return cudaStreamSynchronize(st) == cudaSuccess ? PERFT_OK : PERFT_ERR_CUDA;
     }
 
-    int scan(const u32 *cnt, u64 n, u64 *&scanOut, u32 *&tileFirst, u64 &total)
+    int scan(const u32 *cnt, u64 n, bool tiles, u64 *&scanOut, u32 *&tileFirst, u64 &total)
     {
         const u64 nb = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
         const u64 maxTiles = (n * MAX_LEGAL_MOVES + TILE_CAP - 1) / TILE_CAP + 1;
         scanOut = (u64 *)take(8 * (n + 1));
-        tileFirst = (u32 *)take(4 * maxTiles);
+        tileFirst = tiles ? (u32 *)take(4 * maxTiles) : nullptr;
         const u64 mark = top;
         ScanSums *bsum = (ScanSums *)take(sizeof(ScanSums) * (nb + 1));
-        if (!scanOut || !tileFirst || !bsum) return PERFT_ERR_OUT_OF_MEMORY;
+        if (!scanOut || (tiles && !tileFirst) || !bsum) return PERFT_ERR_OUT_OF_MEMORY;
         top = mark;  // the block sums are done with before the next level is written (stream order)
         u64 *totals = (u64 *)(bsum + nb);
         k_scan_reduce<<<(unsigned)nb, SCAN_NT, 0, st>>>(cnt, n, bsum);
         k_scan_top<<<1, SCAN_TOP_NT, 0, st>>>(bsum, nb, totals);
-        k_scan_apply<false><<<(unsigned)nb, SCAN_NT, SCAN_DYN_SMEM, st>>>(cnt, n, bsum, totals, scanOut, nullptr,
+        k_scan_apply<false><<<(unsigned)nb, SCAN_NT, 0, st>>>(cnt, n, bsum, totals, scanOut, nullptr,
                                                                         tileFirst, TILE_CAP_LOG2);
         if (cudaGetLastError() != cudaSuccess) return PERFT_ERR_CUDA;
         return read_u64(scanOut + n, total);
@@ -3665,7 +3659,7 @@ struct NoallocRun {
         u64 *pscan = nullptr;
         u32 *tileFirst = nullptr;
         u64 total = 0;
-        int rc = scan(L.cnt, L.n, pscan, tileFirst, total);
+        int rc = scan(L.cnt, L.n, remaining > 2, pscan, tileFirst, total);
         if (rc != PERFT_OK || total == 0) return rc;
         if (remaining == 2) return tile(MODE_LEAF, L, pscan, tileFirst, total, nullptr, false, rootCounts);
         const u64 mark = top;

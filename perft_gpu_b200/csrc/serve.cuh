@@ -627,10 +627,10 @@ int Server::scan_level(ServeLevel &S)
     const u64 nb = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
     const u64 maxTiles = (n * MAX_LEGAL_MOVES) / MAX_TILES_PER_NODE_DIV + 2;
     S.pscan = (u64 *)take(8 * (n + 1), S.mem);
-    S.tileFirst = (u32 *)take(4 * maxTiles, S.mem);
+    S.tileFirst = S.r > 2 ? (u32 *)take(4 * maxTiles, S.mem) : nullptr;  // (the count-only ply has no tiles)
     std::vector<std::pair<u64, u64>> tmp;
     ScanSums *bsum = (ScanSums *)take(sizeof(ScanSums) * (nb + 1), tmp);
-    if (!S.pscan || !S.tileFirst || !bsum) {
+    if (!S.pscan || (S.r > 2 && !S.tileFirst) || !bsum) {
         give_back(tmp);
         return PERFT_ERR_OUT_OF_MEMORY;
     }
@@ -638,10 +638,10 @@ int Server::scan_level(ServeLevel &S)
     u64 *totals = (u64 *)(bsum + nb);
     k_scan_top<<<1, SCAN_TOP_NT, 0, st>>>(bsum, nb, totals);
     if (S.live)
-        k_scan_apply<true><<<(unsigned)nb, SCAN_NT, SCAN_DYN_SMEM, st>>>(S.L.cnt, n, bsum, totals, S.pscan, S.live,
+        k_scan_apply<true><<<(unsigned)nb, SCAN_NT, 0, st>>>(S.L.cnt, n, bsum, totals, S.pscan, S.live,
                                                                        S.tileFirst, TILE_CAP_LOG2);
     else
-        k_scan_apply<false><<<(unsigned)nb, SCAN_NT, SCAN_DYN_SMEM, st>>>(S.L.cnt, n, bsum, totals, S.pscan, nullptr,
+        k_scan_apply<false><<<(unsigned)nb, SCAN_NT, 0, st>>>(S.L.cnt, n, bsum, totals, S.pscan, nullptr,
                                                                         S.tileFirst, TILE_CAP_LOG2);
     launches += 3;
     // a table level's nodes leave the pending count in its finish pass
