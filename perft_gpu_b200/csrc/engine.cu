@@ -86,9 +86,12 @@ constexpr int TILE_MIN_LOG2 = 10;  // small levels use tiles down to 1024 items 
 constexpr u64 MAX_TILES_PER_NODE_DIV = 1ull << TILE_MIN_LOG2;
 constexpr int TILE_MAXP = TILE_NT;
 // The count-only ply: CTA size and resident CTAs, and the item list, which
-// holds the listed moves of LEAF_NT parents (about a third of theirs) or all
-// moves of LEAF_FEW.  Large CTAs in step fetch each instruction for more
-// warps; the L1 that shared memory leaves holds the move tables.
+// holds the listed moves of LEAF_NT parents or all moves of LEAF_FEW.  Large
+// CTAs in step fetch each instruction for more warps; the L1 that shared
+// memory leaves holds the move tables.  With 24 items per parent the list
+// overflowed where half the moves are listed (exposed kings) and the unit was
+// generated again in parts: depth 6 of one such position 0.61 -> 0.57 ms, two
+// table positions 220 -> 198 ms with 32; 40 takes 1% more (less L1).
 #ifndef PG_LEAF_NT
 #define PG_LEAF_NT 256
 #endif
@@ -97,7 +100,7 @@ constexpr int TILE_MAXP = TILE_NT;
 #endif
 constexpr int LEAF_NT = PG_LEAF_NT;
 constexpr int LEAF_MINB = PG_LEAF_MINB;
-constexpr u32 LEAF_ITEMS = 24 * LEAF_NT;
+constexpr u32 LEAF_ITEMS = 32 * LEAF_NT;
 constexpr int LEAF_FEW = LEAF_NT / 64;
 static_assert(LEAF_FEW * 2 * 218 <= LEAF_ITEMS, "a few parents always fit, whatever their pieces");
 // A CTA takes LEAF_NT parents at a time, or fewer (down to this) while some
@@ -1187,7 +1190,7 @@ __global__ void __launch_bounds__(LEAF_NT, LEAF_MINB) k_leaf(const TileParams Pi
                 __syncthreads();
                 if (tid == 0) sCount = 0;
                 __syncthreads();
-                step >>= 2;
+                step >>= 1;
                 continue;
             }
             quietReplies += replies;
