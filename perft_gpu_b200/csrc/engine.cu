@@ -1593,6 +1593,68 @@ __global__ void __launch_bounds__(SMALL_NT, SMALL_MINB) k_small_trees(const __gr
     }
 }
 
+// The first two plies of a single-root graph in one launch: a CTA per root
+// move writes that move's children to level 2.  As two plies of the level
+// pipeline (root, scan, tile launch, scan, tile launch) they took 75 us, most
+// of it the latency of launches with a handful of busy warps; one position at
+// depth 6 takes 571 -> 537 us with this.  The graph's plan
+// has level 2's buffers; a root or child with more moves than any game's
+// raises the overflow flag (the host-driven path then runs).
+constexpr int FRONT_LEVEL = 2;
+constexpr u64 FRONT_NODES = (u64)MAX_LEGAL_MOVES * MAX_LEGAL_MOVES;
+__global__ void __launch_bounds__(SMALL_NT, SMALL_MINB) k_dd_front(DevPlan *plan, const u64 *__restrict__ pos48, u32 *err)
+{
+    extern __shared__ __align__(16) unsigned char smallShared[];
+    SmallShared &S = *reinterpret_cast<SmallShared *>(smallShared);
+    const int tid = threadIdx.x;
+    if (tid == 0) S.flags = 0;
+    __syncthreads();
+    if (tid == 0 || tid == 32) {
+        u64 p[6];
+#pragma unroll
+        for (int k = 0; k < 6; k++) p[k] = pos48[k];
+        if (tid == 32) {
+            if (validate_pos48(p) != 0) atomicOr(&S.flags, DERR_BAD_POSITION);
+        } else {
+            const Board b = from_pos48(p);
+            MoveCtx c;
+            const u32 n = count_moves_fused<SV_KOGGE>(b, -1, -1, 0, 0, &c);
+            S.b[SMALL_ROOT] = b;
+            S.c[SMALL_ROOT] = c;
+            S.cnt[SMALL_ROOT] = (uint8_t)n;
+            if (n > (u32)MAX_LEGAL_MOVES) atomicOr(&S.flags, SMALL_OVERFLOW);
+        }
+    }
+    __syncthreads();
+    if (!S.flags) {  // (uniform: no position is stored before the barriers of small_list)
+        const int n1 = S.cnt[SMALL_ROOT];
+        if ((int)blockIdx.x >= n1) return;
+        small_list(S, SMALL_ROOT, 1);
+        small_process(S, 0, (u32)n1, 1, SMALL_FIRST0);
+        __syncthreads();
+        const u32 total = small_first(S, SMALL_FIRST0, n1);
+        LevelDesc &L = plan->lv[FRONT_LEVEL];
+        if (blockIdx.x == 0 && tid == 0) L.n = L.nChild = total;
+        if (!S.flags) {
+            const int c = (int)blockIdx.x;
+            const u32 at = S.first[c], m = S.cnt[SMALL_FIRST0 + c];
+            small_list(S, SMALL_FIRST0 + c, 1);
+            small_process(S, 0, m, 1, SMALL_CHILD0);
+            __syncthreads();
+            for (u32 i = tid; i < m; i += SMALL_NT) {
+                level_put(L.planes, L.stride, at + i, S.b[SMALL_CHILD0 + i]);
+                L.cnt[at + i] = S.cnt[SMALL_CHILD0 + i];
+                L.root[at + i] = 0;
+                if (L.weight) L.weight[at + i] = 1ull;
+            }
+        }
+    }
+    if (tid == 0 && S.flags) {
+        if (S.flags & DERR_BAD_POSITION) atomicOr(err, DERR_BAD_POSITION);
+        if (S.flags & SMALL_OVERFLOW) plan->overflow = 1;
+    }
+}
+
 // ====================================================== transposition table
 // Lockless table of 16-byte entries {verify ^ value, value} at the slot the
 // slot key picks: a torn or foreign entry fails the XOR check (the
@@ -1949,6 +2011,7 @@ private:
         cudaEvent_t evLeaf0 = nullptr, evLeaf1 = nullptr;  // recorded around the count-only ply
         std::vector<double> predLv;  // predicted nodes per level (empty: no prediction)
         u64 otherLaunches = 0;       // root, scan and join kernels per replay
+        u64 expandLaunches = 0;
         cudaGraph_t graph = nullptr;
         cudaGraphExec_t exec = nullptr;
         DevPlan *hTemplate = nullptr;  // pinned
@@ -2157,6 +2220,7 @@ int Engine::init(const perft_config &cfg)
         ENG_TRY(cudaHostAlloc(&hSmall, sizeof(SmallResult), cudaHostAllocMapped));
         ENG_TRY(cudaFuncSetAttribute(k_small_trees<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)SMALL_DYN_SMEM));
+        ENG_TRY(cudaFuncSetAttribute(k_dd_front, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMALL_DYN_SMEM));
         ENG_TRY(cudaFuncSetAttribute(k_small_trees<SMALL_BATCH>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)SMALL_DYN_SMEM));
         int perSm = 0;
@@ -2772,6 +2836,19 @@ int Engine::build_dd(DDGraph &G)
     u64 *sPlanes = (u64 *)place(48 * std::max<u64>(sStride, 32));
     u32 *sCnt = (u32 *)place(4 * std::max<u64>(sStride, 32));
     u32 *sRoot = (u32 *)place(4 * std::max<u64>(sStride, 32));
+    // a single root's first two plies are one launch (k_dd_front)
+    const bool front = n == 1 && d - 2 > FRONT_LEVEL && smallEnabled;
+    LevelDesc L2{};
+    if (front) {
+        L2.stride = (FRONT_NODES + 31) & ~31ULL;
+        L2.planes = (u64 *)place(48 * L2.stride);
+        L2.cnt = (u32 *)place(4 * L2.stride);
+        L2.root = (u32 *)place(4 * L2.stride);
+        L2.weight = merge ? (unsigned long long *)place(8 * L2.stride) : nullptr;
+        L2.pscan = (u64 *)place(8 * (FRONT_NODES + 1));
+        L2.tileFirst = (u32 *)place(4 * ((FRONT_NODES * MAX_LEGAL_MOVES) / MAX_TILES_PER_NODE_DIV + 2));
+        L2.bsum = (ScanSums *)place(sizeof(ScanSums) * ((FRONT_NODES + SCAN_CHUNK - 1) / SCAN_CHUNK + 1));
+    }
     if (bump > cap) return PERFT_ERR_OUT_OF_MEMORY;
 
     ENG_TRY(cudaMallocHost(&G.hTemplate, sizeof(DevPlan)));
@@ -2791,6 +2868,7 @@ int Engine::build_dd(DDGraph &G)
     G.hTemplate->rootDepth = dDepths;
     for (int lv = MERGE_MIN_PLIES; lv <= d - 2; lv++) G.hTemplate->mergeLv[lv] = merge;
     G.hTemplate->lv[0] = L0;
+    if (front) G.hTemplate->lv[FRONT_LEVEL] = L2;
     for (int dd = 2; dd < d; dd++) {
         G.hTemplate->joinN[d - dd] = nAt[dd];
         G.hTemplate->joinIds[d - dd] = dIds + offAt[dd];
@@ -2837,12 +2915,16 @@ int Engine::build_dd(DDGraph &G)
             k_init_roots<<<(nAt[dd] + 127) / 128, 128, 0, stream>>>(G.dPos, dIds + offAt[dd], nAt[dd], sPlanes,
                                                                    sStride, sCnt, sRoot, nullptr, dd,
                                                                    (unsigned long long *)G.dOut, dErr);
-    if (d >= 2)
+    if (front)
+        k_dd_front<<<MAX_LEGAL_MOVES, SMALL_NT, SMALL_DYN_SMEM, stream>>>(dPlan, G.dPos, dErr);
+    else if (d >= 2)
         k_init_roots<<<(unsigned)((n0 + 127) / 128), 128, 0, stream>>>(G.dPos, dIds + offAt[d], (u32)n0,
                                                                       L0.planes, L0.stride, L0.cnt, L0.root,
                                                                       L0.weight, d,
                                                                       (unsigned long long *)G.dOut, dErr);
-    for (int lv = 0; lv <= d - 2; lv++) {
+    const int lv0 = front ? FRONT_LEVEL : 0;
+    G.expandLaunches = d > 2 ? d - 2 - lv0 : 0;
+    for (int lv = lv0; lv <= d - 2; lv++) {
         const int last = lv == d - 2;
         // levels predicted small take one single-block scan launch instead of three
         if ((int)G.predLv.size() > lv && G.predLv[lv] <= 32768.0) {
@@ -2997,7 +3079,7 @@ int Engine::run_dd(const u64 *dPos, const uint8_t *depths, u32 n, u64 *dOut, boo
     ENG_TRY(cudaGraphLaunch(G->exec, stream));
     ENG_TRY(cudaStreamSynchronize(stream));
     stats.other_launches += G->otherLaunches;
-    stats.expand_launches += d > 2 ? d - 2 : 0;
+    stats.expand_launches += G->expandLaunches;
     stats.leaf_launches += d >= 2 ? 1 : 0;
     stats.graph_launches += 1;
     if ((u32)G->hFlags[0]) {  // overflow: rerun host-driven, now and on later calls

@@ -41,3 +41,16 @@ def test_positions_the_kernel_cannot_hold(engine, oracle):
         engine.perft_batch(np.stack([start, bad]), 3)
     assert ei.value.status == engine.PERFT_ERR_INVALID_ARG
     assert [int(x) for x in engine.perft_batch(np.stack([start, start]), 3)] == [8902, 8902]
+
+
+def test_first_two_plies_in_one_launch(engine, oracle):
+    """Single roots below depth 5 start from the second ply (k_dd_front): a
+    mated and a stalemated root, a root whose moves all mate or stalemate,
+    bare kings, and playouts of every phase."""
+    fens = ["rnb1kbnr/pppp1ppp/8/4p3/6Pq/5P2/PPPPP2P/RNBQKBNR w KQkq - 0 1", "7k/5Q2/6K1/8/8/8/8/8 b - - 0 1",
+            "7k/8/5QK1/8/8/8/8/8 b - - 0 1", "4k3/8/8/8/8/8/8/4K3 w - - 0 1"]
+    pos = [engine.fen_to_pos(f) for f in fens]
+    pos += list(engine.random_playouts(seed=611, n=4, min_plies=0, max_plies=6))
+    pos += list(engine.random_playouts(seed=612, n=8, min_plies=60, max_plies=200))
+    for p in pos:
+        assert engine.perft(p, 6) == oracle.perft(p, 6)
