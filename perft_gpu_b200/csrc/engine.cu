@@ -2970,11 +2970,16 @@ int Engine::build_dd(DDGraph &G)
                 G.otherLaunches += 1;
             }
             if (G.hTemplate->mergeLv[lv + 1]) {
-                // grid-stride: any grid is correct; a block per 256 predicted nodes
+                // grid-stride: any grid is correct; a block per 256 predicted nodes, up
+                // to 512 blocks per SM.  The prediction takes 0.7 of a merged level to
+                // remain; openings keep far less, and most of its blocks would find no
+                // node (an opening at depth 8 7.16 -> 6.74 ms, 512 positions at depths
+                // 4-6 38.7 -> 38.3 ms; 128, 256 and 1024 blocks per SM: 6.82, 6.80 and
+                // 6.75 ms).
                 double mg = 64.0 * nsm;
                 if ((int)G.predLv.size() > lv + 1) mg = std::max(8.0, G.predLv[lv + 1] / 256.0);
                 k_dd_merge_prepare<<<(unsigned)std::min(mg, 64.0 * nsm), 256, 0, stream>>>(dPlan, lv + 1, d - (lv + 1));
-                k_dd_merge_nodes<<<(unsigned)std::min(mg, 1e9), 256, 0, stream>>>(dPlan, lv + 1, d - (lv + 1));
+                k_dd_merge_nodes<<<(unsigned)std::min(mg, 512.0 * nsm), 256, 0, stream>>>(dPlan, lv + 1, d - (lv + 1));
                 G.otherLaunches += 2;
             }
         }
