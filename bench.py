@@ -127,17 +127,18 @@ def int32_peak(device):
             "imad_hi": out[5], "imad_wide_lop3": out[6]}
 
 
-def traffic_from_profiles(workload, items_per_launch):
-    """DRAM bytes per leaf launch: the ncu-measured bytes per item of a
-    captured launch (profiles/leaf_kernel_traffic.json) scaled to this run's
-    items per launch (traffic grows with the items processed)."""
+def captured_per_item(workload, key):
+    """A figure per item of the count-only kernel from its ncu capture
+    (profiles/leaf_kernel_traffic.json), or None."""
     path = os.path.join(ROOT, "profiles", "leaf_kernel_traffic.json")
     if not os.path.exists(path):
         return None
     with open(path) as f:
-        d = json.load(f)
-    per_item = d.get(workload, {}).get("dram_bytes_per_item")
-    return per_item * items_per_launch if per_item is not None else None
+        return json.load(f).get(workload, {}).get(key)
+
+
+def scaled(per_item, items):
+    return per_item * items if per_item is not None else None
 
 
 # ------------------------------------------------------------------ workloads
@@ -584,22 +585,30 @@ def run_ours(args):
     wf = load_work_figures()[wf_key]
     peaks = int32_peak(local)
     launches = max(1, st["leaf_launches"])
-    w_int = 2.0 * (st["leaf_items"] * (wf["c_make"] + wf["c_count"]) + st["leaf_parents"] * wf["c_gen"])
+    # The kernel sums most replies without making the move, so the operations
+    # of the reference's algorithm (make and count every move) say nothing
+    # about its use of the integer pipes: `achieved` is the instructions that
+    # it issues per item (ncu capture) over its time.
+    w_ref = 2.0 * (st["leaf_items"] * (wf["c_make"] + wf["c_count"]) + st["leaf_parents"] * wf["c_gen"])
     leaf_s = st["leaf_ms"] / 1e3
-    achieved = w_int / leaf_s if leaf_s > 0 else None
+    w_int = scaled(captured_per_item(wf_key, "thread_inst_per_item"), st["leaf_items"])
+    achieved = w_int / leaf_s if (leaf_s > 0 and w_int) else None
     peak = max(peaks.values()) if peaks else None
     roofline = {
         "bound": "int32",
-        "kernel": "k_tile<MODE_LEAF> (count-only last ply)",
+        "kernel": "k_leaf (count-only last ply)",
         "achieved": achieved / 1e12 if achieved else None,
         "peak": peak / 1e12 if peak else None,
-        "unit": "Tops/s (32-bit integer ops, reference-algorithm work)",
+        "unit": "Tops/s (32-bit thread instructions issued: ncu instructions/item x items / time)",
         "frac": (achieved / peak) if (achieved and peak) else None,
         "peak_source": "of measured: best of the integer instruction mixes timed on this GPU by libperft_probe.so",
         "peak_variants_tops": {k: v / 1e12 for k, v in peaks.items()} if peaks else None,
-        "traffic": traffic_from_profiles(wf_key, st["leaf_items"] / launches),
+        "traffic": scaled(captured_per_item(wf_key, "dram_bytes_per_item"), st["leaf_items"] / launches),
         "traffic_unit": "bytes per leaf launch (ncu bytes/item x items/launch)",
-        "work_per_launch_ops": w_int / launches,
+        "work_per_launch_ops": w_int / launches if w_int else None,
+        "items_per_launch": st["leaf_items"] / launches,
+        "leaves_per_step_searched_once": "equal positions of a level and root are merged, each counted once",
+        "reference_algorithm_tops": w_ref / leaf_s / 1e12 if leaf_s > 0 else None,
         "leaf_launch_ms_avg": st["leaf_ms"] / launches,
         "leaf_share_of_step": (st["leaf_ms"] / ms) if ms > 0 else None,
         "work_figures": {k: wf[k] for k in ("c_count", "c_make", "c_gen")},
@@ -626,6 +635,7 @@ def run_ours(args):
                 "sliders": {"leaf": pg.SLIDER_NAMES.get(st["sliders_leaf"], "?"),
                             "interior": pg.SLIDER_NAMES.get(st["sliders_expand"], "?"),
                             "chosen_by": args.sliders, "per_depth": tuning},
+                "transpositions": "equal positions of one level and root are merged within the call; no table",
                 "l2": "no flush: each step streams multi-GB level buffers through HBM (>> 126 MB L2)",
                 "parallelism": f"independent batches, {ws} GPU(s)"})
     line = {

@@ -67,7 +67,8 @@ typedef struct perft_config {
     uint64_t arena_bytes;     /* level-buffer budget in HBM; 0 = 85% of free */
     int      sliders_expand;  /* PERFT_SLIDERS_* for interior plies */
     int      sliders_leaf;    /* PERFT_SLIDERS_* for the count-only last ply */
-    int      tt_log2_entries; /* transposition table size; 0 = no table */
+    int      tt_log2_entries; /* transposition table size; 0 = no table (equal positions that
+                                 meet in one level of one call are searched once either way) */
     uint64_t zobrist_seed;    /* seed of the two sets of 781 Zobrist keys (TT only) */
 } perft_config;
 
@@ -138,7 +139,8 @@ int perft_batch_noalloc(const perft_pos48 *d_pos, const uint8_t *depths, uint32_
  * fits the budget.  Counts are identical to perft(). */
 typedef struct perft_serve_config {
     uint64_t memory_bytes;   /* budget for resident frontiers (0: 90% of the free arena) */
-    uint64_t step_items;     /* items a level may advance per iteration (0: 2^27) */
+    uint64_t step_items;     /* items a level may advance per iteration (0: 2^27); the count-only
+                                ply advances by step_items / 32 parents */
     uint32_t max_in_flight;  /* admitted queries at once (0: 4096, at most 65536) */
     int32_t  use_tt;         /* 1 (default): frontier levels two and three plies above the leaves
                                 probe, de-duplicate and store into the engine's transposition table
@@ -245,10 +247,11 @@ int perft_position_features(const perft_pos48 *pos, uint32_t *features);
 
 /* ------------------------------------------------------------- statistics */
 typedef struct perft_stats {
-    uint64_t leaf_launches;      /* count-only tile kernel launches */
+    uint64_t leaf_launches;      /* count-only launches (small batches in one launch included) */
     uint64_t expand_launches;    /* interior tile kernel launches */
     uint64_t other_launches;     /* scan / init kernels */
-    uint64_t leaf_items;         /* (parent, move) pairs counted by leaf kernels */
+    uint64_t leaf_items;         /* moves of the leaf kernels' parents, each parent once however
+                                    many paths reach it */
     uint64_t leaf_parents;       /* parents whose moves the leaf kernels generated */
     uint64_t expand_items;       /* children written by interior kernels */
     double   leaf_ms;            /* CUDA-event time of leaf kernels */
@@ -261,9 +264,10 @@ typedef struct perft_stats {
     uint64_t tt_entries;         /* transposition-table size (0: no table) */
     uint64_t tt_probes;          /* nodes looked up */
     uint64_t tt_hits;            /* lookups answered by the table */
-    uint64_t tt_duplicates;      /* same-level transpositions expanded once */
+    uint64_t tt_duplicates;      /* same-level transpositions expanded once (levels with a table, or
+                                    of related roots) */
     uint64_t tt_stores;          /* entries written */
-    uint64_t graph_launches;     /* batches run as one replayed device-driven graph */
+    uint64_t graph_launches;     /* batches run as one replayed graph */
     uint64_t small_launches;     /* single positions of depth 2..5 counted in one launch */
 } perft_stats;
 
@@ -279,7 +283,8 @@ typedef struct perft_tune_entry {
     int    leaf;         /* 1: count-only last ply; 0: interior ply */
     int    remaining;    /* remaining depth of the parent level */
     int    sliders;      /* PERFT_SLIDERS_* variant */
-    int    tile_log2;    /* largest tile (log2 items); small levels use smaller tiles */
+    int    tile_log2;    /* largest tile (log2 items); small levels use smaller tiles (the
+                            count-only ply works on parents and ignores it) */
     int    ctas_per_sm;  /* resident CTAs per SM; 0: all that fit */
     double calib_ms;     /* median calibration time of this key; 0: not timed */
 } perft_tune_entry;
