@@ -74,6 +74,21 @@ def test_deep_and_divide_match_oracle(api, oracle):
             assert paths == oracle.perft(pos, split + 1) and boards <= paths
 
 
+@pytest.mark.parametrize("which, split", [(0, 0), (0, 1), (0, 2), (1, 0), (1, 1), (3, 2)])
+def test_frontier_boards_are_distinct(api, which, split):
+    """Below and above the sizes (2,048 boards and doublings) at which the frontier's index grows."""
+    pos = positions()[which]
+    level = {pos.tobytes(): (pos, 1)}
+    for _ in range(split + 1):
+        below = {}
+        for p, paths in level.values():
+            for m in pg.legal_moves(p):
+                c = pg.apply_move(p, m)
+                below[c.tobytes()] = (c, below.get(c.tobytes(), (c, 0))[1] + paths)
+        level = below
+    assert pg.deep_frontier(pos, split + 2, split) == (len(level), sum(n for _, n in level.values()))
+
+
 def test_shards_split_the_frontier(api):
     pos = positions()[1]
     whole_total, whole = pg.deep(pos, 4, 2)
