@@ -500,6 +500,11 @@ struct DevPlan {
 // they run one at a time on the engine's stream.
 __constant__ TileParams c_ddTile;
 
+// Nodes of a level as the scans see it.  Once the plan has overflowed every
+// level is empty: buffers of levels that were planned but not written hold
+// whatever an earlier call left there.
+__device__ __forceinline__ u64 dd_nodes(const DevPlan *plan, const LevelDesc &L) { return plan->overflow ? 0 : L.n; }
+
 __device__ __forceinline__ void *dd_take(DevPlan *plan, u64 bytes)
 {
     const u64 a = (plan->bump + 255) & ~255ULL;
@@ -515,7 +520,7 @@ __global__ void __launch_bounds__(SCAN_NT) k_dd_scan_reduce(DevPlan *plan, int l
 {
     __shared__ u64 sw[SCAN_NT / 32];
     const LevelDesc &L = plan->lv[lv];
-    const u64 n = L.n, nb = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
+    const u64 n = dd_nodes(plan, L), nb = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
     for (u64 b = blockIdx.x; b < nb; b += gridDim.x) scan_reduce_chunk(L.cnt, n, b, L.bsum, sw);
 }
 
@@ -525,7 +530,7 @@ __global__ void __launch_bounds__(SCAN_TOP_NT) k_dd_scan_top(DevPlan *plan, int 
 {
     __shared__ u64 sw[SCAN_TOP_NT / 32];
     LevelDesc &L = plan->lv[lv];
-    const ScanSums total = scan_top_block(L.bsum, (L.n + SCAN_CHUNK - 1) / SCAN_CHUNK, sw);
+    const ScanSums total = scan_top_block(L.bsum, (dd_nodes(plan, L) + SCAN_CHUNK - 1) / SCAN_CHUNK, sw);
     if (threadIdx.x == 0) dd_plan_level(plan, lv, last, total);
 }
 
@@ -540,7 +545,7 @@ __global__ void __launch_bounds__(1024) k_dd_scan_small(DevPlan *plan, int lv, i
     __shared__ u64 sw[32];
     __shared__ int sCap;
     LevelDesc &L = plan->lv[lv];
-    const u64 n = L.n;
+    const u64 n = dd_nodes(plan, L);
     const u32 *cnt = L.cnt;
     u32 c[IPT];
     u64 x, tot;  // this thread's place in the pass's scan, and the pass's sums
@@ -605,10 +610,11 @@ __global__ void __launch_bounds__(1024) k_dd_scan_small(DevPlan *plan, int lv, i
 __device__ void dd_plan_level(DevPlan *plan, int lv, int last, ScanSums sums)
 {
     LevelDesc &L = plan->lv[lv];
+    const u64 n = dd_nodes(plan, L);
     const u64 total = sums.items;
-    const u64 nParents = L.live ? sums.live : L.n;
-    if (L.n) L.pscan[nParents] = total;
-    L.total = plan->overflow ? 0 : total;
+    const u64 nParents = L.live ? sums.live : n;
+    if (n) L.pscan[nParents] = total;
+    L.total = total;  // (0 when the plan has overflowed: the sums are those of no nodes)
     int cap = plan->capMax[lv] ? plan->capMax[lv] : TILE_CAP_LOG2;
     while (cap > TILE_MIN_LOG2 && (total >> cap) < plan->tileTarget) cap--;
     L.capLog2 = cap;
@@ -645,6 +651,7 @@ __device__ void dd_plan_level(DevPlan *plan, int lv, int last, ScanSums sums)
     if (plan->overflow) {
         C.n = 0;
         L.total = 0;  // nothing is expanded into a level that does not exist
+        T.nParents = 0;
     }
     // The merge set lies above the bump mark: it is done with before the next
     // level's buffers are placed there.  A set that does not fit leaves the
@@ -666,7 +673,7 @@ __global__ void __launch_bounds__(SCAN_NT) k_dd_scan_apply(DevPlan *plan, int lv
 {
     __shared__ ScanShared S;
     const LevelDesc &L = plan->lv[lv];
-    const u64 n = L.n, nb = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
+    const u64 n = dd_nodes(plan, L), nb = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
     for (u64 b = blockIdx.x; b < nb; b += gridDim.x)
         scan_apply_chunk<COMPACT>(L.cnt, n, b, L.bsum, L.pscan, L.live, L.tileFirst, L.capLog2, S);
 }
@@ -679,7 +686,7 @@ __global__ void k_dd_join(DevPlan *plan, int lv, const u64 *__restrict__ pos48, 
     const LevelDesc &C = plan->lv[lv];
     const u32 nj = plan->joinN[lv];
     const u32 i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nj || C.n == 0 || plan->overflow) return;
+    if (i >= nj || dd_nodes(plan, C) == 0) return;
     const u32 id = plan->joinIds[lv][i];
     u64 p[6];
 #pragma unroll
@@ -836,7 +843,7 @@ __global__ void __launch_bounds__(256, MERGE_CTAS) k_merge_linked(const MergeLev
 __device__ __forceinline__ MergeLevel dd_merge_level(const DevPlan *plan, int lv, int remaining)
 {
     const LevelDesc &C = plan->lv[lv];
-    return MergeLevel{C.planes, C.stride, C.set ? C.n : 0, C.cnt, C.root, C.weight, C.set,
+    return MergeLevel{C.planes, C.stride, C.set ? dd_nodes(plan, C) : 0, C.cnt, C.root, C.weight, C.set,
                       plan->segs, plan->rootDepth, remaining, false, nullptr, nullptr, nullptr};
 }
 __global__ void __launch_bounds__(256) k_dd_merge_prepare(const DevPlan *plan, int lv, int remaining)
@@ -1599,7 +1606,9 @@ __global__ void __launch_bounds__(SMALL_NT, SMALL_MINB) k_small_trees(const __gr
 // of it the latency of launches with a handful of busy warps; one position at
 // depth 6 takes 571 -> 537 us with this.  The graph's plan
 // has level 2's buffers; a root or child with more moves than any game's
-// raises the overflow flag (the host-driven path then runs).
+// raises the overflow flag (the host-driven path then runs).  Every CTA makes
+// all of the root's children, so all see the same flags before they write:
+// level 2 has nodes only when every CTA writes its share of them.
 constexpr int FRONT_LEVEL = 2;
 constexpr u64 FRONT_NODES = (u64)MAX_LEGAL_MOVES * MAX_LEGAL_MOVES;
 __global__ void __launch_bounds__(SMALL_NT, SMALL_MINB) k_dd_front(DevPlan *plan, const u64 *__restrict__ pos48, u32 *err)
@@ -1634,9 +1643,9 @@ __global__ void __launch_bounds__(SMALL_NT, SMALL_MINB) k_dd_front(DevPlan *plan
         __syncthreads();
         const u32 total = small_first(S, SMALL_FIRST0, n1);
         LevelDesc &L = plan->lv[FRONT_LEVEL];
-        if (blockIdx.x == 0 && tid == 0) L.n = L.nChild = total;
         if (!S.flags) {
             const int c = (int)blockIdx.x;
+            if (c == 0 && tid == 0) L.n = L.nChild = total;
             const u32 at = S.first[c], m = S.cnt[SMALL_FIRST0 + c];
             small_list(S, SMALL_FIRST0 + c, 1);
             small_process(S, 0, m, 1, SMALL_CHILD0);
