@@ -102,7 +102,7 @@ constexpr int LEAF_NT = PG_LEAF_NT;
 constexpr int LEAF_MINB = PG_LEAF_MINB;
 constexpr u32 LEAF_ITEMS = 32 * LEAF_NT;
 constexpr int LEAF_FEW = LEAF_NT / 64;
-static_assert(LEAF_FEW * 2 * 218 <= LEAF_ITEMS, "a few parents always fit, whatever their pieces");
+static_assert(LEAF_FEW * MAX_ANY_MOVES <= LEAF_ITEMS, "a few parents always fit, whatever their pieces");
 // A CTA takes LEAF_NT parents at a time, or fewer (down to this) while some
 // CTA would get none: 100 positions at depth 2 take 95 us with 16, 104 with
 // 32, 110 with 4 or always LEAF_NT.
@@ -116,6 +116,19 @@ constexpr int SCAN_NT = 512;
 constexpr int SCAN_IPT = 8;
 constexpr int SCAN_CHUNK = SCAN_NT * SCAN_IPT;
 constexpr int SCAN_TOP_NT = 1024;
+
+// Entries of the index that holds the first parent of each tile of a level of
+// n nodes: MAX_LEGAL_MOVES items per node in the smallest tiles.  Placements
+// that no game reaches have more moves (never more than MAX_ANY_MOVES); their
+// levels use tiles large enough for the index (tile_log2_for).
+__host__ __device__ constexpr u64 tile_index_len(u64 n) { return (n * MAX_LEGAL_MOVES) / MAX_TILES_PER_NODE_DIV + 2; }
+static_assert((u64)MAX_ANY_MOVES << TILE_MIN_LOG2 <= (u64)MAX_LEGAL_MOVES << TILE_CAP_LOG2,
+              "the largest tiles always fit the index");
+__host__ __device__ inline int tile_log2_for(u64 total, u64 n, int capLog2)
+{
+    while (capLog2 < TILE_CAP_LOG2 && (total >> capLog2) >= tile_index_len(n)) capLog2++;
+    return capLog2;
+}
 
 constexpr u32 DERR_GEN_MISMATCH = 1u;
 constexpr u32 DERR_BAD_ITEM = 2u;
@@ -617,6 +630,7 @@ __device__ void dd_plan_level(DevPlan *plan, int lv, int last, ScanSums sums)
     L.total = total;  // (0 when the plan has overflowed: the sums are those of no nodes)
     int cap = plan->capMax[lv] ? plan->capMax[lv] : TILE_CAP_LOG2;
     while (cap > TILE_MIN_LOG2 && (total >> cap) < plan->tileTarget) cap--;
+    cap = tile_log2_for(total, n, cap);
     L.capLog2 = cap;
     *plan->tileCounter = 0;  // the next launch is this level's tile launch
     TileParams &T = plan->tp[lv];  // host fields (cursor, outputs, error word) come from the template
@@ -645,7 +659,7 @@ __device__ void dd_plan_level(DevPlan *plan, int lv, int last, ScanSums sums)
     C.live = plan->mergeLv[lv + 1] ? (u32 *)dd_take(plan, 4 * C.stride) : nullptr;
     C.pscan = (u64 *)dd_take(plan, 8 * (m + 1));
     C.tileFirst = lv + 1 < plan->lastLv
-                      ? (u32 *)dd_take(plan, 4 * ((m * MAX_LEGAL_MOVES) / MAX_TILES_PER_NODE_DIV + 2))
+                      ? (u32 *)dd_take(plan, 4 * tile_index_len(m))
                       : nullptr;
     C.bsum = (ScanSums *)dd_take(plan, sizeof(ScanSums) * ((m + SCAN_CHUNK - 1) / SCAN_CHUNK + 1));
     if (plan->overflow) {
@@ -2353,10 +2367,9 @@ int Engine::scan(const u32 *cnt, u64 n, int remaining, bool compact, ParentIndex
 {
     const u64 nb = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
     const bool tiles = remaining > 2;
-    const u64 maxTiles = (n * MAX_LEGAL_MOVES) / MAX_TILES_PER_NODE_DIV + 2;
     ix.pscan = (u64 *)alloc(8 * (n + 1));
     ix.live = compact ? (u32 *)alloc(4 * n) : nullptr;
-    ix.tileFirst = tiles ? (u32 *)alloc(4 * maxTiles) : nullptr;
+    ix.tileFirst = tiles ? (u32 *)alloc(4 * tile_index_len(n)) : nullptr;
     ScanSums *bsum = (ScanSums *)alloc(sizeof(ScanSums) * (nb + 1));
     if (!ix.pscan || (tiles && !ix.tileFirst) || !bsum || (compact && !ix.live)) return PERFT_ERR_OUT_OF_MEMORY;
     u64 *totals = (u64 *)(bsum + nb);
@@ -2373,6 +2386,7 @@ int Engine::scan(const u32 *cnt, u64 n, int remaining, bool compact, ParentIndex
     const TuneCfg &tc = cfg_for(mode, remaining);
     ix.capLog2 = tc.cap;
     while (ix.capLog2 > TILE_MIN_LOG2 && (ix.total >> ix.capLog2) < 2ull * grid_for(mode, tc)) ix.capLog2--;
+    ix.capLog2 = tile_log2_for(ix.total, n, ix.capLog2);
     if (compact)
         k_scan_apply<true><<<(unsigned)nb, SCAN_NT, 0, stream>>>(cnt, n, bsum, totals, ix.pscan, ix.live,
                                                                             ix.tileFirst, ix.capLog2);
@@ -2837,7 +2851,7 @@ int Engine::build_dd(DDGraph &G)
     L0.root = (u32 *)place(4 * L0.stride);
     L0.weight = merge ? (unsigned long long *)place(8 * L0.stride) : nullptr;
     L0.pscan = (u64 *)place(8 * (n0 + 1));
-    L0.tileFirst = (u32 *)place(4 * ((n0 * MAX_LEGAL_MOVES) / MAX_TILES_PER_NODE_DIV + 2));
+    L0.tileFirst = (u32 *)place(4 * tile_index_len(n0));
     L0.bsum = (ScanSums *)place(sizeof(ScanSums) * ((n0 + SCAN_CHUNK - 1) / SCAN_CHUNK + 1));
     // scratch level for the roots of depth 0 and 1 (counts only)
     const u64 nShallow = std::max<u64>(nAt[0], nAt[1]);
@@ -2855,7 +2869,7 @@ int Engine::build_dd(DDGraph &G)
         L2.root = (u32 *)place(4 * L2.stride);
         L2.weight = merge ? (unsigned long long *)place(8 * L2.stride) : nullptr;
         L2.pscan = (u64 *)place(8 * (FRONT_NODES + 1));
-        L2.tileFirst = (u32 *)place(4 * ((FRONT_NODES * MAX_LEGAL_MOVES) / MAX_TILES_PER_NODE_DIV + 2));
+        L2.tileFirst = (u32 *)place(4 * tile_index_len(FRONT_NODES));
         L2.bsum = (ScanSums *)place(sizeof(ScanSums) * ((FRONT_NODES + SCAN_CHUNK - 1) / SCAN_CHUNK + 1));
     }
     if (bump > cap) return PERFT_ERR_OUT_OF_MEMORY;
@@ -3709,14 +3723,22 @@ struct NoallocRun {
         const u64 mark = top;
         ScanSums *bsum = (ScanSums *)take(sizeof(ScanSums) * (nb + 1));
         if (!scanOut || (tiles && !tileFirst) || !bsum) return PERFT_ERR_OUT_OF_MEMORY;
-        top = mark;  // the block sums are done with before the next level is written (stream order)
         u64 *totals = (u64 *)(bsum + nb);
         k_scan_reduce<<<(unsigned)nb, SCAN_NT, 0, st>>>(cnt, n, bsum);
         k_scan_top<<<1, SCAN_TOP_NT, 0, st>>>(bsum, nb, totals);
+        if (cudaGetLastError() != cudaSuccess) return PERFT_ERR_CUDA;
+        const int rc = read_u64(totals, total);
+        if (rc != PERFT_OK) return rc;
+        const u64 nTiles = (total + TILE_CAP - 1) / TILE_CAP;
+        if (tiles && nTiles > maxTiles) {  // more moves than any game's: an index of its own size
+            tileFirst = (u32 *)take(4 * nTiles);
+            if (!tileFirst) return PERFT_ERR_OUT_OF_MEMORY;
+        } else {
+            top = mark;  // the block sums are done with before the next level is written (stream order)
+        }
         k_scan_apply<false><<<(unsigned)nb, SCAN_NT, 0, st>>>(cnt, n, bsum, totals, scanOut, nullptr,
                                                                         tileFirst, TILE_CAP_LOG2);
-        if (cudaGetLastError() != cudaSuccess) return PERFT_ERR_CUDA;
-        return read_u64(scanOut + n, total);
+        return cudaGetLastError() == cudaSuccess ? PERFT_OK : PERFT_ERR_CUDA;
     }
 
     int tile(int mode, const DeviceLevel &par, const u64 *pscan, const u32 *tileFirst, u64 total,

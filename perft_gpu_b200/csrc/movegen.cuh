@@ -1712,6 +1712,13 @@ PG_HD void gen_moves_quiet(const Board &b, const QuietCtx &q, Sink &out, u32 &n,
     }
 }
 
+// Most legal moves of any placement that validate_pos48 accepts (a game's
+// positions have at most 218): a square is reached by at most one piece from
+// each of eight directions and by eight knights, three of the directions may
+// be pawns with four promotions each on the eighth rank, and the own king's
+// square is never a target.  Plus two castling moves.
+constexpr int MAX_ANY_MOVES = 63 * 16 + 8 * 3 * 3 + 2;
+
 // ---------------------------------------------------------- validation
 // 0 when a pos48 board is a position the generator can search: piece planes
 // disjoint (bishop and rook planes overlap only as queens), white pieces

@@ -625,9 +625,8 @@ int Server::scan_level(ServeLevel &S)
     if (S.tt && !S.live) S.live = (u32 *)take(4 * S.L.n, S.mem);  // hits and copies make no parents (without: all do)
     const u64 n = S.L.n;
     const u64 nb = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
-    const u64 maxTiles = (n * MAX_LEGAL_MOVES) / MAX_TILES_PER_NODE_DIV + 2;
     S.pscan = (u64 *)take(8 * (n + 1), S.mem);
-    S.tileFirst = S.r > 2 ? (u32 *)take(4 * maxTiles, S.mem) : nullptr;  // (the count-only ply has no tiles)
+    S.tileFirst = S.r > 2 ? (u32 *)take(4 * tile_index_len(n), S.mem) : nullptr;  // (the count-only ply has no tiles)
     std::vector<std::pair<u64, u64>> tmp;
     ScanSums *bsum = (ScanSums *)take(sizeof(ScanSums) * (nb + 1), tmp);
     if (!S.pscan || (S.r > 2 && !S.tileFirst) || !bsum) {
