@@ -1498,14 +1498,15 @@ __global__ void __launch_bounds__(SMALL_NT, SMALL_MINB) k_small_trees(const __gr
 
     if (tid == 0) S.flags = 0;
     __syncthreads();
-    // the position's count and its check at the same time
+    // the position's count and its check at the same time (no count without
+    // both kings: it would read outside the tables)
     if (tid == 0 || tid == 32) {
         u64 p[6];
 #pragma unroll
         for (int k = 0; k < 6; k++) p[k] = P.dPos ? P.dPos[6 * at + k] : P.pos[6 * at + k];
         if (tid == 32) {
             if (validate_pos48(p) != 0) atomicOr(&S.flags, DERR_BAD_POSITION);
-        } else {
+        } else if (one_king_each(p)) {
             const Board b = from_pos48(p);
             MoveCtx c;
             const u32 n = count_moves_fused<SV_KOGGE>(b, -1, -1, 0, 0, &c);
@@ -1638,7 +1639,7 @@ __global__ void __launch_bounds__(SMALL_NT, SMALL_MINB) k_dd_front(DevPlan *plan
         for (int k = 0; k < 6; k++) p[k] = pos48[k];
         if (tid == 32) {
             if (validate_pos48(p) != 0) atomicOr(&S.flags, DERR_BAD_POSITION);
-        } else {
+        } else if (one_king_each(p)) {
             const Board b = from_pos48(p);
             MoveCtx c;
             const u32 n = count_moves_fused<SV_KOGGE>(b, -1, -1, 0, 0, &c);

@@ -1720,6 +1720,10 @@ PG_HD void gen_moves_quiet(const Board &b, const QuietCtx &q, Sink &out, u32 &n,
 constexpr int MAX_ANY_MOVES = 63 * 16 + 8 * 3 * 3 + 2;
 
 // ---------------------------------------------------------- validation
+// What the generator needs of a board to stay within its tables: they are
+// indexed by both kings' squares.
+PG_HD bool one_king_each(const u64 p[6]) { return popc(p[5] & p[0]) == 1 && popc(p[5] & ~p[0]) == 1; }
+
 // 0 when a pos48 board is a position the generator can search: piece planes
 // disjoint (bishop and rook planes overlap only as queens), white pieces
 // within the occupancy, one king per side, en-passant file 0..8, and the
@@ -1732,7 +1736,7 @@ PG_HD int validate_pos48(const u64 p[6])
     const u64 occ = pawns | p[2] | sl | p[5];
     if ((pawns & p[2]) | (pawns & sl) | (pawns & p[5]) | (p[2] & sl) | (p[2] & p[5]) | (p[5] & sl)) return 1;
     if (p[0] & ~occ) return 2;
-    if (popc(p[5] & p[0]) != 1 || popc(p[5] & ~p[0]) != 1) return 3;
+    if (!one_king_each(p)) return 3;
     if (((p[1] >> 4) & 15) > 8) return 4;
     // the opponent's king must not be capturable
     const bool black = (p[1] >> 63) & 1;
