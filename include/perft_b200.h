@@ -99,8 +99,13 @@ int perft_batch(const perft_pos48 *pos, const uint8_t *depths, uint32_t n, uint6
 int perft_batch_device(const perft_pos48 *d_pos, const uint8_t *depths, uint32_t n,
                        uint64_t *d_out);
 
+/* Most legal moves of any placement that is accepted.  Positions of games
+ * have at most 218. */
+#define PERFT_MAX_MOVES 1082
+
 /* Divided perft: the legal moves of pos (UCI strings, 6 bytes each incl.
- * NUL) and the perft(depth-1) of each child.  Replaces dividedPerft's
+ * NUL) and the perft(depth-1) of each child.  moves and counts have an entry
+ * for every legal move of pos.  Replaces dividedPerft's
  * per-move subtotals (launcher.h:1392-1450, 456-464). */
 int perft_divide(const perft_pos48 *pos, uint32_t depth, char (*moves)[6], uint64_t *counts,
                  uint32_t *n_moves);
@@ -173,7 +178,8 @@ int perft_serve_get_stats(perft_serve_stats *out);
  * distinct positions split_plies below it are merged with their path counts
  * (a host transposition merge, like the reference's complete TT,
  * launcher.h:585-697) and searched on the GPU at the remaining depth.
- * moves/counts (optional, 256 entries) receive the per-move subtotals, the
+ * moves/counts (optional, an entry for every legal move of pos: 256 hold those
+ * of any game's position, PERFT_MAX_MOVES any) receive the per-move subtotals, the
  * divided perft of launcher.h:1344-1351.  Counts are 64-bit: when the total
  * does not fit (the reference switches to InfInt there), PERFT_ERR_OVERFLOW
  * is returned with every per-move subtotal filled in, to be summed wider by

@@ -22,6 +22,8 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 # PERFT_B200_LIB points the binding at another build of the same library
 LIB_PATH = os.environ.get("PERFT_B200_LIB") or os.path.join(_HERE, "libperft_b200.so")
 
+_MAX_MOVES = 1082  # most legal moves of any placement the library accepts (PERFT_MAX_MOVES)
+
 PERFT_OK = 0
 PERFT_PENDING = 1
 PERFT_ERR_INVALID_ARG = -1
@@ -262,8 +264,8 @@ def perft_batch_device(d_pos_ptr: int, depths, n: int, d_out_ptr: int) -> None:
 
 def divide(pos, depth: int) -> dict:
     p = _pos(pos)
-    moves = (ctypes.c_char * (6 * 256))()
-    counts = (ctypes.c_uint64 * 256)()
+    moves = (ctypes.c_char * (6 * _MAX_MOVES))()
+    counts = (ctypes.c_uint64 * _MAX_MOVES)()
     n = ctypes.c_uint32(0)
     _check(lib().perft_divide(ctypes.byref(p), int(depth), moves, counts, ctypes.byref(n)), "perft_divide")
     raw = bytes(moves)
@@ -310,8 +312,8 @@ def deep(pos, depth: int, split_plies: int = 2, shard: int = 0, n_shards: int = 
     merging and GPU batches.  With n_shards > 1 only this shard's frontier
     boards are searched; the shards' results sum to the full count."""
     p = _pos(pos)
-    moves = (ctypes.c_char * (6 * 256))()
-    counts = (ctypes.c_uint64 * 256)()
+    moves = (ctypes.c_char * (6 * _MAX_MOVES))()
+    counts = (ctypes.c_uint64 * _MAX_MOVES)()
     n, total = ctypes.c_uint32(0), ctypes.c_uint64(0)
     rc = lib().perft_deep_shard(ctypes.byref(p), int(depth), int(split_plies), int(shard), int(n_shards), moves,
                                 counts, ctypes.byref(n), ctypes.byref(total))
@@ -420,7 +422,7 @@ def pos_to_fen(pos) -> str:
 
 
 def legal_moves(pos) -> List[str]:
-    buf = ctypes.create_string_buffer(6 * 256)
+    buf = ctypes.create_string_buffer(6 * _MAX_MOVES)
     n = ctypes.c_uint32(0)
     p = _pos(pos)
     _check(lib().perft_legal_moves_uci(ctypes.byref(p), buf, len(buf), ctypes.byref(n)), "legal_moves")

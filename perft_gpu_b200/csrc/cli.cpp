@@ -205,8 +205,8 @@ int run_deep_shard(int argc, char **argv)
         setenv("PERFT_DEVICE", getenv("PERFT_SHARD_DEVICE"), 1);
     }
     if (ensure_init() != PERFT_OK) return 1;
-    char mv[256][6];
-    uint64_t c[256], t = 0;
+    char mv[PERFT_MAX_MOVES][6];
+    uint64_t c[PERFT_MAX_MOVES], t = 0;
     uint32_t nm = 0;
     const int rc = perft_deep_shard(&pos, depth, split, shard, n, mv, c, &nm, &t);
     if (rc != PERFT_OK && !(rc == PERFT_ERR_OVERFLOW && nm > 0)) {
@@ -224,8 +224,8 @@ int run_deep_shard(int argc, char **argv)
 int divided(const perft_pos48 &pos, uint32_t depth, std::vector<std::string> &moves,
             std::vector<uint64_t> &counts, u128 *total)
 {
-    char mv[256][6];
-    uint64_t c[256];
+    char mv[PERFT_MAX_MOVES][6];
+    uint64_t c[PERFT_MAX_MOVES];
     uint32_t n = 0;
     uint64_t t64 = 0;
     int rc;

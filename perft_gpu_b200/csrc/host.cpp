@@ -90,7 +90,7 @@ struct BoardKeyHash {
     }
 };
 
-constexpr int MAX_MOVES_BUF = 256;  // more than the 218 legal moves any position has
+static_assert(PERFT_MAX_MOVES == MAX_ANY_MOVES, "the header names the generator's bound");
 
 struct ArraySink {
     u32 *m;
@@ -111,7 +111,7 @@ void enumerate_counts(const Board &b, u32 plies, BoardCounts &out)
         out[key_of(b)] += 1;
         return;
     }
-    u32 mv[MAX_MOVES_BUF];
+    u32 mv[MAX_ANY_MOVES];
     ArraySink sink{mv, 0};
     gen_moves<SV_KOGGE>(b, sink);
     for (u32 i = 0; i < sink.n; i++) enumerate_counts(make_child(b, mv[i]), plies - 1, out);

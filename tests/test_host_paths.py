@@ -426,3 +426,20 @@ def test_deep_property_random_positions(api, oracle):
         assert sorted(acc.values()) == sorted(oracle.perft(c, depth - 1) for c in oracle.children(pos))
 
     check()
+
+
+def test_more_moves_than_any_game_has(api):
+    """A root whose only move leaves White 263 legal moves: frontiers through
+    that position, and its own divided and host-split counts."""
+    pos = np.array([0x3f21c181818181ff, 0x80c0000000000000, 0x4000000000000000, 0x3f21c181818181fe,
+                    0x3f21c181818181fe, 0x8000000000000001], dtype=np.uint64)
+    (only,) = pg.legal_moves(pos)
+    many = pg.apply_move(pos, only)
+    moves = pg.legal_moves(many)
+    assert len(moves) == 263
+    replies = {m: len(pg.legal_moves(pg.apply_move(many, m))) for m in moves}
+    assert pg.deep_frontier(pos, 4, 1) == (263, 263)
+    assert pg.deep_frontier(pos, 4, 2)[1] == sum(replies.values())
+    assert pg.deep(pos, 3, 1) == (sum(replies.values()), {only: sum(replies.values())})
+    assert pg.divide(many, 2) == replies
+    assert pg.deep(many, 2, 0) == (sum(replies.values()), replies)
