@@ -253,9 +253,9 @@ int perft_position_features(const perft_pos48 *pos, uint32_t *features);
 
 /* ------------------------------------------------------------- statistics */
 typedef struct perft_stats {
-    uint64_t leaf_launches;      /* count-only launches (small batches in one launch included) */
+    uint64_t leaf_launches;      /* launches of the count-only ply's kernel */
     uint64_t expand_launches;    /* interior tile kernel launches */
-    uint64_t other_launches;     /* scan / init kernels */
+    uint64_t other_launches;     /* scan, merge, table and root kernels; a small batch's one launch */
     uint64_t leaf_items;         /* moves of the leaf kernels' parents, each parent once however
                                     many paths reach it */
     uint64_t leaf_parents;       /* parents whose moves the leaf kernels generated */
@@ -273,7 +273,9 @@ typedef struct perft_stats {
     uint64_t tt_duplicates;      /* same-level transpositions expanded once (levels with a table, or
                                     of related roots) */
     uint64_t tt_stores;          /* entries written */
-    uint64_t graph_launches;     /* batches run as one replayed graph */
+    uint64_t graph_launches;     /* batches run as one replayed graph: the levels of a batch, or one
+                                    launch that counts up to 64 positions of depth 0..4 whole (then
+                                    no leaf or interior launches) */
     uint64_t small_launches;     /* single positions of depth 2..5 counted in one launch */
 } perft_stats;
 

@@ -54,3 +54,52 @@ def test_first_two_plies_in_one_launch(engine, oracle):
     pos += list(engine.random_playouts(seed=612, n=8, min_plies=60, max_plies=200))
     for p in pos:
         assert engine.perft(p, 6) == oracle.perft(p, 6)
+
+
+def test_small_batches_and_level_graphs_are_told_apart(engine, oracle, monkeypatch):
+    """A batch in one launch is one graph launch without a count-only or
+    interior launch; with the one-launch kernel off, batches of the same
+    depths are captured and replayed as graphs of levels."""
+    pos = engine.random_playouts(seed=71, n=32, min_plies=2, max_plies=40)
+    want = {d: oracle.perft_batch_mt(pos, d) for d in (2, 3, 4)}
+    try:
+        for small in ("1", "0"):
+            monkeypatch.setenv("PERFT_SMALL_TREE", small)
+            engine.init(device=0, arena_bytes=4 << 30)
+            engine.reset_stats()
+            for _ in range(3):  # with levels: captured, then replayed
+                for d in (2, 3, 4):
+                    assert np.array_equal(engine.perft_batch(pos, d), want[d])
+            st = engine.stats()
+            assert st["graph_launches"] == 9 and st["small_launches"] == 0
+            if small == "1":
+                assert st["leaf_launches"] == st["expand_launches"] == st["leaf_items"] == 0
+                assert st["other_launches"] == 9
+            else:
+                assert st["leaf_launches"] == 9 and st["expand_launches"] == 9
+                assert st["leaf_items"] > 0 and st["leaf_parents"] > 0 and st["leaf_ms"] > 0
+    finally:
+        monkeypatch.delenv("PERFT_SMALL_TREE")
+        engine.init(device=0, arena_bytes=8 << 30)
+
+
+def test_more_moves_than_the_kernel_holds(engine, oracle):
+    """Positions with 249 moves as a root and as the children of a root with
+    four moves: counted by the level pipeline, alone and in a batch."""
+    few = np.array([0xfe8181818181013f, 0x800000000000c000, 0, 0xfe8181818181017e, 0xfe8181818181013e, 0x81],
+                   dtype=np.uint64)
+    many = oracle.children(few)[0]
+    assert oracle.count(few) == 4 and oracle.count(many) == 249
+    above = engine.random_playouts(seed=5, n=1, min_plies=8, max_plies=8)[0]
+    for p, depths in ((many, (2, 3, 4)), (few, (3, 4, 5))):
+        for d in depths:
+            want = oracle.perft(p, d)
+            engine.reset_stats()
+            assert engine.perft(p, d) == want
+            assert engine.stats()["small_launches"] == 0
+            if d <= 4:
+                engine.reset_stats()
+                assert [int(x) for x in engine.perft_batch(np.stack([above, p, p]), d)] == \
+                    [oracle.perft(above, d), want, want]
+                assert engine.stats()["leaf_launches"] > 0
+    assert engine.perft(above, 4) == oracle.perft(above, 4)
