@@ -1141,6 +1141,7 @@ __global__ void __launch_bounds__(LEAF_NT, LEAF_MINB) k_leaf(const TileParams Pi
     __shared__ u32 sroot[LEAF_NT];
     __shared__ unsigned long long sweight[LEAF_NT];  // paths that reach each parent
     __shared__ u32 sreplies[LEAF_NT];  // to each parent's listed moves
+    __shared__ uint16_t scounted[LEAF_NT];  // each parent's moves as the level counted them
     __shared__ unsigned long long ssum;
     __shared__ u32 smoves;
     __shared__ int sdone;
@@ -1170,8 +1171,9 @@ __global__ void __launch_bounds__(LEAF_NT, LEAF_MINB) k_leaf(const TileParams Pi
             sdone = 0;
         }
         if (inUnit) {
-            const u64 beg = P.pscan[q];
-            active = beg >= P.itemBase && beg < P.itemEnd && P.pscan[q + 1] != beg;
+            const u64 beg = P.pscan[q], end = P.pscan[q + 1];
+            active = beg >= P.itemBase && beg < P.itemEnd && end != beg;
+            scounted[tid] = (uint16_t)(end - beg);
             const u64 node = P.live ? P.live[q] : q;
             sroot[tid] = P.proot ? P.proot[node] : (u32)node;  // no root array: account to the parent itself
             sweight[tid] = P.pweight ? P.pweight[node] : 1ull;
@@ -1215,6 +1217,8 @@ __global__ void __launch_bounds__(LEAF_NT, LEAF_MINB) k_leaf(const TileParams Pi
                 continue;
             }
             quietReplies += replies;
+            if (active && tid >= g && tid < g + step && !moves_as_counted(scounted[tid], nMoves))
+                atomicOr(P.err, DERR_GEN_MISMATCH);
             nMoves = __reduce_add_sync(0xffffffffu, nMoves);
             if (lane == 0) atomicAdd(&smoves, nMoves);
             if (listed > LEAF_ITEMS && tid == 0) atomicOr(P.err, DERR_BAD_ITEM);

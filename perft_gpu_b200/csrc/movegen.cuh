@@ -1719,6 +1719,11 @@ PG_HD void gen_moves_quiet(const Board &b, const QuietCtx &q, Sink &out, u32 &n,
 // square is never a target.  Plus two castling moves.
 constexpr int MAX_ANY_MOVES = 63 * 16 + 8 * 3 * 3 + 2;
 
+// Whether the moves that the count-only ply generated for a parent are those
+// that its level counted.  Only the level's roots are counted there: the other
+// parents stand in it with one item each.
+PG_HD bool moves_as_counted(u32 counted, u32 generated) { return counted == 1 || counted == generated; }
+
 // ---------------------------------------------------------- validation
 // What the generator needs of a board to stay within its tables: they are
 // indexed by both kings' squares.
