@@ -48,6 +48,10 @@ namespace {
 
 constexpr u32 SERVE_MAX_SLOTS = 1u << 16;
 constexpr int SERVE_MAX_R = 21;
+// Memory of the server's block that no level of items takes: new queries' roots
+// and the copies of their positions (under 180 bytes for each of 65536), and
+// room for the free ranges being split.
+constexpr u64 SERVE_MARGIN = 16ull << 20;
 constexpr u64 SERVE_MOVES_PER_PARENT = 32;  // in round numbers: step_items in parents of the count-only ply
 
 __global__ void k_serve_admit(const u64 *__restrict__ stagePos, const u32 *__restrict__ slots,
@@ -130,7 +134,6 @@ struct ServeLevel {
     int r = 0;
     int depth = 0;  // of its queries (a level's queries all have one depth)
     bool scanned = false;
-    bool merged = false;  // merged, or found not worth it
     bool tt = false;  // a table level: per-node sums, finished by k_serve_tt_finish
     // a remaining-depth-2 level expanded from a table level of remaining depth
     // 3: its root array holds parent indices into that level, its counts go
@@ -140,7 +143,12 @@ struct ServeLevel {
     std::vector<std::pair<u64, u64>> ttMem;  // its hashes, sums and aliases
     u64 *pscan = nullptr;
     u32 *live = nullptr;  // merged and table levels: the nodes with items
+    u32 *liveMem = nullptr;  // where they are listed, should the level be merged
     u32 *tileFirst = nullptr;
+    // until the level is scanned: the scan's block sums, and a table level's merge set
+    ScanSums *bsum = nullptr;
+    unsigned long long *set = nullptr;
+    std::vector<std::pair<u64, u64>> scanMem;
     u64 nParents = 0, total = 0, next = 0;
     std::vector<std::pair<u64, u64>> mem;  // (offset, bytes) in the server block
 };
@@ -172,6 +180,11 @@ private:
     int admit();
     int advance();
     int complete();
+    template <class Take>
+    bool level_memory(ServeLevel &S, u64 n, bool weighted, Take take);
+    bool take_level(ServeLevel &S, u64 n, bool weighted);
+    u64 reserve_below(int r);
+    bool table_level(int r) const { return tt && (r == 2 || r == 3); }
     int scan_level(ServeLevel &S);
     int launch(int mode, ServeLevel &S, u64 lo, u64 hi, DeviceLevel *child);
     int probe_level(ServeLevel &S);
@@ -257,6 +270,64 @@ void Server::give_back(std::vector<std::pair<u64, u64>> &owner)
         freeRanges[off] = size;
     }
     owner.clear();
+}
+
+// Everything that a level with n nodes needs until its items are taken from
+// it, each piece through take(bytes, owner): its nodes, the scan's arrays, and
+// a table level's hashes, sums and merge set.  Taken together when the level
+// is made, so that a level that exists can always be scanned.
+template <class Take>
+bool Server::level_memory(ServeLevel &S, u64 n, bool weighted, Take take)
+{
+    const u64 nb = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
+    const bool table = table_level(S.r), merges = mergeEnabled && !tt && S.r + MERGE_MIN_PLIES <= S.depth;
+    S.L.n = n;
+    S.L.stride = (n + 31) & ~31ULL;
+    bool ok = (S.L.planes = (u64 *)take(48 * S.L.stride, S.mem)) && (S.L.cnt = (u32 *)take(4 * S.L.stride, S.mem)) &&
+              (S.L.root = (u32 *)take(4 * S.L.stride, S.mem)) && (S.pscan = (u64 *)take(8 * (n + 1), S.mem)) &&
+              (S.bsum = (ScanSums *)take(sizeof(ScanSums) * (nb + 1), S.scanMem));
+    if (ok && weighted) ok = (S.L.weight = (unsigned long long *)take(8 * S.L.stride, S.mem));
+    if (ok && (table || merges)) ok = (S.liveMem = (u32 *)take(4 * n, S.mem));
+    if (ok && S.r > 2) ok = (S.tileFirst = (u32 *)take(4 * tile_index_len(n), S.mem));  // (the count-only ply has no tiles)
+    if (ok && table)
+        ok = (S.L.hash = (u64 *)take(8 * S.L.stride, S.ttMem)) && (S.L.hash2 = (u64 *)take(8 * S.L.stride, S.ttMem)) &&
+             (S.L.acc = (unsigned long long *)take(8 * S.L.stride, S.ttMem)) &&
+             (S.L.alias = (u32 *)take(4 * S.L.stride, S.ttMem)) &&
+             (S.set = (unsigned long long *)take(8 * MERGE_SLOTS * n, S.scanMem));
+    return ok;
+}
+
+bool Server::take_level(ServeLevel &S, u64 n, bool weighted)
+{
+    if (level_memory(S, n, weighted, [this](u64 b, std::vector<std::pair<u64, u64>> &o) { return take(b, o); }))
+        return true;
+    give_back(S.mem);
+    give_back(S.ttMem);
+    give_back(S.scanMem);
+    return false;
+}
+
+// What must stay free when a level r plies above the leaves has been made: a
+// smallest step of items for each ply below it.  Every level of items leaves
+// this much, so the level nearest the leaves always finds memory for its next
+// step, whatever else is admitted: a small budget makes work wait, and never
+// stops it.  Without this rule 13 of 145 combinations of a budget of 1 MB to
+// 2 GB and queries of depths 3-7 ended in advance()'s out-of-memory error, and
+// 60 with a table; with it none, at the same times where memory is ample.
+u64 Server::reserve_below(int r)
+{
+    u64 bytes = SERVE_MARGIN;
+    for (int k = 2; k < r; k++) {
+        ServeLevel S;
+        S.r = k;
+        S.depth = SERVE_MAX_R;
+        auto add = [&bytes](u64 b, std::vector<std::pair<u64, u64>> &) {
+            bytes += (b + 255) & ~255ULL;
+            return (void *)&bytes;  // (only counted)
+        };
+        level_memory(S, TILE_CAP, mergeEnabled && !tt, add);
+    }
+    return bytes;
 }
 
 int Server::start(const perft_serve_config &cfg, char *block, u64 bytes, int device)
@@ -365,7 +436,10 @@ int Server::submit(const u64 pos[6], u32 depth, u64 *ticket)
     q->depth = depth;
     q->tSubmit = now_s();
     // predicted peak frontier: root branching ^ (depth - 2) nodes of the last
-    // materialised ply, 65 bytes each, with a safety margin
+    // materialised ply, 65 bytes each, with a safety margin that also covers a
+    // merged level's weights, list and set (28 bytes a node, of 0.6 times the
+    // nodes).  It decides how many queries run at once; a query that takes
+    // more makes others wait (reserve_below).
     const Board b = from_pos48(pos);
     double bf = std::min(45.0, std::max(20.0, (double)count_moves<SV_KOGGE>(b)));
     double nodes = 1.0;
@@ -477,13 +551,7 @@ int Server::admit()
         ServeLevel *S = new ServeLevel();
         S->r = S->depth = (int)depth;
         const u64 cnt = i1 - i0;
-        S->L.n = cnt;
-        S->L.stride = (cnt + 31) & ~31ULL;
-        S->L.planes = (u64 *)take(48 * S->L.stride, S->mem);
-        S->L.cnt = (u32 *)take(4 * S->L.stride, S->mem);
-        S->L.root = (u32 *)take(4 * S->L.stride, S->mem);
-        if (!S->L.planes || !S->L.cnt || !S->L.root) {
-            give_back(S->mem);
+        if (!take_level(*S, cnt, false)) {
             delete S;
             give_back(tmp);
             return PERFT_ERR_OUT_OF_MEMORY;
@@ -495,6 +563,7 @@ int Server::admit()
         if (depth >= 2) pools[depth].push_back(S);
         else {
             give_back(S->mem);
+            give_back(S->scanMem);
             delete S;
         }
         i0 = i1;
@@ -509,26 +578,15 @@ int Server::admit()
 int Server::probe_level(ServeLevel &S)
 {
     const u64 n = S.L.n;
-    S.L.hash = (u64 *)take(8 * S.L.stride, S.ttMem);
-    S.L.hash2 = (u64 *)take(8 * S.L.stride, S.ttMem);
-    S.L.acc = (unsigned long long *)take(8 * S.L.stride, S.ttMem);
-    S.L.alias = (u32 *)take(4 * S.L.stride, S.ttMem);
-    std::vector<std::pair<u64, u64>> tmp;
-    unsigned long long *set = (unsigned long long *)take(8 * MERGE_SLOTS * n, tmp);
-    if (!S.L.hash || !S.L.hash2 || !S.L.acc || !S.L.alias || !set) {
-        give_back(tmp);
-        give_back(S.ttMem);  // the next iteration retries from scratch
-        return PERFT_ERR_OUT_OF_MEMORY;
-    }
     const unsigned nb = (unsigned)((n + 255) / 256);
-    if (cudaMemsetAsync(set, 0xFF, 8 * MERGE_SLOTS * n, st) != cudaSuccess) return PERFT_ERR_CUDA;
-    const MergeLevel M{S.L.planes, S.L.stride, n,   S.L.cnt,   nullptr, nullptr, set,
+    if (cudaMemsetAsync(S.set, 0xFF, 8 * MERGE_SLOTS * n, st) != cudaSuccess) return PERFT_ERR_CUDA;
+    const MergeLevel M{S.L.planes, S.L.stride, n,   S.L.cnt,   nullptr, nullptr, S.set,
                        nullptr,    nullptr,    S.r, false,     S.L.alias, S.L.acc, &dTTStats->aliases};
     k_merge_linked<<<nb, 256, 0, st>>>(M);
     k_tt_probe<<<std::min(nb, 8u * nsm), 256, 0, st>>>(S.L.planes, S.L.stride, n, S.r, ttKeyMask, S.L.cnt, S.L.hash,
                                                        S.L.hash2, S.L.acc, S.L.alias, tt, ttMask, dTTStats);
     launches += 2;
-    give_back(tmp);  // reused only by later launches on this stream
+    S.live = S.liveMem;  // hits and copies make no parents
     S.tt = true;
     return cudaGetLastError() == cudaSuccess ? PERFT_OK : PERFT_ERR_CUDA;
 }
@@ -537,7 +595,8 @@ int Server::probe_level(ServeLevel &S)
 // levels do: nodes at least MERGE_MIN_PLIES below their query's position.
 // Small levels stay as they are (two launches would cost more than their
 // copies), and so do levels while less than a quarter of the server's memory
-// is free: weights and set must not displace admitted work.  A server with a
+// is free, or where weights and set would take what the plies below need:
+// merging must not displace admitted work.  A server with a
 // table merges its table levels instead (probe_level).
 // 200 queries of depths 3-6 submitted at once: 66.1 -> 28.5 ms.
 constexpr u64 SERVE_MERGE_MIN = 4096;
@@ -546,20 +605,19 @@ int Server::merge_level(ServeLevel &S)
     const u64 n = S.L.n;
     if (!mergeEnabled || tt || S.r + MERGE_MIN_PLIES > S.depth || n < SERVE_MERGE_MIN ||
         blockBytes - inUse < blockBytes / 4)
-        return PERFT_OK;
+        return PERFT_OK;  // (no liveMem where the level is not deep enough)
     std::vector<std::pair<u64, u64>> tmp, own;
     const bool init = S.L.weight == nullptr;
     unsigned long long *weight = init ? (unsigned long long *)take(8 * S.L.stride, own) : S.L.weight;
     unsigned long long *set = (unsigned long long *)take(8 * MERGE_SLOTS * n, tmp);
-    S.live = (u32 *)take(4 * n, own);
-    if (!weight || !set || !S.live) {
-        S.live = nullptr;
+    if (!weight || !set || blockBytes - inUse < reserve_below(S.r)) {
         give_back(tmp);
         give_back(own);
         return PERFT_OK;
     }
     S.mem.insert(S.mem.end(), own.begin(), own.end());
     S.L.weight = weight;
+    S.live = S.liveMem;
     const MergeLevel M{S.L.planes, S.L.stride,  n,   S.L.cnt, S.L.root, weight, set,
                        segs,       nullptr,     S.r, init,    nullptr,  nullptr, nullptr};
     const unsigned blocks = (unsigned)((n + 255) / 256);
@@ -613,26 +671,11 @@ int Server::retire(ServeLevel *S)
 
 int Server::scan_level(ServeLevel &S)
 {
-    if (tt && (S.r == 2 || S.r == 3) && !S.tt) {
-        const int rc = probe_level(S);
-        if (rc != PERFT_OK) return rc;
-    }
-    if (!S.merged) {
-        const int rc = merge_level(S);
-        if (rc != PERFT_OK) return rc;
-        S.merged = true;  // (a scan that finds no memory is retried)
-    }
-    if (S.tt && !S.live) S.live = (u32 *)take(4 * S.L.n, S.mem);  // hits and copies make no parents (without: all do)
+    const int rcMerge = table_level(S.r) ? probe_level(S) : merge_level(S);
+    if (rcMerge != PERFT_OK) return rcMerge;
     const u64 n = S.L.n;
     const u64 nb = (n + SCAN_CHUNK - 1) / SCAN_CHUNK;
-    S.pscan = (u64 *)take(8 * (n + 1), S.mem);
-    S.tileFirst = S.r > 2 ? (u32 *)take(4 * tile_index_len(n), S.mem) : nullptr;  // (the count-only ply has no tiles)
-    std::vector<std::pair<u64, u64>> tmp;
-    ScanSums *bsum = (ScanSums *)take(sizeof(ScanSums) * (nb + 1), tmp);
-    if (!S.pscan || (S.r > 2 && !S.tileFirst) || !bsum) {
-        give_back(tmp);
-        return PERFT_ERR_OUT_OF_MEMORY;
-    }
+    ScanSums *bsum = S.bsum;
     k_scan_reduce<<<(unsigned)nb, SCAN_NT, 0, st>>>(S.L.cnt, n, bsum);
     u64 *totals = (u64 *)(bsum + nb);
     k_scan_top<<<1, SCAN_TOP_NT, 0, st>>>(bsum, nb, totals);
@@ -649,7 +692,7 @@ int Server::scan_level(ServeLevel &S)
         launches++;
     }
     const bool readOk = cudaMemcpyAsync(hostTotal, totals, 16, cudaMemcpyDeviceToHost, st) == cudaSuccess;
-    give_back(tmp);  // reused only by later launches on this stream
+    give_back(S.scanMem);  // reused only by later launches on this stream
     if (!readOk || cudaStreamSynchronize(st) != cudaSuccess) return PERFT_ERR_CUDA;
     S.total = hostTotal[0];
     S.nParents = S.live ? hostTotal[1] : n;
@@ -719,11 +762,7 @@ int Server::advance()
         for (size_t li = 0; li < work.size(); li++) {
             ServeLevel *S = work[li];
             if (!S->scanned) {
-                int rc = scan_level(*S);
-                if (rc == PERFT_ERR_OUT_OF_MEMORY) {  // retry next iteration
-                    keep.push_back(S);
-                    continue;
-                }
+                const int rc = scan_level(*S);
                 if (rc != PERFT_OK) return rc;
             }
             // (the count-only ply's parents count as one item each, see k_tile)
@@ -739,15 +778,12 @@ int Server::advance()
                         C = new ServeLevel();
                         C->r = r - 1;
                         C->depth = S->depth;
-                        const u64 m = hi - lo;
-                        C->L.n = m;
-                        C->L.stride = (m + 31) & ~31ULL;
-                        C->L.planes = (u64 *)take(48 * C->L.stride, C->mem);
-                        C->L.cnt = (u32 *)take(4 * C->L.stride, C->mem);
-                        C->L.root = (u32 *)take(4 * C->L.stride, C->mem);
-                        if (S->L.weight) C->L.weight = (unsigned long long *)take(8 * C->L.stride, C->mem);
-                        if (C->L.planes && C->L.cnt && C->L.root && (C->L.weight || !S->L.weight)) break;
-                        give_back(C->mem);
+                        if (take_level(*C, hi - lo, S->L.weight != nullptr)) {
+                            if (blockBytes - inUse >= reserve_below(C->r)) break;
+                            give_back(C->mem);
+                            give_back(C->ttMem);
+                            give_back(C->scanMem);
+                        }
                         delete C;
                         C = nullptr;
                         if (hi - lo <= (u64)TILE_CAP) break;
