@@ -120,17 +120,28 @@ void enumerate_counts(const Board &b, u32 plies, BoardCounts &out)
 // Ids of distinct boards by board: open addressing over the board list itself,
 // at most half full.  The merge of the root moves' maps is serial and looks up
 // every (root move, board) pair once, so with a hash node per board it took
-// most of a frontier's time.  Initial position on 8 cores, with the maps'
-// buffers above: 5,362 boards 1.8 -> 1.1 ms, 72,078 boards 37 -> 15 ms, 822,518
-// boards 1.3 -> 0.6 s.  The boards' order is unchanged.
+// most of a frontier's time.  On 8 cores, with the maps' buffers above: initial
+// position 5,362 boards 1.5 -> 0.8 ms, 72,078 boards 28 -> 13 ms, 822,518 boards
+// 781 -> 324 ms; a middlegame's 557,213 boards 398 -> 170 ms.  The boards' order
+// is unchanged.
 struct BoardIndex {
     static constexpr u32 NONE = 0xFFFFFFFFu;
+    int log2Slots = 12;
     std::vector<u32> slots = std::vector<u32>(1u << 12, NONE);
 
+    // A board's first slot, from the top bits of one more multiplication: the
+    // low bits of the hash do not depend on the top ranks' bits of the board,
+    // and with slots taken from them neighbouring boards filled the same runs:
+    // that middlegame took 272 ms, 19,312 boards of a rook ending 8.1 ms
+    // (a hash node per board 5.3, these slots 2.2).
+    size_t home(const BoardKey &k) const
+    {
+        return (size_t)(((u64)BoardKeyHash()(k) * 0x9E3779B97F4A7C15ULL) >> (64 - log2Slots));
+    }
     size_t slot_of(const std::vector<BoardKey> &boards, const BoardKey &k) const
     {
         const size_t mask = slots.size() - 1;
-        size_t at = BoardKeyHash()(k) & mask;
+        size_t at = home(k);
         while (slots[at] != NONE && !(boards[slots[at]] == k)) at = (at + 1) & mask;
         return at;
     }
@@ -143,6 +154,7 @@ struct BoardIndex {
         boards.push_back(k);
         slots[at] = id;
         if (2 * boards.size() > slots.size()) {
+            log2Slots++;
             slots.assign(2 * slots.size(), NONE);
             for (u32 i = 0; i <= id; i++) slots[slot_of(boards, boards[i])] = i;
         }
