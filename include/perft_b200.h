@@ -145,7 +145,8 @@ int perft_batch_noalloc(const perft_pos48 *d_pos, const uint8_t *depths, uint32_
 typedef struct perft_serve_config {
     uint64_t memory_bytes;   /* budget for resident frontiers (0: 90% of the free arena) */
     uint64_t step_items;     /* items a level may advance per iteration (0: 2^27); the count-only
-                                ply advances by step_items / 32 parents */
+                                ply advances by step_items / 32 parents, 8192 at least: about
+                                260,000 moves, of which it makes a quarter */
     uint32_t max_in_flight;  /* admitted queries at once (0: 4096, at most 65536) */
     int32_t  use_tt;         /* 1 (default): frontier levels two and three plies above the leaves
                                 probe, de-duplicate and store into the engine's transposition table

@@ -8,8 +8,9 @@
 //   1. admit queued queries while slots are free and the predicted
 //      level-buffer memory of all admitted queries fits the budget;
 //   2. advance every pool, the count-only last ply first, each level by at
-//      most `step_items` (tile-aligned), so a large level never blocks the
-//      small levels of newer queries for more than one step;
+//      most `step_items` (tile-aligned; the count-only ply by as many parents
+//      as have about that many moves, see advance), so a large level never
+//      blocks the small levels of newer queries for more than one step;
 //   3. read back the per-query pending-node counters (maintained on the
 //      device by the tracking tile kernels) and complete every query whose
 //      counter reached zero.
@@ -20,9 +21,11 @@
 //
 // Transposition table: with an engine table and use_tt, every level two or
 // three plies above the leaves (remaining depth 2 or 3) is hashed and probed
-// before its scan, exactly as the engine's own table levels are (k_tt_probe,
-// k_tt_dedup): table hits take the stored count and generate nothing, and
-// identical nodes of the level are searched once.  Counts then flow up per
+// before its scan, exactly as the engine's own table levels are: identical
+// nodes of the level are searched once (k_merge_linked), and the others that
+// hit the table take the stored count and generate nothing (k_tt_probe).
+// Levels further above the leaves are not merged then; without a table every
+// level is, within each query (merge_level).  Table levels' counts flow up per
 // node, not per query:
 //   * a remaining-depth-3 level expands without pending-count tracking; each
 //     child level (remaining depth 2) it produces sums its leaf ply per node
@@ -572,9 +575,9 @@ int Server::admit()
     return cudaGetLastError() == cudaSuccess ? PERFT_OK : PERFT_ERR_CUDA;
 }
 
-// Hashes and probes a level two or three plies above the leaves, and
-// de-duplicates its misses; hits and duplicates get no items.  The level
-// keeps the hashes, per-node sums and aliases until it is finished.
+// Merges a level two or three plies above the leaves over all its queries, then
+// hashes and probes the nodes that stay; copies and hits get no items.  The
+// level keeps the hashes, per-node sums and aliases until it is finished.
 int Server::probe_level(ServeLevel &S)
 {
     const u64 n = S.L.n;
@@ -765,7 +768,12 @@ int Server::advance()
                 const int rc = scan_level(*S);
                 if (rc != PERFT_OK) return rc;
             }
-            // (the count-only ply's parents count as one item each, see k_tile)
+            // The count-only ply's parents count as one item each (see k_tile), but
+            // the positions of depth-2 queries as their moves.  At least 8192 of them:
+            // the launch is most of a smaller step's time, so that no query gets
+            // done sooner.  200 queries of depths 3-6 with step_items 8192: a tenth
+            // done after 2.0 ms and all after 0.72 s; in steps of 256 parents 2.5 ms
+            // and 4.4 s.
             const u64 step = r == 2 ? std::max<u64>(stepItems / SERVE_MOVES_PER_PARENT, TILE_CAP) : stepItems;
             u64 lo = S->next, hi = std::min(S->total, lo + step);
             if (lo < hi) {
