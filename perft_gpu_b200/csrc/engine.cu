@@ -64,9 +64,6 @@ namespace {
 #ifndef PG_ONE_RUN_VOTE
 #define PG_ONE_RUN_VOTE 1  // one block vote for windows whose parents share one root
 #endif
-#ifndef PG_ONE_RUN_SUM
-#define PG_ONE_RUN_SUM 1  // such windows sum their counts with a plain warp reduction
-#endif
 #ifndef PG_MIRRORED_STAGE
 #define PG_MIRRORED_STAGE 1  // parents staged mirrored: children are made in their own frame
 #endif
@@ -148,8 +145,10 @@ constexpr u64 NODE_BYTES_MERGE = 6 * 8 + 4 + 4 + 8 + 8 * MERGE_SLOTS + 1;
 // Plies from the root at which merging starts: two plies reach almost no
 // position twice, the third brings the first a-x-b = b-x-a pairs.
 constexpr int MERGE_MIN_PLIES = 3;
-// Share of a merged level's nodes predicted to stay (measured: 0.54-0.68 in
-// 8-30-ply playouts); predictions only choose the path and the grids.
+// Share of a merged level's nodes predicted to stay; predictions only choose
+// the path and the grids.  The third and fourth plies keep 0.58-0.61 of their
+// children, in openings and in 8-30-ply playouts alike, the initial position's
+// fifth 0.46: the deeper the level, the more it is below the prediction.
 constexpr double MERGE_KEPT = 0.7;
 
 // ------------------------------------------------------- level node boards
@@ -493,7 +492,7 @@ struct DevPlan {
     // roots that join level k (their depth is the level's remaining depth)
     u32 joinN[DD_MAX_LEVELS];
     const u32 *joinIds[DD_MAX_LEVELS];
-    int capMax[DD_MAX_LEVELS];  // largest tile (log2 items) for the items of level k
+    int capMax[DD_MAX_LEVELS];  // largest tile (log2 items) for the items of level k (interior plies)
     int lastLv;                    // the count-only ply's level
     int weighted;                  // levels carry path weights (some level is merged)
     int mergeLv[DD_MAX_LEVELS];    // level k's transpositions are merged
@@ -628,9 +627,12 @@ __device__ void dd_plan_level(DevPlan *plan, int lv, int last, ScanSums sums)
     const u64 nParents = L.live ? sums.live : n;
     if (n) L.pscan[nParents] = total;
     L.total = total;  // (0 when the plan has overflowed: the sums are those of no nodes)
-    int cap = plan->capMax[lv] ? plan->capMax[lv] : TILE_CAP_LOG2;
-    while (cap > TILE_MIN_LOG2 && (total >> cap) < plan->tileTarget) cap--;
-    cap = tile_log2_for(total, n, cap);
+    int cap = TILE_CAP_LOG2;
+    if (!last) {  // (the count-only ply has no tiles)
+        cap = plan->capMax[lv];
+        while (cap > TILE_MIN_LOG2 && (total >> cap) < plan->tileTarget) cap--;
+        cap = tile_log2_for(total, n, cap);
+    }
     L.capLog2 = cap;
     *plan->tileCounter = 0;  // the next launch is this level's tile launch
     TileParams &T = plan->tp[lv];  // host fields (cursor, outputs, error word) come from the template
@@ -1898,8 +1900,8 @@ private:
 
 public:
     // Launch configuration per (ply kind, remaining depth of the parent level):
-    // slider variant, largest tile (log2 items) and resident CTAs per SM.  The
-    // count-only ply always has remaining depth 2; interior plies have 3..20
+    // slider variant, largest tile (log2 items; interior plies) and resident CTAs
+    // per SM.  The count-only ply always has remaining depth 2; interior plies have 3..20
     // and use the entry of the nearest calibrated depth.
     struct TuneCfg {
         int sv = SV_KOGGE;
@@ -2389,11 +2391,12 @@ int Engine::scan(const u32 *cnt, u64 n, int remaining, bool compact, ParentIndex
     ix.nParents = compact ? hPinned[1] : n;
     // tile size: the tuned largest tile for this ply, made smaller while some
     // resident CTA would get no second tile
-    const int mode = remaining == 2 ? MODE_LEAF : MODE_EXPAND;
-    const TuneCfg &tc = cfg_for(mode, remaining);
-    ix.capLog2 = tc.cap;
-    while (ix.capLog2 > TILE_MIN_LOG2 && (ix.total >> ix.capLog2) < 2ull * grid_for(mode, tc)) ix.capLog2--;
-    ix.capLog2 = tile_log2_for(ix.total, n, ix.capLog2);
+    if (tiles) {
+        const TuneCfg &tc = cfg_for(MODE_EXPAND, remaining);
+        ix.capLog2 = tc.cap;
+        while (ix.capLog2 > TILE_MIN_LOG2 && (ix.total >> ix.capLog2) < 2ull * grid_for(MODE_EXPAND, tc)) ix.capLog2--;
+        ix.capLog2 = tile_log2_for(ix.total, n, ix.capLog2);
+    }
     if (compact)
         k_scan_apply<true><<<(unsigned)nb, SCAN_NT, 0, stream>>>(cnt, n, bsum, totals, ix.pscan, ix.live,
                                                                             ix.tileFirst, ix.capLog2);
@@ -2550,7 +2553,7 @@ int Engine::process_level(const DeviceLevel &L, int remaining, unsigned long lon
 // to its (ply kind, remaining depth) key, and each key keeps the median of
 // its three runs.  Coordinate search, every key at once:
 //   1. slider variant (all five), largest tiles, all resident CTAs;
-//   2. largest tile 2^13 / 2^12 / 2^11 items with each key's variant;
+//   2. interior plies: largest tile 2^13 / 2^12 / 2^11 items with each key's variant;
 //   3. resident CTAs per SM: all that fit, or one fewer.
 // A candidate replaces a key's current choice only when it is more than 1%
 // faster, so near-ties resolve to the same (earlier) choice on every run.
@@ -2670,12 +2673,12 @@ int Engine::autotune(bool leaf, bool expand)
             }
         });
     }
-    // stage 2: largest tile
-    for (int cap = TILE_CAP_LOG2 - 1; cap >= TILE_CAP_LOG2 - 2 && cap >= TILE_MIN_LOG2; cap--) {
-        keys([&](int m, int r) { apply(m, r, TuneCfg{chosen[m][r].sv, cap, 0, 0}); });
+    // stage 2: largest tile (interior plies; the count-only ply has none)
+    for (int cap = TILE_CAP_LOG2 - 1; expand && cap >= TILE_CAP_LOG2 - 2 && cap >= TILE_MIN_LOG2; cap--) {
+        keys([&](int m, int r) { apply(m, r, m == MODE_LEAF ? chosen[m][r] : TuneCfg{chosen[m][r].sv, cap, 0, 0}); });
         if ((rc = measure()) != PERFT_OK) return rc;
         keys([&](int m, int r) {
-            if (med[m][r] < 0.99 * best[m][r]) {
+            if (m != MODE_LEAF && med[m][r] < 0.99 * best[m][r]) {
                 best[m][r] = med[m][r];
                 chosen[m][r] = TuneCfg{chosen[m][r].sv, cap, 0, med[m][r]};
             }
@@ -2913,7 +2916,7 @@ int Engine::build_dd(DDGraph &G)
         c.sv = ddSv(c.sv);
         lvSv[lv] = c.sv;
         lvGrid[lv] = grid_for(mode, c);
-        G.hTemplate->capMax[lv] = c.cap;
+        if (!last) G.hTemplate->capMax[lv] = c.cap;
         TileParams &T = G.hTemplate->tp[lv];  // the scan fills the level fields on the device
         T.tileCounter = dCounter;
         T.rootCounts = (unsigned long long *)G.dOut;
@@ -3002,7 +3005,7 @@ int Engine::build_dd(DDGraph &G)
             if (G.hTemplate->mergeLv[lv + 1]) {
                 // grid-stride: any grid is correct; a block per 256 predicted nodes, up
                 // to 512 blocks per SM.  The prediction takes 0.7 of a merged level to
-                // remain; openings keep far less, and most of its blocks would find no
+                // remain; deep levels keep less, and most of its blocks would find no
                 // node (an opening at depth 8 7.16 -> 6.74 ms, 512 positions at depths
                 // 4-6 38.7 -> 38.3 ms; 128, 256 and 1024 blocks per SM: 6.82, 6.80 and
                 // 6.75 ms).
@@ -3612,10 +3615,11 @@ int perft_reset_stats(void)
 // device memory — processes whose HBM is already reserved by another
 // allocator (a serving framework or torch's caching allocator holding the
 // device), and latency-critical callers for which cudaMalloc's implicit
-// device-wide synchronisation is unacceptable.  It runs the same kernels as
-// perft_batch_device, but every level buffer, scan, tile index and counter
-// lives in one fixed scratch array compiled into this library, so the call
-// allocates nothing.  Trees whose levels do not fit the scratch are refused
+// device-wide synchronisation is unacceptable.  It runs the interior and
+// count-only kernels of perft_batch_device, but every level buffer, scan, tile
+// index and counter lives in one fixed scratch array compiled into this
+// library, so the call allocates nothing.  The scratch has no room for merge
+// sets: equal nodes are not merged, every move path is searched.  Trees whose levels do not fit the scratch are refused
 // (PERFT_ERR_OUT_OF_MEMORY); the arena engine handles those by chunking.
 //
 // The scratch is a file-scope __device__ array: every GPU that loads this
