@@ -720,9 +720,9 @@ __global__ void k_dd_join(DevPlan *plan, int lv, const u64 *__restrict__ pos48, 
 
 // ------------------------------------------------- merged transpositions
 // Different move orders reach the same position.  From the third ply below a
-// root on, a level therefore holds many equal nodes (42% of the third ply's
-// children and again 42% of the fourth's in 8-30-ply playouts), and each
-// copy's whole subtree would be searched again.  Before a level is scanned,
+// root on, a level therefore holds many equal nodes (about 40% of the third
+// ply's children and again 40% of the fourth's, in openings and in 8-30-ply
+// playouts), and each copy's whole subtree would be searched again.  Before a level is scanned,
 // equal nodes of one root are merged: one of them, the owner, keeps its
 // moves and takes over the others' path weights; the others lose theirs
 // (cnt = 0).  A node's weight is the number of move paths from its root that
@@ -1308,6 +1308,12 @@ __global__ void __launch_bounds__(LEAF_NT, LEAF_MINB) k_leaf(const TileParams Pi
 constexpr int SMALL_NT = 128;  // threads per CTA: small CTAs put more subtrees in flight
 constexpr int SMALL_MINB = 4;
 constexpr int SMALL_MAX_DEPTH = 5;
+// Largest batch: at depth 4 alone one launch and a replayed graph of levels
+// meet here (64 positions 216 us in one launch, 220 as levels; 32 positions 117
+// and 211).  Shallower and mixed batches still gain at this size (64 of depths
+// 1-4 90 and 221 us, and 451 in the first call with a new mix).  A depth-5
+// position fills the device by itself (smallGrid CTAs), so batches of them are
+// left to the levels.
 constexpr int SMALL_BATCH = 64;
 constexpr int SMALL_BATCH_DEPTH = 4;
 constexpr u32 SMALL_LIST_CAP = 4096;  // most subtree roots of a depth-5 position (larger trees: level pipeline)
@@ -3035,10 +3041,11 @@ int Engine::build_dd(DDGraph &G)
 // Batches whose predicted tree fits the arena run as one replayed graph,
 // whatever their depth mix: the launch sequence is fixed and the sizes live
 // on the device, so the host only waits once.  The prediction charges each
-// root its own move count times 35 per further ply, 72 bytes per node of the
-// last materialised ply (planes, count, root, scan entry, tile index) and of
-// the plies above it, against 80% of the free arena.  `handled` stays false
-// when the batch is not eligible or the device plan overflowed; the caller
+// root its own move count times 32 per further ply (times MERGE_KEPT from the
+// third ply on, where levels are merged) and 72 bytes per node of every
+// materialised ply (planes, count, root, scan entry, tile index; 92 with path
+// weights, live list and merge set), against 85% of the free arena.  `handled`
+// stays false when the batch is not eligible or the device plan overflowed; the caller
 // then runs the host-driven path.
 int Engine::run_dd(const u64 *dPos, const uint8_t *depths, u32 n, u64 *dOut, bool &handled)
 {
@@ -3059,10 +3066,8 @@ int Engine::run_dd(const u64 *dPos, const uint8_t *depths, u32 n, u64 *dOut, boo
     if (G && G->overflowed) return PERFT_OK;
     std::vector<double> predLv;
     if (!G && !ddForce) {
-        // Predicted bytes of the materialised plies: each root's own move
-        // count times 32 per further ply (the measured mean is about 30),
-        // 72 bytes per node.  The positions are read back once, when the
-        // graph is built; a replay needs no prediction.
+        // (The measured mean is about 30 moves.)  The positions are read back
+        // once, when the graph is built; a replay needs no prediction.
         std::vector<u64> hp(6ull * n);
         ENG_TRY(cudaMemcpyAsync(hp.data(), dPos, 48ull * n, cudaMemcpyDeviceToHost, stream));
         ENG_TRY(cudaStreamSynchronize(stream));
@@ -3220,11 +3225,15 @@ int Engine::run_small(const u64 *dPos, const u64 *pos, const uint8_t *depths, u3
 // Whether a batch's trees meet often enough to be searched as one: positions
 // of one depth whose occupied squares differ in at most RELATED_SQUARES from
 // the first one's, as the boards of a divided or host-split search do (five
-// plies move at most ten squares; unrelated playouts differ in 20-30), and
+// plies move at most ten squares; unrelated middlegames differ in 20-30), and
 // enough work to pay for the linked levels' host round trips.  Measured,
 // searched together against root by root, by predicted parents of the
 // count-only ply: 0.4 M 0.91 / 0.78 ms, 0.54 M 0.52 / 0.37, 0.9 M 0.94 / 1.14
-// and 1.30 / 2.13, 5.6 M 3.2 / 5.2, 12 M 15.4 / 61.7 ms.
+// and 1.30 / 2.13, 5.6 M 3.2 / 5.2, 12 M 15.4 / 61.7 ms.  Unrelated openings of
+// up to 3 plies qualify too: 1000 of depth 4 (0.9 M) 0.41 / 0.29 ms, 100 of
+// depth 5 (2.7 M) 0.60 / 0.48, 400 of depth 5 (11 M) 0.97 / 1.30, 30 and 60 of
+// depth 6 (24 and 49 M) 1.58 / 1.66 and 1.90 / 2.82 (openings of 4-8 plies did
+// not qualify).
 constexpr int RELATED_SQUARES = 12;
 constexpr double RELATED_MIN_NODES = double(3u << 18);
 bool related_roots(const u64 *pos, const uint8_t *depths, u32 n)
