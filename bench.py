@@ -306,6 +306,9 @@ def run_reference(args):
             "cpu_baseline": {"value": v, "unit": UNIT, "cores": last["cores"], "kind": last["kind"],
                              "cpu": last["cpu"], "library": last["library"], "sample": last["sample"]},
             "e2e": {"value": v, "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
+    if last["kind"] != "reference":
+        line["unavailable"] = ("the reference's own library (oracle/_ref) is not built here; "
+                               "the figures are those of this repository's CPU oracle")
     print(json.dumps(line), flush=True)
     return 0
 
@@ -600,6 +603,8 @@ def run_ours(args):
         "achieved": achieved / 1e12 if achieved else None,
         "peak": peak / 1e12 if peak else None,
         "unit": "Tops/s (32-bit thread instructions issued: ncu instructions/item x items / time)",
+        "work_source": "instructions per item of one ncu capture of the kernel on 16 positions "
+                       "(profiles/leaf_kernel_traffic.json), not counted in this run",
         "frac": (achieved / peak) if (achieved and peak) else None,
         "peak_source": "of measured: best of the integer instruction mixes timed on this GPU by libperft_probe.so",
         "peak_variants_tops": {k: v / 1e12 for k, v in peaks.items()} if peaks else None,

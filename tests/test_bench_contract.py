@@ -75,3 +75,9 @@ def test_reference_arm_loads_no_engine_library():
     assert "ENGINE_NOT_MAPPED" in r.stdout
     line = json.loads(next(x for x in r.stdout.splitlines() if x.startswith("{")))
     assert line["cpu_baseline"]["library"].startswith("oracle/")
+
+
+def test_reference_arm_says_when_the_reference_is_not_there():
+    """Figures of the oracle are not passed off as the reference's."""
+    d = _run("--steps", "1", "--warmup", "0", "--cpu-seconds", "1")
+    assert ("unavailable" in d) == (d["cpu_baseline"]["kind"] != "reference")
