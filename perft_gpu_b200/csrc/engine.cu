@@ -772,6 +772,10 @@ struct MergeLevel {
 constexpr u32 ALIAS_HIT = 0xFFFFFFFFu;     // final value in acc: from the table, or no moves
 constexpr u32 ALIAS_NOSLOT = 0xFFFFFFFEu;  // searched by itself (no slot found in the set)
 
+// Multiplies each word by an odd constant and finishes with xor-shifts.  The
+// constants are known 64-bit hash multipliers: 2^64 / golden ratio, two of
+// xxHash64's primes (the second and third), degski's 64-bit mixer's multiplier
+// and two of wyhash's defaults.
 __device__ __forceinline__ u64 board_hash(const Board &b)
 {
     u64 h = b.mine * 0x9E3779B97F4A7C15ULL + b.pawns * 0xC2B2AE3D27D4EB4FULL + b.knights * 0x165667B19E3779F9ULL +
