@@ -1464,10 +1464,15 @@ PG_HD void quiet_setup(const Board &f, QuietCtx &q)
     L.V = (kAtt & L.notB) | kB;
     L.bad = 0;
     L.attacked = 0;
-    if (st & 1) L.V |= 0x60ULL;
+    // (a move from or to a rook's corner takes the right: without its rook,
+    // which a position's state may claim all the same, a quiet one does)
+    if (st & 1) {
+        L.V |= 0x60ULL;
+        L.bad |= 0x80ULL;
+    }
     if (st & 2) {
         L.V |= 0x0CULL;
-        L.bad |= 0x0EULL;
+        L.bad |= 0x0FULL;
     }
     const u64 aB = f.bq & A, aR = f.rq & A;
     // pins, and sliders one more piece away from a pin

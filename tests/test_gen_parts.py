@@ -103,3 +103,18 @@ def test_quiet_replies_playouts(gp, oracle, plies):
             quiet += _check_replies(gp, oracle, p)
             moves += len(kids)
     assert quiet > moves // 4  # the sets do carry the bulk of the moves
+
+
+@pytest.mark.parametrize("fen", [
+    "4k3/8/8/8/8/8/8/B3K3 w k - 0 1", "4k2B/8/8/8/8/8/8/4K3 w k - 0 1", "B3k3/8/8/8/8/8/8/4K3 w q - 0 1",
+    "4k3/8/8/8/8/8/8/4K2B w q - 0 1", "b3k3/8/8/8/8/8/8/4K3 b K - 0 1", "4k3/8/8/8/8/8/8/4K2b b K - 0 1",
+    "4k2b/8/8/8/8/8/8/4K3 b Q - 0 1", "4k3/8/8/8/8/8/8/b3K3 b Q - 0 1"])
+def test_quiet_replies_with_rights_that_have_no_rook(gp, oracle, fen):
+    """A position's state may claim a castling right whose corner holds no
+    rook; a quiet move from or to that corner takes the right all the same,
+    as it does when the move is made and its replies are counted."""
+    pos = oracle.fen_to_pos(fen)
+    n = ctypes.c_uint32(0)
+    got = gp.gp_replies(P6(*[int(x) for x in pos]), ctypes.byref(n))
+    assert n.value > 0
+    assert got == sum(oracle.count(np.array(k, dtype=np.uint64)) for k in _children(gp, pos))
