@@ -1515,7 +1515,7 @@ __global__ void __launch_bounds__(SMALL_NT, SMALL_MINB) k_small_trees(const __gr
     if (tid == 0) S.flags = 0;
     __syncthreads();
     // the position's count and its check at the same time (no count without
-    // both kings: it would read outside the tables)
+    // both kings: the move tables are indexed by their squares)
     if (tid == 0 || tid == 32) {
         u64 p[6];
 #pragma unroll

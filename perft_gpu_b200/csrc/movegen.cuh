@@ -1730,8 +1730,9 @@ constexpr int MAX_ANY_MOVES = 63 * 16 + 8 * 3 * 3 + 2;
 PG_HD bool moves_as_counted(u32 counted, u32 generated) { return counted == 1 || counted == generated; }
 
 // ---------------------------------------------------------- validation
-// What the generator needs of a board to stay within its tables: they are
-// indexed by both kings' squares.
+// What the generator needs of a board before anything else: its tables are
+// indexed by both kings' squares.  (Without a king the bit scan gives square
+// 31, or with PG_CTZ32 0 an index outside the tables.)
 PG_HD bool one_king_each(const u64 p[6]) { return popc(p[5] & p[0]) == 1 && popc(p[5] & ~p[0]) == 1; }
 
 // 0 when a pos48 board is a position the generator can search: piece planes
